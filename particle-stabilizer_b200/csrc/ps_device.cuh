@@ -131,9 +131,10 @@ struct SceneParams {
   uint32_t mesh_tris;
   uint32_t mesh_bin_base;  // first bin of this scene's triangle bins
   int32_t mesh_nb[3];      // triangle-bin grid
-  T mesh_lo[3];            // triangle-bin grid origin = lower corner of the mesh AABB
-  T mesh_hi[3];            // upper corner of the mesh AABB
+  T mesh_lo[3];            // triangle-bin grid origin: the mesh AABB widened by mesh_reach
+  T mesh_hi[3];            // its upper corner
   T mesh_iv;               // triangle-bin edge
+  T mesh_reach;            // largest radius the bins' lists are made for
   int32_t edge_quirk;
   // unsigned division by nz and by ny with a multiply-high (Granlund &
   // Montgomery): q = (t + ((x - t) >> sh1)) >> sh2, t = umulhi(x, m)
@@ -167,7 +168,7 @@ inline void fast_udiv_magic(uint32_t d, uint32_t& m, uint32_t& sh1, uint32_t& sh
 // Device error word bits (read by the host after a step block).
 enum : uint32_t {
   PS_DEVERR_SCAN_TIMEOUT = 1u << 0,   // decoupled look-back gave up waiting
-  PS_DEVERR_MESH_OVERFLOW = 1u << 1,  // reserved: hits beyond the buffer now take further passes
+  PS_DEVERR_MESH_OVERFLOW = 1u << 1,  // reserved: a sphere may touch any number of triangles
   PS_DEVERR_BAD_CELL = 1u << 2,       // a cell id fell outside its scene (never expected)
   PS_DEVERR_LIST_OVERFLOW = 1u << 3,  // neighbour-list mode: a list or a sphere's overlap buffer was full
   PS_DEVERR_LIST_BARRIER = 1u << 4,   // neighbour-list mode: a grid barrier of the rebuild gave up waiting

@@ -93,7 +93,7 @@ struct GridHost {
   int32_t nb[3];
   int64_t n_cells, cbase;
   // triangle bins
-  double mesh_lo[3], mesh_hi[3], mesh_iv;
+  double mesh_lo[3], mesh_hi[3], mesh_iv, mesh_reach;
   int32_t mesh_nb[3];
   int64_t n_bins, bin_base, tri_base, n_tri;
 };
@@ -132,7 +132,7 @@ struct ps_sim {
   StatsPartial* d_stats = nullptr;
   StatsPartial* d_stats_out = nullptr;
   // triangle data
-  void *d_tri = nullptr, *d_nrm = nullptr, *d_aabb = nullptr;
+  void *d_tri = nullptr, *d_aabb = nullptr;
   uint32_t *d_bin_offset = nullptr, *d_bin_tri = nullptr;
   MeshView* d_mesh_view = nullptr;
 
@@ -640,6 +640,7 @@ SceneParams<T> make_params(const ps_scene_desc& d, const GridHost& g, int64_t pb
   sp.mesh_tris = (uint32_t)g.n_tri;
   sp.mesh_bin_base = (uint32_t)g.bin_base;
   sp.mesh_iv = (T)g.mesh_iv;
+  sp.mesh_reach = (T)g.mesh_reach;
   sp.edge_quirk = d.edge_quirk;
   fast_udiv_magic((uint32_t)std::max(1, g.nb[2]), sp.div_nz_m, sp.div_nz_sh1, sp.div_nz_sh2);
   fast_udiv_magic((uint32_t)std::max(1, g.nb[1]), sp.div_ny_m, sp.div_ny_sh1, sp.div_ny_sh2);
@@ -734,13 +735,21 @@ int upload_bounds(ps_sim* s) {
   return PS_OK;
 }
 
-// Triangle data in precision T for every scene, binned by AABB.
+// Triangle data in precision T for every scene, and the bins' lists: a bin
+// lists the triangles that a sphere of radius mesh_reach or less with its
+// centre in the bin can touch.  Such a sphere's box meets the triangle's, so
+// the bins are those that the triangle's box, widened by mesh_reach, covers;
+// and the point it touches lies in the triangle's plane, so bins further
+// than mesh_reach from the plane are left out (a third of the entries of a
+// slanted wall remain).
 template <class T>
 int upload_mesh(ps_sim* s) {
-  std::vector<T> tri, nrm, aabb;
+  std::vector<T> tri, aabb;
+  std::vector<double> nrm;
   std::vector<uint32_t> bin_offset((size_t)s->bins_total + 1, 0), bin_tri;
-  std::vector<std::vector<uint32_t>> per_bin_counts;
-  tri.reserve((size_t)s->tri_total * 9);
+  tri.reserve((size_t)s->tri_total * 12);
+  aabb.reserve((size_t)s->tri_total * 8);
+  nrm.reserve((size_t)s->tri_total * 3);
   for (int sc = 0; sc < s->n_scenes; ++sc) {
     const GridHost& g = s->grids[sc];
     const std::vector<double>& soup = s->tris[sc];
@@ -752,11 +761,14 @@ int upload_mesh(ps_sim* s) {
       const double r1x = v[6] - v[0], r1y = v[7] - v[1], r1z = v[8] - v[2];
       const double nx = r0y * r1z - r0z * r1y, ny = r0z * r1x - r0x * r1z, nz = r0x * r1y - r0y * r1x;
       const double len = std::sqrt(nx * nx + ny * ny + nz * nz);
-      nrm.push_back((T)(nx / len));
-      nrm.push_back((T)(ny / len));
-      nrm.push_back((T)(nz / len));
+      for (const double c : {nx / len, ny / len, nz / len}) {
+        nrm.push_back(c);
+        tri.push_back((T)c);
+      }
       for (int a = 0; a < 3; ++a) aabb.push_back(std::min(std::min((T)v[a], (T)v[3 + a]), (T)v[6 + a]));
+      aabb.push_back(T(0));
       for (int a = 0; a < 3; ++a) aabb.push_back(std::max(std::max((T)v[a], (T)v[3 + a]), (T)v[6 + a]));
+      aabb.push_back(T(0));
     }
   }
   // two passes: count, then fill (ascending triangle id inside each bin)
@@ -771,16 +783,26 @@ int upload_mesh(ps_sim* s) {
       const GridHost& g = s->grids[sc];
       const T lo[3] = {(T)g.mesh_lo[0], (T)g.mesh_lo[1], (T)g.mesh_lo[2]};
       const T iv = (T)g.mesh_iv;
+      double size = g.mesh_iv;  // of the coordinates, for the rounding of the device's own tests
+      for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
+      const double reach = 1.001 * g.mesh_reach + 1e-6 * size;
       for (int64_t t = 0; t < g.n_tri; ++t) {
         const int64_t gt = g.tri_base + t;
         int32_t b0[3], b1[3];
         for (int a = 0; a < 3; ++a) {
-          b0[a] = host_mesh_axis<T>(aabb[6 * gt + a], lo[a], iv, g.mesh_nb[a]);
-          b1[a] = host_mesh_axis<T>(aabb[6 * gt + 3 + a], lo[a], iv, g.mesh_nb[a]);
+          b0[a] = host_mesh_axis<T>((T)((double)aabb[8 * gt + a] - reach), lo[a], iv, g.mesh_nb[a]);
+          b1[a] = host_mesh_axis<T>((T)((double)aabb[8 * gt + 4 + a] + reach), lo[a], iv, g.mesh_nb[a]);
         }
+        const double* n = nrm.data() + 3 * gt;
+        const double* v0 = s->tris[sc].data() + 9 * t;
+        const double far = reach + (0.5 + 1e-3) * g.mesh_iv * (std::fabs(n[0]) + std::fabs(n[1]) + std::fabs(n[2])) + 1e-5 * size;
         for (int32_t x = b0[0]; x <= b1[0]; ++x)
           for (int32_t y = b0[1]; y <= b1[1]; ++y)
             for (int32_t z = b0[2]; z <= b1[2]; ++z) {
+              const double h = n[0] * (g.mesh_lo[0] + (x + 0.5) * g.mesh_iv - v0[0]) +
+                               n[1] * (g.mesh_lo[1] + (y + 0.5) * g.mesh_iv - v0[1]) +
+                               n[2] * (g.mesh_lo[2] + (z + 0.5) * g.mesh_iv - v0[2]);
+              if (std::fabs(h) > far) continue;  // (a triangle without a normal stays)
               const int64_t bin = g.bin_base + ((int64_t)x * g.mesh_nb[1] + y) * g.mesh_nb[2] + z;
               if (pass == 0)
                 bin_offset[bin + 1] += 1;
@@ -790,21 +812,18 @@ int upload_mesh(ps_sim* s) {
       }
     }
   }
-  const size_t bt = tri.size() * sizeof(T), bn = nrm.size() * sizeof(T), ba = aabb.size() * sizeof(T);
+  const size_t bt = tri.size() * sizeof(T), ba = aabb.size() * sizeof(T);
   PS_CUDA(cudaMalloc(&s->d_tri, std::max<size_t>(bt, 16)));
-  PS_CUDA(cudaMalloc(&s->d_nrm, std::max<size_t>(bn, 16)));
   PS_CUDA(cudaMalloc(&s->d_aabb, std::max<size_t>(ba, 16)));
   PS_CUDA(cudaMalloc(&s->d_bin_offset, bin_offset.size() * sizeof(uint32_t)));
   PS_CUDA(cudaMalloc(&s->d_bin_tri, std::max<size_t>(bin_tri.size(), 1) * sizeof(uint32_t)));
   PS_CUDA(cudaMalloc(&s->d_mesh_view, sizeof(MeshView)));
   PS_CUDA(cudaMemcpy(s->d_tri, tri.data(), bt, cudaMemcpyHostToDevice));
-  PS_CUDA(cudaMemcpy(s->d_nrm, nrm.data(), bn, cudaMemcpyHostToDevice));
   PS_CUDA(cudaMemcpy(s->d_aabb, aabb.data(), ba, cudaMemcpyHostToDevice));
   PS_CUDA(cudaMemcpy(s->d_bin_offset, bin_offset.data(), bin_offset.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
   if (!bin_tri.empty())
     PS_CUDA(cudaMemcpy(s->d_bin_tri, bin_tri.data(), bin_tri.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
   const MeshView mv{s->d_tri,
-                    s->d_nrm,
                     s->d_aabb,
                     s->d_bin_offset,
                     s->d_bin_tri,
@@ -927,13 +946,21 @@ int size_grids(ps_sim* s, const double* aos) {
       g.n_tri = d.n_tri;
       g.tri_base = tri_base;
       tri_base += d.n_tri;
-      // bin edge: at least one particle cell, at most 128 bins along the longest side
+      // The lists serve radii up to half a grid cell, the largest a later
+      // upload may bring, but not beyond 2.2 r_max (large cells would fill
+      // them with triangles out of reach; mesh_large takes what exceeds it).
+      // Bin edge: at least one sphere, at most 128 bins along the longest side.
+      const double cell = d.cell_size > 0.0 ? d.cell_size : r_max * 2.0 * 1.05;
+      g.mesh_reach = std::min(0.5 * cell, 2.2 * r_max) * 1.0001;
       g.mesh_iv = std::max(r_max * 2.0 * 1.05, ext / 128.0);
       if (!(g.mesh_iv > 0.0)) g.mesh_iv = 1.0;
-      for (int a = 0; a < 3; ++a) {
-        double span = 0.0;
-        for (int64_t k = 0; k < 3 * d.n_tri; ++k) span = std::max(span, soup[3 * k + a] - g.mesh_lo[a]);
-        g.mesh_nb[a] = (int32_t)(span / g.mesh_iv) + 1;
+      double size = 0.0;
+      for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
+      for (int a = 0; a < 3; ++a) {  // room for every centre that can touch the mesh
+        const double room = 1.01 * g.mesh_reach + 1e-5 * size;
+        g.mesh_lo[a] -= room;
+        g.mesh_hi[a] += room;
+        g.mesh_nb[a] = (int32_t)((g.mesh_hi[a] - g.mesh_lo[a]) / g.mesh_iv) + 1;
       }
       g.n_bins = (int64_t)g.mesh_nb[0] * g.mesh_nb[1] * g.mesh_nb[2];
       g.bin_base = bin_base;
@@ -1042,7 +1069,6 @@ void free_sim(ps_sim* s) {
   cudaFree(s->d_scenes);
   cudaFree(s->d_bounds);
   cudaFree(s->d_tri);
-  cudaFree(s->d_nrm);
   cudaFree(s->d_aabb);
   cudaFree(s->d_bin_offset);
   cudaFree(s->d_bin_tri);
@@ -1640,8 +1666,7 @@ namespace {
 int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
-  void** bufs_to_free[] = {&s->cell_arena, &s->d_scenes, &s->d_bounds, &s->d_tri, &s->d_nrm, &s->d_aabb,
-                           &s->adj_arena};
+  void** bufs_to_free[] = {&s->cell_arena, &s->d_scenes, &s->d_bounds, &s->d_tri, &s->d_aabb, &s->adj_arena};
   for (void** b : bufs_to_free) {
     cudaFree(*b);
     *b = nullptr;
