@@ -120,7 +120,15 @@ int ps_get_state(ps_sim* sim, double* aos_out, int64_t n_total);
 
 /* Advance every scene by n_steps steps (the loop body of
  * PhysicsEngineCUDA::startSimulationLoop, PhysicsEngineCUDA.cpp:38-42).
- * Asynchronous on the simulation's stream; blocks of steps run as CUDA graphs. */
+ * Asynchronous on the simulation's stream.  A call of 8 steps or more runs up
+ * to 512 steps per kernel launch, on neighbour lists that the kernel rebuilds
+ * when the motion since the last build requires it (134 bytes per particle,
+ * taken with the first ps_set_state and given up when another allocation of
+ * the simulation needs them).  Shorter calls, simulations without that
+ * memory, and scenes that move too fast for lists to last run as CUDA graphs
+ * of the step kernels, which rebuild the grid in every step.  All give the
+ * same states bit for bit.  The first such call on a simulation's grid waits
+ * for its first five steps, to see which of the two the scene calls for. */
 int ps_step(ps_sim* sim, int64_t n_steps);
 
 /* Wait for the stream and check the device error word. */
@@ -199,6 +207,8 @@ int ps_backward(ps_sim* sim, const double* dl_dstate, ps_grad* grads, double* dl
  * of that scene; f >= 1) and a graph block length L (steps per captured CUDA
  * graph), keeps the fastest pair, and restores the state.  ms_table (may be
  * NULL) receives n_factors x n_blocks milliseconds per step, factor-major.
+ * The trials run the step kernels, to which graph blocks and contact kernels
+ * belong; the chosen cell size holds for every path.
  * The cell size changes the grid and with it the summation order of the
  * contacts, so later trajectories are those of the chosen grid: deterministic,
  * and equal to the oracle's with that cell size, but not bit-equal to runs
@@ -252,7 +262,7 @@ typedef struct ps_tune_result {
 int ps_autotune(ps_sim* sim, int64_t trial_steps, const double* cell_factors, int32_t n_factors,
                 const int64_t* graph_blocks, int32_t n_blocks, double* ms_table, ps_tune_result* out);
 
-/* The contact kernel's neighbour walk.  The reference runs 27 threads per
+/* The neighbour walk of the step kernels' contact kernel.  The reference runs 27 threads per
  * particle, one per neighbour cell (ParticleModel_kernels.cu:136-201,
  * launch :342-372); there is nothing to choose there.  PS_WALK_LANE: each
  * thread loops over its own nine slot ranges (the 27 cells as nine

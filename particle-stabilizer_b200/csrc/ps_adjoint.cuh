@@ -113,7 +113,7 @@ template <class T, bool MULTI>
 __global__ void __launch_bounds__(STEP_THREADS) k_adj_contacts(StepBufs<T> b, AdjBufs<T> a, SceneParams<T> sp0) {
   // one wave of CTAs (occupancy x SMs, the host's choice) loops over the particles
   for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += gridDim.x * STEP_THREADS) {
-    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b.scenes, b.pbase, b.n_scenes);
+    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
     const vec4_t<T> P = b.P0[i];
     const vec4_t<T> V = b.V0[i];
     const uint32_t oi = b.orig[i];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_walls_integrate(StepBufs<T
                                                                       SceneParams<T> sp0) {
   const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
   if (p >= b.n) return;
-  const SceneParams<T>& sp = scene_of<T, MULTI>(p, sp0, b.scenes, b.pbase, b.n_scenes);
+  const SceneParams<T>& sp = scene_of<T, MULTI>(p, sp0, b);
   const uint32_t o = a.tape.o[p];
   vec4_t<T> P = a.tape.p[p];
   vec4_t<T> V = a.tape.v[p];

@@ -24,6 +24,7 @@
 #include "particle_stabilizer_b200.h"
 #include "ps_adjoint.cuh"
 #include "ps_lists.cuh"
+#include "ps_run.cuh"
 #include "ps_scan.cuh"
 #include "ps_stats.cuh"
 #include "ps_step_kernels.cuh"
@@ -146,7 +147,8 @@ struct ps_sim {
   int64_t last_launches = 0;
   std::map<int32_t, void*> checkpoints;  // slot -> device copy of (P0, V1, orig)
   cudaAccessPolicyWindow l2_window{};     // count + offset arrays kept in L2
-  bool l2_window_on = false;
+  bool l2_window_on = false, l2_window_tried = false;
+  size_t cell_bytes = 0;                  // of cell_arena
   size_t l2_limit = 0;                    // persisting set-aside this simulation wants
   size_t l2_prev_limit = 0;               // the context's set-aside before this simulation changed it
   bool l2_limit_set = false;
@@ -169,6 +171,15 @@ struct ps_sim {
   int64_t list_win_steps = 0, list_win_rebuilds = 0, list_backoff = 0, list_backoff_len = 0;
   unsigned list_rebuild_grid = 0;         // CTAs of the cooperative rebuild (one wave)
   unsigned list_step_grid = 0;            // CTAs of the list step kernel (one wave)
+  // the kernel of many steps (ps_run.cuh)
+  uint32_t* d_chunk_scene = nullptr;      // scene of every SCENE_CHUNK-th slot (several scenes only)
+  void* run_arena = nullptr;              // lists, count words, control words
+  unsigned run_grid = 0;                  // CTAs: one wave, or fewer for a small scene
+  bool run_off = false;                   // ps_autotune times the step kernels
+  uint32_t run_id = 0, run_seen = 0;      // runs launched, and the last one whose report was read (run_read)
+  bool run_settled = false;               // what that report said
+  bool run_known = false;                 // a run was launched on this grid
+  int64_t run_backoff = 0, run_backoff_len = 0;  // steps left to the step kernels after an unsettled run
 };
 
 namespace {
@@ -216,6 +227,7 @@ StepBufs<T> bufs(ps_sim* s) {
   b.err = s->err;
   b.scenes = static_cast<const SceneParams<T>*>(s->d_scenes);
   b.pbase = s->d_pbase;
+  b.chunk_scene = s->d_chunk_scene;
   b.n_scenes = s->n_scenes;
   b.n = (uint32_t)s->n_total;
   b.tile_sum = s->tile_sum;
@@ -530,15 +542,43 @@ int regrid(ps_sim* s) {
   return PS_OK;
 }
 
+// Words of the error block: the error bits, the upload check's lowest failing
+// index, and the last run's report (its number, and 1 when most of its steps
+// rebuilt the grid).
+constexpr int ERR_BITS = 0, ERR_BAD = 8, ERR_RUN = 16, ERR_WORDS = 18;
+
+// After a run most of whose steps rebuilt the grid, the next
+// RUN_BACKOFF_MIN steps (doubling up to RUN_BACKOFF_MAX while that repeats)
+// take the step kernels, which pipeline a rebuild better.
+constexpr int64_t RUN_BACKOFF_MIN = 1024, RUN_BACKOFF_MAX = 65536;
+
+void run_read(ps_sim* s, uint32_t run, bool unsettled) {
+  if (run == s->run_seen) return;
+  s->run_seen = run;
+  s->run_settled = !unsettled;
+  s->run_backoff_len = unsettled ? std::min(std::max(2 * s->run_backoff_len, RUN_BACKOFF_MIN), RUN_BACKOFF_MAX) : 0;
+  s->run_backoff = s->run_backoff_len;
+}
+
+// Waits for the stream; reads the error bits and, on the way, the report.
 int check_device_error(ps_sim* s) {
-  uint32_t e = 0;
-  PS_CUDA(cudaMemcpyAsync(&e, s->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
+  uint32_t words[ERR_WORDS] = {};
+  PS_CUDA(cudaMemcpyAsync(words, s->err, sizeof(words), cudaMemcpyDeviceToHost, s->stream));
   PS_CUDA(cudaStreamSynchronize(s->stream));
+  run_read(s, words[ERR_RUN], words[ERR_RUN + 1] != 0u);
+  const uint32_t e = words[ERR_BITS];
   if (e != 0) {
     std::string m = "device error word 0x" + std::to_string(e) + ":";
     if (e & PS_DEVERR_SCAN_TIMEOUT) m += " scan look-back wait expired;";
     if (e & PS_DEVERR_BAD_CELL) m += " cell id outside its scene;";
     if (e & PS_DEVERR_BOUNDS) m += " index out of bounds (bounds-checked build; the access was skipped);";
+    if (e & PS_DEVERR_LIST_BARRIER) {
+      m += " grid barrier wait expired;";
+      // a run left in the middle: its counts and control words
+      cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)n_scan(s), s->stream);
+      cudaMemsetAsync(s->tile_sum, 0, sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), s->stream);
+      if (s->run_arena != nullptr) cudaMemsetAsync(s->run_arena, 0, 256, s->stream);
+    }
     uint32_t zero = 0;
     cudaMemcpyAsync(s->err, &zero, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
     cudaStreamSynchronize(s->stream);
@@ -838,16 +878,21 @@ int upload_mesh(ps_sim* s) {
 // scattered atomics, scattered clears and random offset reads every step,
 // while the particle arrays stream through.  The persisting carve-out is a
 // limit of this process's CUDA context only.
-void setup_l2_window(ps_sim* s, size_t bytes) {
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, s->device) != cudaSuccess) return;
-  if (prop.persistingL2CacheMaxSize <= 0 || prop.accessPolicyMaxWindowSize <= 0) return;
+// Set up by the first call that runs the step kernels.
+void setup_l2_window(ps_sim* s) {
+  if (s->l2_window_tried) return;
+  s->l2_window_tried = true;
+  int max_lines = 0, max_window = 0;
+  if (cudaDeviceGetAttribute(&max_lines, cudaDevAttrMaxPersistingL2CacheSize, s->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, s->device) != cudaSuccess)
+    return;
+  if (max_lines <= 0 || max_window <= 0) return;
   if (std::getenv("PSB200_NO_L2_WINDOW") != nullptr) return;
-  const size_t win = std::min<size_t>(bytes, (size_t)prop.accessPolicyMaxWindowSize);
+  const size_t win = std::min<size_t>(s->cell_bytes, (size_t)max_window);
   size_t cur = 0;
   cudaDeviceGetLimit(&cur, cudaLimitPersistingL2CacheSize);
   if (!s->l2_limit_set) s->l2_prev_limit = cur;
-  const size_t want = std::min<size_t>((size_t)prop.persistingL2CacheMaxSize, win);
+  const size_t want = std::min<size_t>((size_t)max_lines, win);
   if (cur != want && cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, want) != cudaSuccess) {
     cudaGetLastError();
     return;
@@ -899,6 +944,9 @@ void apply_l2_window(ps_sim* s, cudaGraph_t g, bool clear = false) {
   }
   cudaGetLastError();
 }
+
+void run_alloc(ps_sim* s);
+cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes);
 
 // Size every scene's grid from its radii and allocate the per-cell arrays.
 int size_grids(ps_sim* s, const double* aos) {
@@ -1009,7 +1057,7 @@ int size_grids(ps_sim* s, const double* aos) {
   s->offset = reinterpret_cast<uint32_t*>(c + cells_b);
   s->tile_sum = reinterpret_cast<uint32_t*>(c + 2 * cells_b);
   PS_CUDA(cudaMemset(s->cell_arena, 0, 2 * cells_b + tiles_b));
-  setup_l2_window(s, 2 * cells_b + tiles_b);
+  s->cell_bytes = 2 * cells_b + tiles_b;
 
   {
     std::vector<double> iv((size_t)s->n_scenes);
@@ -1040,6 +1088,7 @@ int size_grids(ps_sim* s, const double* aos) {
     if (rc != PS_OK) return rc;
   }
   s->grid_sized = true;
+  if (s->n_total > 0) run_alloc(s);
   return PS_OK;
 }
 
@@ -1049,6 +1098,7 @@ void free_sim(ps_sim* s) {
   cudaFree(s->adj_arena);
   cudaFree(s->list_arena);
   cudaFree(s->list_ckpt);
+  cudaFree(s->run_arena);
   if (s->l2_window_on) {
     cudaStreamAttrValue v{};
     v.accessPolicyWindow.num_bytes = 0;
@@ -1081,7 +1131,7 @@ size_t state_bytes(const ps_sim* s) { return (size_t)(s->precision == PS_FP32 ? 
 
 int save_state(ps_sim* s, void*& buf) {
   const size_t vb = state_bytes(s), ob = 4 * (size_t)s->n_total;
-  if (buf == nullptr) PS_CUDA(cudaMalloc(&buf, std::max<size_t>(2 * vb + ob, 16)));
+  if (buf == nullptr) PS_CUDA(dev_alloc(s, &buf, std::max<size_t>(2 * vb + ob, 16)));
   char* p = static_cast<char*>(buf);
   PS_CUDA(cudaMemcpyAsync(p, s->P0, vb, cudaMemcpyDeviceToDevice, s->stream));
   PS_CUDA(cudaMemcpyAsync(p + vb, s->V1, vb, cudaMemcpyDeviceToDevice, s->stream));
@@ -1199,7 +1249,7 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
     cudaFree(s->adj_arena);
     s->adj_arena = nullptr;
     s->adj_bytes = 0;
-    PS_CUDA(cudaMalloc(&s->adj_arena, need));
+    PS_CUDA(dev_alloc(s, &s->adj_arena, need));
     s->adj_bytes = need;
   }
   char* p = static_cast<char*>(s->adj_arena);
@@ -1324,8 +1374,9 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   const size_t n = (size_t)std::max<int64_t>(s->n_total, 1);
   const size_t b4 = align_up(vb * n, 256), bu = align_up(4 * n, 256), bs = align_up(64 * n, 256);
   const size_t bp = align_up(4 * (size_t)(n_scenes + 1), 256), bi = align_up(8 * (size_t)n_scenes, 256);
+  const size_t chunks = s->multi ? n / SCENE_CHUNK + 2 : 0, bc = align_up(4 * chunks, 256);
   cudaError_t e = cudaMalloc(&s->part_arena,
-                             4 * b4 + 5 * bu + bs + 256 + bp + bi + 2 * sizeof(StatsPartial) * kStatsBlocks + 256);
+                             4 * b4 + 5 * bu + bs + 256 + bp + bi + bc + 2 * sizeof(StatsPartial) * kStatsBlocks + 256);
   if (e != cudaSuccess) {
     delete s;
     return fail(e == cudaErrorMemoryAllocation ? PS_ERR_NOMEM : PS_ERR_CUDA, std::string("ps_create: ") + cudaGetErrorString(e));
@@ -1344,6 +1395,7 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   s->err = reinterpret_cast<uint32_t*>(p); p += 256;
   s->d_pbase = reinterpret_cast<uint32_t*>(p); p += bp;
   s->d_interval = reinterpret_cast<double*>(p); p += bi;
+  s->d_chunk_scene = reinterpret_cast<uint32_t*>(p); p += bc;
   s->d_stats = reinterpret_cast<StatsPartial*>(p); p += sizeof(StatsPartial) * kStatsBlocks;
   s->d_stats_out = reinterpret_cast<StatsPartial*>(p);
   std::vector<uint32_t> pb(n_scenes + 1);
@@ -1351,6 +1403,15 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemcpy(s->d_pbase, pb.data(), 4 * pb.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(s->err, 0, 256);
+  if (e == cudaSuccess && s->multi) {
+    std::vector<uint32_t> cs(chunks);
+    uint32_t sc = 0;
+    for (size_t k = 0; k < chunks; ++k) {  // entries past the last slot hold the last scene
+      while (sc + 1 < (uint32_t)n_scenes && s->pbase[sc + 1] <= (int64_t)(k * SCENE_CHUNK)) ++sc;
+      cs[k] = sc;
+    }
+    e = cudaMemcpy(s->d_chunk_scene, cs.data(), 4 * chunks, cudaMemcpyHostToDevice);
+  }
   if (e != cudaSuccess) {
     free_sim(s);
     delete s;
@@ -1378,7 +1439,7 @@ extern "C" int ps_set_state(ps_sim* s, const double* aos, int64_t n_total) {
     // a later state must fit the grid the first one sized; checked on the
     // device (a host loop over the records cost milliseconds per upload at
     // 1M particles), before the state is replaced
-    uint32_t* bad = s->err + 8;
+    uint32_t* bad = s->err + ERR_BAD;
     uint32_t h_bad = 0;
     PS_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), s->stream));
     k_upload_check<<<g, STEP_THREADS, 0, s->stream>>>(s->staging, s->d_pbase, s->n_scenes, s->d_interval, bad,
@@ -1432,6 +1493,10 @@ namespace {
 // Run n_steps as CUDA graphs of up to graph_block steps (grid path, or the
 // neighbour-list path when `lists`), asynchronously.
 int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
+  if (!lists) {
+    setup_l2_window(s);
+    ensure_l2_limit(s);
+  }
   int64_t left = n_steps;
   while (left > 0) {
     const int64_t L = std::min(left, s->graph_block);
@@ -1465,6 +1530,148 @@ int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
   return PS_OK;
 }
 
+// ---- many steps in one launch ------------------------------------------------
+// Steps a launch covers: a launch starts with a rebuild (0.2 ms at 1M
+// spheres, 1 us a step over 512), and stays below a second or so.
+int64_t run_block(const ps_sim* s) {
+  return std::min<int64_t>(512, std::max<int64_t>(32, (int64_t)2000000000 / std::max<int64_t>(s->n_total, 1)));
+}
+
+// Spheres of one CTA of the run kernel.
+uint32_t run_share(const ps_sim* s) {
+  const int64_t stride = (int64_t)s->run_grid * STEP_THREADS;
+  return (uint32_t)((s->n_total + stride - 1) / stride) * STEP_THREADS;
+}
+
+template <class T>
+RunBufs<T> run_bufs(ps_sim* s) {
+  const size_t n = (size_t)s->n_total;
+  RunBufs<T> R;
+  R.P[0] = static_cast<vec4_t<T>*>(s->P0);
+  R.P[1] = static_cast<vec4_t<T>*>(s->P1);
+  R.V[0] = static_cast<vec4_t<T>*>(s->V0);
+  R.V[1] = static_cast<vec4_t<T>*>(s->V1);
+  char* p = static_cast<char*>(s->run_arena);
+  R.ctl = reinterpret_cast<uint32_t*>(p);
+  p += 256;
+  R.cnt = reinterpret_cast<uint16_t*>(p);
+  p += align_up(2 * n, 256);
+  R.list = reinterpret_cast<uint32_t*>(p);
+  p += align_up(4 * n * RUN_LIST_CAP, 256);
+  R.later = reinterpret_cast<uint32_t*>(p);
+  R.later_stride = run_share(s);
+  R.cap = RUN_LIST_CAP;
+  R.report = s->err + ERR_RUN;
+  return R;
+}
+
+template <class T, bool MULTI, bool MESH>
+int run_prepare(ps_sim* s) {
+  int per_sm = 0, sms = 0;
+  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH>, STEP_THREADS, 0));
+  PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_step: the run kernel cannot be resident");
+  s->run_grid = std::min<unsigned>((unsigned)(per_sm * sms),
+                                   std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
+  return PS_OK;
+}
+
+template <class T, bool MULTI, bool MESH>
+int run_launch(ps_sim* s, uint32_t steps) {
+  const StepBufs<T> b = bufs<T>(s);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(s->run_grid);
+  cfg.blockDim = dim3(STEP_THREADS);
+  cfg.stream = s->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  // the cell arrays are read by rebuilds alone: not the stream's window, which keeps them in L2
+  at[1].id = cudaLaunchAttributeAccessPolicyWindow;
+  at[1].val.accessPolicyWindow = cudaAccessPolicyWindow{};
+  cfg.attrs = at;
+  cfg.numAttrs = s->l2_window_on ? 2 : 1;
+  PS_CUDA(cudaLaunchKernelEx(&cfg, k_run<T, MULTI, MESH>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
+                             run_bufs<T>(s), steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
+                             (uint32_t)move_blocks(s->n_total, 0), ++s->run_id));
+  return PS_OK;
+}
+
+template <class T>
+int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
+  if (s->multi) {
+    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true>(s, steps);
+    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false>(s, steps);
+  }
+  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true>(s, steps);
+  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false>(s, steps);
+}
+
+// The lists' memory (134 B per sphere), unless it would be more than a
+// quarter of what the device has left (asked only where it is large: the
+// question takes as long as the allocation); without it every call takes the
+// step kernels.
+void run_alloc(ps_sim* s) {
+  const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, 0, true) : run_dispatch<double>(s, 0, true);
+  if (rc != PS_OK) return;
+  const size_t n = (size_t)s->n_total;
+  const size_t need = 256 + align_up(2 * n, 256) + align_up(4 * n * RUN_LIST_CAP, 256) +
+                      4 * (size_t)s->run_grid * run_share(s);
+  size_t left = 4 * need, total = 0;
+  if ((need > ((size_t)1 << 30) && cudaMemGetInfo(&left, &total) != cudaSuccess) || need > left / 4 ||
+      cudaMalloc(&s->run_arena, need) != cudaSuccess) {
+    cudaGetLastError();
+    s->run_arena = nullptr;
+    return;
+  }
+  cudaMemsetAsync(s->run_arena, 0, 256, s->stream);
+}
+
+// For the library's own later allocations: the lists give way to them.
+cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && s->run_arena != nullptr) {
+    cudaGetLastError();
+    cudaStreamSynchronize(s->stream);
+    cudaFree(s->run_arena);
+    s->run_arena = nullptr;
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
+// A simulation's first run is of RUN_PROBE_STEPS steps, whose report the
+// call waits for; after a backoff such a probe is followed by the step
+// kernels until a call that waits for the stream anyway has read its report.
+// What a report says only chooses the path; both give the same states.  Five
+// steps tell: two calm ones come before the first lists, and a grid step in
+// the run takes 145 us where the step kernels take 83 us (1M spheres, FP32).
+constexpr int64_t RUN_PROBE_STEPS = 5;
+
+int step_run(ps_sim* s, int64_t n_steps) {
+  for (int64_t left = n_steps; left > 0;) {
+    int64_t L;
+    int rc;
+    const bool waiting = !s->run_settled && s->run_seen != s->run_id;  // a probe is on its way
+    if (s->run_backoff > 0 || waiting) {
+      L = std::min(left, waiting ? RUN_BACKOFF_MIN : s->run_backoff);
+      s->run_backoff = std::max<int64_t>(0, s->run_backoff - L);
+      rc = step_graphs(s, L, false);
+      s->grid_valid = true;
+    } else {
+      L = std::min(left, s->run_settled ? run_block(s) : RUN_PROBE_STEPS);
+      rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, false) : run_dispatch<double>(s, (uint32_t)L, false);
+      s->grid_valid = false;  // the grid arrays are those of the last rebuild
+      s->last_launches += 1;
+      if (rc == PS_OK && !s->run_known && left > L) rc = check_device_error(s);
+      s->run_known = true;
+    }
+    if (rc != PS_OK) return rc;
+    left -= L;
+  }
+  return PS_OK;
+}
+
 // A rebuild costs a few list steps; when a window of at least
 // LIST_BACKOFF_WINDOW list steps rebuilt more often than once per
 // LIST_BACKOFF_RATE steps (a scene moving fast against its skin, or
@@ -1490,7 +1697,7 @@ int step_lists(ps_sim* s, int64_t n_steps) {
         ++it;
       }
     }
-    PS_CUDA(cudaMalloc(&s->list_arena, need));
+    PS_CUDA(dev_alloc(s, &s->list_arena, need));
     s->list_bytes = need;
   }
   if (s->list_rebuild_grid == 0) {
@@ -1593,7 +1800,6 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
   s->last_launches = 0;
   if (n_steps == 0 || s->n_total == 0) return PS_OK;
   DeviceGuard guard(s->device);
-  ensure_l2_limit(s);
   const bool lists = s->list_skin > 0.0;
   int rc = PS_OK;
   int64_t left = n_steps;
@@ -1604,9 +1810,13 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
     s->list_grid_steps += g;
     left -= g;
   }
-  if (rc == PS_OK && left > 0) rc = lists ? step_lists(s, left) : step_graphs(s, left, false);
+  if (!lists && left >= RUN_MIN_STEPS && s->run_arena != nullptr && !s->run_off) {
+    rc = step_run(s, left);
+  } else if (rc == PS_OK && left > 0) {
+    rc = lists ? step_lists(s, left) : step_graphs(s, left, false);
+    s->grid_valid = !lists;  // after the list path the grid arrays do not describe the at-rest state
+  }
   if (rc != PS_OK) return rc;
-  s->grid_valid = !lists;  // after the list path the grid arrays do not describe the at-rest state
   s->stepped = true;
   return PS_OK;
 }
@@ -1617,7 +1827,7 @@ extern "C" int ps_checkpoint_save(ps_sim* s, int32_t slot) {
   DeviceGuard guard(s->device);
   const size_t vb = (s->precision == PS_FP32 ? 16 : 32) * (size_t)s->n_total, ob = 4 * (size_t)s->n_total;
   void*& buf = s->checkpoints[slot];
-  if (buf == nullptr) PS_CUDA(cudaMalloc(&buf, std::max<size_t>(2 * vb + ob, 16)));
+  if (buf == nullptr) PS_CUDA(dev_alloc(s, &buf, std::max<size_t>(2 * vb + ob, 16)));
   char* p = static_cast<char*>(buf);
   PS_CUDA(cudaMemcpyAsync(p, s->P0, vb, cudaMemcpyDeviceToDevice, s->stream));
   PS_CUDA(cudaMemcpyAsync(p + vb, s->V1, vb, cudaMemcpyDeviceToDevice, s->stream));
@@ -1677,8 +1887,13 @@ int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   s->d_bin_offset = s->d_bin_tri = nullptr;
   s->d_mesh_view = nullptr;
   s->adj_bytes = 0;
+  s->run_grid = 0;
+  cudaFree(s->run_arena);
+  s->run_arena = nullptr;
+  s->run_seen = s->run_id;
+  s->run_settled = s->run_known = false;
   s->fwd_steps = 0;
-  s->l2_window_on = false;
+  s->l2_window_on = s->l2_window_tried = false;
   s->grid_sized = false;
   s->grid_valid = false;
   return size_grids(s, host_state.data());
@@ -1699,6 +1914,11 @@ extern "C" int ps_autotune(ps_sim* s, int64_t trial_steps, const double* cell_fa
   for (int32_t l = 0; l < n_blocks; ++l)
     if (graph_blocks[l] < 1) return fail(PS_ERR_INVALID, "ps_autotune: graph blocks must be >= 1");
   DeviceGuard guard(s->device);
+  struct StepKernelsOnly {  // the trials time the step kernels
+    ps_sim* s;
+    explicit StepKernelsOnly(ps_sim* sim) : s(sim) { s->run_off = true; }
+    ~StepKernelsOnly() { s->run_off = false; }
+  } step_kernels_only(s);
   // the starting state, on the host (radii for the cell sizes) and on the device
   std::vector<double> host((size_t)8 * (size_t)std::max<int64_t>(s->n_total, 1));
   int rc = ps_get_state(s, host.data(), s->n_total);
@@ -1884,6 +2104,8 @@ extern "C" int ps_profile_steps(ps_sim* s, int64_t n_steps, double* kernel_ms, i
   }
   if (s->n_total == 0) return PS_OK;
   DeviceGuard guard(s->device);
+  setup_l2_window(s);
+  ensure_l2_limit(s);
   std::vector<LaunchRecord> rec((size_t)(1 + 4 * n_steps));
   for (auto& r : rec) {
     PS_CUDA(cudaEventCreate(&r.a));
@@ -1920,6 +2142,11 @@ extern "C" int ps_forward_checkpointed(ps_sim* s, int64_t n_steps, int64_t every
   for (int64_t blk = 0; blk < n_blocks; ++blk) {
     int rc = save_state(s, s->fwd_ckpt[(size_t)blk]);
     if (rc == PS_OK) rc = ps_step(s, std::min(every, n_steps - blk * every));
+    // The backward pass hands its adjoints from block to block by slot: a
+    // checkpoint is in the order of the grid of its own positions, which is
+    // the order in which recomputing the block before it ends.  Runs and
+    // lists leave the order of an earlier grid.
+    if (rc == PS_OK && !s->grid_valid) rc = regrid(s);
     if (rc != PS_OK) return rc;
   }
   int rc = save_state(s, s->fwd_ckpt.back());
@@ -1938,6 +2165,7 @@ extern "C" int ps_backward(ps_sim* s, const double* dl_dstate, ps_grad* grads, d
     return PS_OK;
   }
   DeviceGuard guard(s->device);
+  setup_l2_window(s);
   ensure_l2_limit(s);
   if (s->precision == PS_FP32)
     return s->multi ? backward_impl<float, true>(s, dl_dstate, grads, dl_dstate0)

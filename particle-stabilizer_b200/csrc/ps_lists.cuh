@@ -88,7 +88,7 @@ __device__ __forceinline__ void axis_span(T x, T reach, T lo, T iv, int32_t nb, 
 template <class T, bool MULTI, bool COH>
 __device__ __forceinline__ void list_build_one(uint32_t i, const StepBufs<T>& b, const SceneParams<T>& sp0,
                                                const ListBufs<T>& L, int dst) {
-  const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b.scenes, b.pbase, b.n_scenes);
+  const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
   const vec4_t<T> P = b.P0[i];
   L.P[dst][i] = P;
   L.V[dst][i] = b.V0[i];
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 3)
   const bool valid = i < b.n;
   bool moved = false;
   if (valid) {
-    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b.scenes, b.pbase, b.n_scenes);
+    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
     const vec4_t<T>* __restrict__ Ps = L.P[src];
     vec4_t<T> P = Ps[i];
     const vec4_t<T> Vi = L.V[src][i];

@@ -241,4 +241,23 @@ __device__ __forceinline__ void mesh_contacts(vec4_t<T>& P, vec4_t<T>& V, const 
   P.z = A::add(c.z, m.x.z);
 }
 
+// Whether a sphere at P may touch a triangle once each of its coordinates
+// has moved by up to `skin`: its plane and its box both within that reach.
+template <class T>
+__device__ __forceinline__ bool mesh_within(const vec4_t<T>& P, T skin, const SceneParams<T>& sp, const MeshView& mv,
+                                            uint32_t* err) {
+  if (!(P.w <= sp.mesh_reach)) return true;
+  const T reach = P.w + skin, along = (P.w + T(1.75) * skin) * T(1.001);  // sqrt(3) skin along a normal
+  const V3<T> lo = {P.x - reach, P.y - reach, P.z - reach}, hi = {P.x + reach, P.y + reach, P.z + reach};
+  bool found = false;
+  mesh_bins<T>({P.x - skin, P.y - skin, P.z - skin}, {P.x + skin, P.y + skin, P.z + skin}, sp, mv, err,
+               [&](uint32_t t) {
+                 if (found || !in_box<T>(mv, t, lo, hi)) return;
+                 const Triangle<T> g = triangle<T>(mv, t);
+                 const T h = (P.x - g.a.x) * g.n.x + (P.y - g.a.y) * g.n.y + (P.z - g.a.z) * g.n.z;
+                 found = !(fabs(h) > along);  // a triangle without a normal counts
+               });
+  return found;
+}
+
 }  // namespace psb

@@ -77,7 +77,7 @@ struct RunBufs {
   uint16_t* cnt;
   uint32_t* later;      // per CTA: slots that the step takes after the others (run_late)
   uint32_t* ctl;
-  volatile uint64_t* report;  // host memory: (run << 32) | unsettled, written when a run ends
+  uint32_t* report;     // number of the last run, and whether most of its steps rebuilt the grid
   uint32_t cap;
   uint32_t later_stride;  // entries of `later` per CTA
   __device__ __forceinline__ vec4_t<T>* p(int k) const { return k ? P[1] : P[0]; }
@@ -684,7 +684,8 @@ __global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 2)
   if (blockIdx.x == 0 && threadIdx.x == 3u) R.ctl[RUN_RMAX] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0u) {
     R.ctl[RUN_STREAK] = streak;
-    *R.report = ((uint64_t)run_id << 32) | (2u * unsettled > steps ? 1u : 0u);
+    R.report[0] = run_id;
+    R.report[1] = 2u * unsettled > steps ? 1u : 0u;
   }
 }
 

@@ -29,23 +29,7 @@
 namespace psb {
 
 constexpr int STEP_THREADS = 256;
-
-// ---- scene lookup ------------------------------------------------------------
-template <class T, bool MULTI>
-__device__ __forceinline__ const SceneParams<T>& scene_of(uint32_t p, const SceneParams<T>& sp0,
-                                                          const SceneParams<T>* sps, const uint32_t* pbase,
-                                                          int n_scenes) {
-  if (!MULTI) return sp0;
-  int lo = 0, hi = n_scenes - 1;  // largest s with pbase[s] <= p
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(pbase + mid) <= p)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return sps[lo];
-}
+constexpr uint32_t SCENE_CHUNK = 256;
 
 // ---- cell hashing (ParticleModel_kernels.cu:42-73) ---------------------------
 // Per-axis index (int)((x - lo) / interval), clamped to [0, nb-1]; NaN and
@@ -163,6 +147,7 @@ struct StepBufs {
   uint32_t* err;
   const SceneParams<T>* scenes;
   const uint32_t* pbase;  // n_scenes entries
+  const uint32_t* chunk_scene;  // scene of every SCENE_CHUNK-th slot, one entry past the last
   int32_t n_scenes;
   uint32_t n;             // particles over all scenes
   uint32_t* tile_sum;     // per-tile totals of `count`, cleared by k_scatter
@@ -180,6 +165,24 @@ struct StepBufs {
   uint32_t* tape_o;
   uint32_t* tape_cell;
 };
+
+// ---- scene lookup ------------------------------------------------------------
+// Scene of slot p: the largest s with pbase[s] <= p.  chunk_scene[k] is the
+// scene of slot SCENE_CHUNK k, so the search runs between the scenes at the
+// two ends of p's chunk, which are nearly always the same one.
+template <class T, bool MULTI>
+__device__ __forceinline__ const SceneParams<T>& scene_of(uint32_t p, const SceneParams<T>& sp0, const StepBufs<T>& b) {
+  if (!MULTI) return sp0;
+  uint32_t lo = __ldg(b.chunk_scene + p / SCENE_CHUNK), hi = __ldg(b.chunk_scene + p / SCENE_CHUNK + 1);
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (__ldg(b.pbase + mid) <= p)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return b.scenes[lo];
+}
 
 // Container step + hash + count on an integrated state, shared by k_begin and
 // the fused epilogue of k_contacts.
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_begin(StepBufs<T> b, ScenePara
   uint32_t c = 0;
   pdl_wait();
   if (valid) {
-    const SceneParams<T>& sp = scene_of<T, MULTI>(p, sp0, b.scenes, b.pbase, b.n_scenes);
+    const SceneParams<T>& sp = scene_of<T, MULTI>(p, sp0, b);
     vec4_t<T> P = b.P0[p];
     vec4_t<T> V = b.V1[p];
     if (INTEGRATE) {
@@ -375,30 +378,45 @@ __global__ void __launch_bounds__(STEP_THREADS) k_rank_move(StepBufs<T> b) {
 // then d2 > s*s, so sqrt(d2) > s and, rounding being monotonic,
 // sqrt_rn(d2) >= s.  The filter therefore rejects only pairs the exact test
 // rejects, and the result stays bit-identical.
-// Contribution of neighbour j (position Pj) to particle i's velocity.
+// f of an overlapping pair: particle i's velocity changes by f d, d = x_i - x_j.
 template <class T>
-__device__ __forceinline__ void contact_one(const vec4_t<T>* __restrict__ V0, uint32_t j, const vec4_t<T>& P,
-                                            const vec4_t<T>& Vi, const vec4_t<T>& Pj, T k, T e, T& vx, T& vy,
-                                            T& vz) {
+__device__ __forceinline__ T contact_force(const vec4_t<T>& Vi, const vec4_t<T>& Vj, T dx, T dy, T dz, T d2, T dist,
+                                           T overlap, T k, T e) {
+  using A = Ar<T>;
+  const T rvx = A::sub(Vi.x, Vj.x), rvy = A::sub(Vi.y, Vj.y), rvz = A::sub(Vi.z, Vj.z);
+  const T rvd = A::fma(rvz, dz, A::fma(rvy, dy, A::mul(rvx, dx)));
+  const T cr = A::div(A::mul(A::mul(A::mul(T(2), Vj.w), rvd), e), A::mul(A::add(Vi.w, Vj.w), d2));
+  const T cs = A::div(A::mul(k, overlap), A::mul(dist, Vi.w));
+  return A::sub(cs, cr);
+}
+
+// Contribution of neighbour j (position Pj) to particle i's velocity; true if
+// they overlap.  COH: inside a kernel that writes V0 itself (plain load), and
+// the sign of a radius word is a mark, not part of the radius (ps_run.cuh).
+template <class T, bool COH = false>
+__device__ __forceinline__ bool contact_one(const vec4_t<T>* V0, uint32_t j, const vec4_t<T>& P, const vec4_t<T>& Vi,
+                                            const vec4_t<T>& Pj, T k, T e, T& vx, T& vy, T& vz) {
   using A = Ar<T>;
   const T margin = T(1) + T(1.0 / 1048576.0);
   const T dx = A::sub(P.x, Pj.x), dy = A::sub(P.y, Pj.y), dz = A::sub(P.z, Pj.z);
   const T d2 = A::fma(dz, dz, A::fma(dy, dy, A::mul(dx, dx)));
-  const T s = A::add(P.w, Pj.w);
-  if (d2 >= A::mul(A::mul(s, s), margin)) return;
+  const T s = COH ? A::add(fabs(P.w), fabs(Pj.w)) : A::add(P.w, Pj.w);
+  if (d2 >= A::mul(A::mul(s, s), margin)) return false;
   const T dist = A::sqrt(d2);
   const T overlap = A::sub(s, dist);
-  if (overlap > T(0)) {
-    const vec4_t<T> Vj = ld4<T>(V0 + j);
-    const T rvx = A::sub(Vi.x, Vj.x), rvy = A::sub(Vi.y, Vj.y), rvz = A::sub(Vi.z, Vj.z);
-    const T rvd = A::fma(rvz, dz, A::fma(rvy, dy, A::mul(rvx, dx)));
-    const T cr = A::div(A::mul(A::mul(A::mul(T(2), Vj.w), rvd), e), A::mul(A::add(Vi.w, Vj.w), d2));
-    const T cs = A::div(A::mul(k, overlap), A::mul(dist, Vi.w));
-    const T f = A::sub(cs, cr);
+  const bool touch = overlap > T(0);
+  if (touch) {
+    vec4_t<T> Vj;
+    if constexpr (COH)
+      Vj = V0[j];
+    else
+      Vj = ld4<T>(V0 + j);
+    const T f = contact_force<T>(Vi, Vj, dx, dy, dz, d2, dist, overlap, k, e);
     vx = A::fma(f, dx, vx);
     vy = A::fma(f, dy, vy);
     vz = A::fma(f, dz, vz);
   }
+  return touch;
 }
 
 // Cell coordinates of a sorted slot from its global cell id.
@@ -600,7 +618,7 @@ __global__ void __launch_bounds__(BLOCK, contact_min_blocks<T, BLOCK>()) k_conta
   pdl_wait();
   // Lanes past the end walk empty ranges: the warp's shuffles and the
   // count's ballot need every lane.
-  const SceneParams<T>& sp = scene_of<T, MULTI>(valid ? i : 0u, sp0, b.scenes, b.pbase, b.n_scenes);
+  const SceneParams<T>& sp = scene_of<T, MULTI>(valid ? i : 0u, sp0, b);
   vec4_t<T> P, Vi;
   uint32_t my_cell = sp.cbase;
   if (valid) {
