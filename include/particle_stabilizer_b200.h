@@ -122,13 +122,13 @@ int ps_get_state(ps_sim* sim, double* aos_out, int64_t n_total);
  * PhysicsEngineCUDA::startSimulationLoop, PhysicsEngineCUDA.cpp:38-42).
  * Asynchronous on the simulation's stream.  A call of 8 steps or more runs up
  * to 512 steps per kernel launch, on neighbour lists that the kernel rebuilds
- * when the motion since the last build requires it (134 bytes per particle,
+ * when the motion since the last build requires it (134 to 198 bytes per particle,
  * taken with the first ps_set_state and given up when another allocation of
  * the simulation needs them).  Shorter calls, simulations without that
  * memory, and scenes that move too fast for lists to last run as CUDA graphs
  * of the step kernels, which rebuild the grid in every step.  All give the
  * same states bit for bit.  The first such call on a simulation's grid waits
- * for its first five steps, to see which of the two the scene calls for. */
+ * for its first six steps, to see which of the two the scene calls for. */
 int ps_step(ps_sim* sim, int64_t n_steps);
 
 /* Wait for the stream and check the device error word. */

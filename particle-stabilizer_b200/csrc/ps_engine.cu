@@ -175,6 +175,7 @@ struct ps_sim {
   uint32_t* d_chunk_scene = nullptr;      // scene of every SCENE_CHUNK-th slot (several scenes only)
   void* run_arena = nullptr;              // lists, count words, control words
   unsigned run_grid = 0;                  // CTAs: one wave, or fewer for a small scene
+  bool run_own = false;                   // those CTAs have a thread for every sphere
   bool run_off = false;                   // ps_autotune times the step kernels
   uint32_t run_id = 0, run_seen = 0;      // runs launched, and the last one whose report was read (run_read)
   bool run_settled = false;               // what that report said
@@ -543,11 +544,11 @@ int regrid(ps_sim* s) {
 }
 
 // Words of the error block: the error bits, the upload check's lowest failing
-// index, and the last run's report (its number, and 1 when most of its steps
-// rebuilt the grid).
+// index, and the last run's report (its number, and 1 when it rebuilt the
+// grid in more than every fourth step; of a short run, in every second).
 constexpr int ERR_BITS = 0, ERR_BAD = 8, ERR_RUN = 16, ERR_WORDS = 18;
 
-// After a run most of whose steps rebuilt the grid, the next
+// After a run that rebuilt so often, the next
 // RUN_BACKOFF_MIN steps (doubling up to RUN_BACKOFF_MAX while that repeats)
 // take the step kernels, which pipeline a rebuild better.
 constexpr int64_t RUN_BACKOFF_MIN = 1024, RUN_BACKOFF_MAX = 65536;
@@ -1560,6 +1561,8 @@ RunBufs<T> run_bufs(ps_sim* s) {
   p += align_up(4 * n * RUN_LIST_CAP, 256);
   R.later = reinterpret_cast<uint32_t*>(p);
   R.later_stride = run_share(s);
+  p += align_up(4 * (size_t)s->run_grid * R.later_stride, 256);
+  R.tris = s->has_mesh ? reinterpret_cast<uint32_t*>(p) : nullptr;
   R.cap = RUN_LIST_CAP;
   R.report = s->err + ERR_RUN;
   return R;
@@ -1568,8 +1571,11 @@ RunBufs<T> run_bufs(ps_sim* s) {
 template <class T, bool MULTI, bool MESH>
 int run_prepare(ps_sim* s) {
   int per_sm = 0, sms = 0;
-  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH>, STEP_THREADS, 0));
   PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, true>, STEP_THREADS, 0));
+  s->run_own = (int64_t)blocks_for(s->n_total) <= (int64_t)per_sm * sms;
+  if (!s->run_own)
+    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, false>, STEP_THREADS, 0));
   if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_step: the run kernel cannot be resident");
   s->run_grid = std::min<unsigned>((unsigned)(per_sm * sms),
                                    std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
@@ -1591,7 +1597,7 @@ int run_launch(ps_sim* s, uint32_t steps) {
   at[1].val.accessPolicyWindow = cudaAccessPolicyWindow{};
   cfg.attrs = at;
   cfg.numAttrs = s->l2_window_on ? 2 : 1;
-  PS_CUDA(cudaLaunchKernelEx(&cfg, k_run<T, MULTI, MESH>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
+  PS_CUDA(cudaLaunchKernelEx(&cfg, s->run_own ? k_run<T, MULTI, MESH, true> : k_run<T, MULTI, MESH, false>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
                              run_bufs<T>(s), steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
                              (uint32_t)move_blocks(s->n_total, 0), ++s->run_id));
   return PS_OK;
@@ -1607,7 +1613,7 @@ int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
   return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false>(s, steps);
 }
 
-// The lists' memory (134 B per sphere), unless it would be more than a
+// The lists' memory (134 B per sphere, 198 B with triangles), unless it would be more than a
 // quarter of what the device has left (asked only where it is large: the
 // question takes as long as the allocation); without it every call takes the
 // step kernels.
@@ -1616,7 +1622,7 @@ void run_alloc(ps_sim* s) {
   if (rc != PS_OK) return;
   const size_t n = (size_t)s->n_total;
   const size_t need = 256 + align_up(2 * n, 256) + align_up(4 * n * RUN_LIST_CAP, 256) +
-                      4 * (size_t)s->run_grid * run_share(s);
+                      align_up(4 * (size_t)s->run_grid * run_share(s), 256) + (s->has_mesh ? 4 * n * RUN_TRI_CAP : 0);
   size_t left = 4 * need, total = 0;
   if ((need > ((size_t)1 << 30) && cudaMemGetInfo(&left, &total) != cudaSuccess) || need > left / 4 ||
       cudaMalloc(&s->run_arena, need) != cudaSuccess) {
@@ -1643,10 +1649,11 @@ cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes) {
 // A simulation's first run is of RUN_PROBE_STEPS steps, whose report the
 // call waits for; after a backoff such a probe is followed by the step
 // kernels until a call that waits for the stream anyway has read its report.
-// What a report says only chooses the path; both give the same states.  Five
-// steps tell: two calm ones come before the first lists, and a grid step in
-// the run takes 145 us where the step kernels take 83 us (1M spheres, FP32).
-constexpr int64_t RUN_PROBE_STEPS = 5;
+// What a report says only chooses the path; both give the same states.  Six
+// steps tell (a sphere pushed out of a wall, two calm steps to the first
+// lists, two on them), and a grid step in the run takes 145 us where the step
+// kernels take 83 us (1M spheres, FP32).
+constexpr int64_t RUN_PROBE_STEPS = 6;
 
 int step_run(ps_sim* s, int64_t n_steps) {
   for (int64_t left = n_steps; left > 0;) {

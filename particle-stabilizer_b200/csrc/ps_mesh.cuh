@@ -209,6 +209,22 @@ __device__ __noinline__ void mesh_large(V3<T> c, T r, vec4_t<T> V, const ScenePa
   }
 }
 
+// The container's effect on a sphere at c, once its hits are summed.
+template <class T>
+__device__ __forceinline__ void mesh_apply(const MeshSums<T>& m, const V3<T>& c, vec4_t<T>& P, vec4_t<T>& V) {
+  using A = Ar<T>;
+  if (m.hits > 0) {  // calcAveragedVelocityKernel: only particles with a hit
+    const T hc = (T)m.hits;
+    V.x = A::div(m.v.x, hc);
+    V.y = A::div(m.v.y, hc);
+    V.z = A::div(m.v.z, hc);
+  }
+  // modifyPositionKernel adds the (possibly zero) correction to every particle
+  P.x = A::add(c.x, m.x.x);
+  P.y = A::add(c.y, m.x.y);
+  P.z = A::add(c.z, m.x.z);
+}
+
 // Triangle container of one particle, CUDA semantics
 // (PolygonContainerCUDA.cpp:130-226): every hit triangle in ascending index.
 template <class T>
@@ -229,35 +245,34 @@ __device__ __forceinline__ void mesh_contacts(vec4_t<T>& P, vec4_t<T>& V, const 
   } else {
     mesh_large<T>(c, r, V, sp, mv, err, &m);
   }
-  if (m.hits > 0) {  // calcAveragedVelocityKernel: only particles with a hit
-    const T hc = (T)m.hits;
-    V.x = A::div(m.v.x, hc);
-    V.y = A::div(m.v.y, hc);
-    V.z = A::div(m.v.z, hc);
-  }
-  // modifyPositionKernel adds the (possibly zero) correction to every particle
-  P.x = A::add(c.x, m.x.x);
-  P.y = A::add(c.y, m.x.y);
-  P.z = A::add(c.z, m.x.z);
+  mesh_apply<T>(m, c, P, V);
 }
 
-// Whether a sphere at P may touch a triangle once each of its coordinates
-// has moved by up to `skin`: its plane and its box both within that reach.
-template <class T>
-__device__ __forceinline__ bool mesh_within(const vec4_t<T>& P, T skin, const SceneParams<T>& sp, const MeshView& mv,
-                                            uint32_t* err) {
-  if (!(P.w <= sp.mesh_reach)) return true;
+// Ascending ids of the triangles that a sphere at P may touch once each of
+// its coordinates has moved by up to `skin` (plane and box within reach), at
+// most CAP of them; the count, or more than CAP when they are not all there.
+template <class T, int CAP>
+__device__ __forceinline__ uint32_t mesh_candidates(const vec4_t<T>& P, T skin, const SceneParams<T>& sp,
+                                                    const MeshView& mv, uint32_t* err, uint32_t (&ids)[CAP]) {
+  if (!(P.w <= sp.mesh_reach)) return CAP + 1;
   const T reach = P.w + skin, along = (P.w + T(1.75) * skin) * T(1.001);  // sqrt(3) skin along a normal
   const V3<T> lo = {P.x - reach, P.y - reach, P.z - reach}, hi = {P.x + reach, P.y + reach, P.z + reach};
-  bool found = false;
+  uint32_t n = 0;
   mesh_bins<T>({P.x - skin, P.y - skin, P.z - skin}, {P.x + skin, P.y + skin, P.z + skin}, sp, mv, err,
                [&](uint32_t t) {
-                 if (found || !in_box<T>(mv, t, lo, hi)) return;
+                 if (n > CAP || !in_box<T>(mv, t, lo, hi)) return;
                  const Triangle<T> g = triangle<T>(mv, t);
                  const T h = (P.x - g.a.x) * g.n.x + (P.y - g.a.y) * g.n.y + (P.z - g.a.z) * g.n.z;
-                 found = !(fabs(h) > along);  // a triangle without a normal counts
+                 if (fabs(h) > along) return;  // (a triangle without a normal stays)
+                 uint32_t k = n;  // several bins: not in order, and not once
+                 while (k > 0u && ids[k - 1] > t) --k;
+                 if (k > 0u && ids[k - 1] == t) return;
+                 if (n < CAP)
+                   for (uint32_t q = n; q > k; --q) ids[q] = ids[q - 1];
+                 if (n < CAP) ids[k] = t;
+                 ++n;
                });
-  return found;
+  return n;
 }
 
 }  // namespace psb

@@ -27,12 +27,15 @@
 //     spheres do not compute a cell at all.
 //   * A sphere with more than the list's capacity of neighbours walks the
 //     cells of the last build instead (run_slow).
+//   * In a triangle container a build also lists the triangles that a sphere
+//     may come to touch; one that moves a good part of the skin at once walks
+//     its bin.
 //
 // When the fastest sphere moves more than RUN_CALM_MAX cells in a step, or
-// did within the last RUN_CALM_STEPS steps, no list would last: such a step
-// rebuilds the grid and walks the 27 cells, like the step kernels.  The skin
-// of a build follows from the speed, so that a build lasts about
-// RUN_STEPS_PER_BUILD steps.
+// did within the last RUN_CALM_STEPS steps, no list would last two steps,
+// below which it does not pay: such a step rebuilds the grid and walks the 27
+// cells, like the step kernels.  The skin of a build follows from the speed,
+// so that a build lasts about RUN_STEPS_PER_BUILD steps.
 //
 // What bounds it: a list step moves 66 B per sphere in FP32 (position and
 // velocity in and out, one 2-byte count), mostly through L2 up to a million
@@ -46,20 +49,22 @@ namespace psb {
 
 constexpr int RUN_MIN_STEPS = 8;
 constexpr uint32_t RUN_LIST_CAP = 32;
-constexpr float RUN_CALM_MAX = 0.02f;
+constexpr float RUN_CALM_MAX = 0.05f;
 constexpr uint32_t RUN_CALM_STEPS = 2;
 constexpr float RUN_STEPS_PER_BUILD = 64.0f;
 constexpr float RUN_SKIN_MIN = 0.02f, RUN_SKIN_MAX = 0.25f;
 
 // count word of a sphere: list length and what its step needs besides
 enum : uint32_t {
-  RUN_COUNT = 0x1fffu,
-  RUN_NEAR_MESH = 1u << 13,  // a triangle may come within reach before the next build
-  RUN_OVERFLOW = 1u << 14,   // more neighbours than the list holds
-  RUN_NEAR_FACE = 1u << 15,  // may leave its cell before the next build
+  RUN_COUNT = 0x3fu,
+  RUN_NEAR_FACE = 1u << 6,  // may leave its cell before the next build
+  RUN_OVERFLOW = 1u << 7,   // more neighbours than the list holds
+  RUN_TRIS = 8,             // shift: triangles that may come within reach, RUN_TRI_MANY if not all are listed
 };
+constexpr int RUN_TRI_CAP = 16;
+constexpr uint32_t RUN_TRI_MANY = RUN_TRI_CAP + 1;
 constexpr uint32_t RUN_FAR_CELL = 0x80000000u;  // list entry: cells not adjacent at the build
-static_assert(RUN_LIST_CAP <= RUN_COUNT, "list length fits the count word");
+static_assert(RUN_LIST_CAP <= 32 && RUN_LIST_CAP <= RUN_COUNT, "a list is at most an entry per lane, its length fits the word");
 
 // control words
 enum : int {
@@ -67,6 +72,7 @@ enum : int {
   RUN_MAXD = 2,     // largest squared displacement of a step, in cells (3 words, by step)
   RUN_STREAK = 5,   // calm steps up to now
   RUN_RMAX = 6,     // largest radius, in cells of its scene
+  RUN_BEFORE = 7,   // largest displacement of the last step, in cells (0: none yet)
 };
 
 template <class T>
@@ -75,9 +81,10 @@ struct RunBufs {
   vec4_t<T>* V[2];
   uint32_t* list;       // [k][slot]
   uint16_t* cnt;
-  uint32_t* later;      // per CTA: slots that the step takes after the others (run_late)
+  uint32_t* tris;       // [k][slot]: triangles within reach (triangle containers)
+  uint32_t* later;      // per CTA: the slots of its RunLate beyond what fits in shared memory
   uint32_t* ctl;
-  uint32_t* report;     // number of the last run, and whether most of its steps rebuilt the grid
+  uint32_t* report;     // number of the last run, and whether it rebuilt too often
   uint32_t cap;
   uint32_t later_stride;  // entries of `later` per CTA
   __device__ __forceinline__ vec4_t<T>* p(int k) const { return k ? P[1] : P[0]; }
@@ -96,22 +103,21 @@ __device__ __forceinline__ bool run_barrier(uint32_t* ctl, uint32_t* err) {
   if (threadIdx.x == 0) {
     int ok = 1;
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(ctl + RUN_BAR);
-    __threadfence();
-    const unsigned long long ticket = atomicAdd(bar, 1ull);
-    const unsigned long long target = (ticket / gridDim.x + 1ull) * gridDim.x;
-    uint32_t spins = 0;
-    unsigned long long seen = ticket + 1ull;
-    while (seen < target) {
+    unsigned long long seen;
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");  // the CTA's writes, gathered by the barrier above
+    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], 1;" : "=l"(seen) : "l"(bar) : "memory");
+    const unsigned long long target = (seen / gridDim.x + 1ull) * gridDim.x;
+    ++seen;
+    for (uint32_t spins = 0; seen < target; ++spins) {
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(bar) : "memory");
-      if (seen >= target) break;
-      if (++spins == RUN_BARRIER_SPIN_LIMIT) {
+      if (spins == RUN_BARRIER_SPIN_LIMIT) {
         atomicOr(err, PS_DEVERR_LIST_BARRIER);
         ok = 0;
         break;
       }
-      __nanosleep(20);
+      if (spins >= 64u) __nanosleep(64);
     }
-    __threadfence();
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
     s_ok = ok;
   }
   __syncthreads();
@@ -253,7 +259,12 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
       if (!inner) word |= RUN_NEAR_FACE;
     }
     if constexpr (MESH) {
-      if (sp.mesh_tris > 0 && mesh_within<T>(P, skin, sp, *mv, b.err)) word |= RUN_NEAR_MESH;
+      if (sp.mesh_tris > 0) {
+        uint32_t ids[RUN_TRI_CAP];
+        const uint32_t nt = min(mesh_candidates<T, RUN_TRI_CAP>(P, skin, sp, *mv, b.err, ids), RUN_TRI_MANY);
+        for (uint32_t q = 0; q < nt && nt <= RUN_TRI_CAP; ++q) R.tris[(size_t)q * b.n + i] = ids[q];
+        word |= nt << RUN_TRIS;
+      }
     }
   }
   if (k > R.cap) word |= RUN_OVERFLOW, k = 0;
@@ -264,14 +275,14 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
 // partners whose cell is adjacent now, by ascending (cell now, original
 // index).  Every lane of the warp calls it with the same sphere.
 //
-// The lanes take the list's entries side by side, each forms its pair's key
-// and force, and the forces are added in the order of the keys.  With the
+// The lanes take the list's entries (`mine`) side by side, each forms its
+// pair's key and force, and the forces are added in the order of the keys.  With the
 // list overflowed the candidates are those of the cells of the last build,
 // and the smallest key above the last one is looked for in turn.
 template <class T>
-__device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, const StepBufs<T>& b,
-                                              const SceneParams<T>& sp, const RunBufs<T>& R, const vec4_t<T>* Ps,
-                                              const vec4_t<T>* Vs, T frac, const vec4_t<T>& P, const vec4_t<T>& Vi) {
+__device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_t mine, const StepBufs<T>& b,
+                                              const SceneParams<T>& sp, const vec4_t<T>* Ps, const vec4_t<T>* Vs,
+                                              T frac, const vec4_t<T>& P, const vec4_t<T>& Vi) {
   using A = Ar<T>;
   const unsigned lane = threadIdx.x & 31u;
   vec4_t<T> V = Vi;
@@ -282,7 +293,8 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, const S
   T f = T(0), dx = T(0), dy = T(0), dz = T(0);
   auto key_of = [&](uint32_t j) -> uint64_t {
     if (j == i) return NONE;
-    const vec4_t<T> Q = Ps[j];
+    const vec4_t<T> Q = Ps[j], W = Vs[j];  // (all three loads before the test)
+    const uint32_t oj = b.orig[j];
     const T margin = T(1) + T(1.0 / 1048576.0);
     dx = A::sub(P.x, Q.x), dy = A::sub(P.y, Q.y), dz = A::sub(P.z, Q.z);
     const T d2 = A::fma(dz, dz, A::fma(dy, dy, A::mul(dx, dx)));
@@ -294,16 +306,14 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, const S
     int32_t jx, jy, jz;
     const uint32_t cj = cell_of<T>(Q.x, Q.y, Q.z, sp, jx, jy, jz);
     if (abs(jx - cx) > 1 || abs(jy - cy) > 1 || abs(jz - cz) > 1) return NONE;
-    f = contact_force<T>(Vi, Vs[j], dx, dy, dz, d2, dist, overlap, sp.k_spring, sp.e_sphere);
-    return ((uint64_t)cj << 32) | (uint64_t)b.orig[j];
+    f = contact_force<T>(Vi, W, dx, dy, dz, d2, dist, overlap, sp.k_spring, sp.e_sphere);
+    return ((uint64_t)cj << 32) | (uint64_t)oj;
   };
   auto smallest = [&](uint64_t key) -> uint64_t {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const uint64_t t = __shfl_xor_sync(0xffffffffu, key, d);
-      key = t < key ? t : key;
-    }
-    return key;
+    const uint32_t cell = (uint32_t)(key >> 32);
+    const uint32_t c = __reduce_min_sync(0xffffffffu, cell);
+    const uint32_t o = __reduce_min_sync(0xffffffffu, cell == c ? (uint32_t)key : 0xffffffffu);
+    return ((uint64_t)c << 32) | (uint64_t)o;
   };
   auto apply = [&](int from) {
     const T g = __shfl_sync(0xffffffffu, f, from);
@@ -312,12 +322,7 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, const S
     V.z = A::fma(g, __shfl_sync(0xffffffffu, dz, from), V.z);
   };
   if (!(word & RUN_OVERFLOW)) {
-    static_assert(RUN_LIST_CAP <= 32, "a list is one entry per lane");
-    uint64_t key = NONE;
-    if (lane < (word & RUN_COUNT)) {
-      const uint32_t j = R.list[(size_t)lane * b.n + i] & ~RUN_FAR_CELL;
-      if (in_bounds(j, b.n, b.err)) key = key_of(j);
-    }
+    uint64_t key = lane < (word & RUN_COUNT) ? key_of(mine) : NONE;
     for (uint64_t best = smallest(key); best != NONE; best = smallest(key)) {
       apply(__ffs(__ballot_sync(0xffffffffu, key == best)) - 1);
       if (key == best) key = NONE;
@@ -489,29 +494,11 @@ __device__ __noinline__ float run_grid_step(const StepBufs<T>& b, const ScenePar
   return m;
 }
 
-// The end of sphere i's step, after its integration: the container, the
-// displacement from `old`, and the mark of a sphere outside its cell of the
-// build.  TEST: triangles are tested; else none is within reach and a
-// triangle container adds zero.
-template <class T, bool MESH, bool TEST>
-__device__ __forceinline__ void run_advance(vec4_t<T>& P, vec4_t<T>& V, uint32_t i, uint32_t word,
-                                            const StepBufs<T>& b, const SceneParams<T>& sp, const MeshView* mv,
-                                            const vec4_t<T>& old, float& m) {
-  if constexpr (MESH) {
-    if (sp.mesh_tris > 0) {
-      if constexpr (TEST) {
-        mesh_contacts<T>(P, V, sp, *mv, b.err);
-      } else {
-        P.x = Ar<T>::add(P.x, T(0));
-        P.y = Ar<T>::add(P.y, T(0));
-        P.z = Ar<T>::add(P.z, T(0));
-      }
-    } else {
-      walls<T>(P, V, sp);
-    }
-  } else {
-    walls<T>(P, V, sp);
-  }
+// The end of sphere i's step after the container: its displacement from
+// `old`, and the mark of a sphere outside its cell of the build.
+template <class T>
+__device__ __forceinline__ void run_finish(vec4_t<T>& P, uint32_t i, uint32_t word, const StepBufs<T>& b,
+                                           const SceneParams<T>& sp, const vec4_t<T>& old, float& m) {
   m = fmaxf(m, moved2<T>(P, old, T(1) / (sp.interval * sp.interval)));
   if (word & RUN_NEAR_FACE) {
     int32_t cx, cy, cz;
@@ -519,120 +506,291 @@ __device__ __forceinline__ void run_advance(vec4_t<T>& P, vec4_t<T>& V, uint32_t
   }
 }
 
-// The list step of the spheres it put aside, whose chains of loads are long:
-// taken inline by their own thread, a handful of them held the whole step up
-// (30,011-sphere pile: 7.2 us a step without any, 14.5 us with forty).  A
-// warp takes each sphere that needs run_slow's order (the first n_slow
-// entries); a thread each near a triangle (the last n_mesh entries, contacts
-// and integration done), which gathers them into full warps.
+// Whether an integrated sphere has to test triangles: some may be within
+// reach since the build, or it moves a good part of the skin at once.
+template <class T>
+__device__ __forceinline__ bool run_near_mesh(const vec4_t<T>& P, const vec4_t<T>& old, uint32_t word, T skin) {
+  const T lim = T(0.25) * skin;
+  const T ex = P.x - old.x, ey = P.y - old.y, ez = P.z - old.z;
+  return (word >> RUN_TRIS) != 0u || !(ex * ex + ey * ey + ez * ez <= lim * lim);
+}
+
+// Spheres that a CTA's list step puts aside, their chains of loads being
+// long: taken inline by their own thread, a handful of them held the whole
+// step up (30,011-sphere pile: 7.2 us a step without any, 14.5 us with forty).
+constexpr uint32_t RUN_LATE_HERE = 256;
+struct RunLate {
+  uint32_t n_slow, n_near;
+  uint32_t slow[RUN_LATE_HERE];  // need run_slow's order
+  uint32_t near[RUN_LATE_HERE];  // need their triangles (contacts and integration done)
+};
+
+template <class T>
+__device__ __forceinline__ void run_put_aside(RunLate& l, const RunBufs<T>& R, uint32_t i, bool slow) {
+  const uint32_t k = atomicAdd(slow ? &l.n_slow : &l.n_near, 1u);
+  uint32_t* const here = slow ? l.slow : l.near;
+  uint32_t* const there = R.later + (size_t)blockIdx.x * R.later_stride;
+  if (k < RUN_LATE_HERE)
+    here[k] = i;
+  else  // one kind from the front, the other from the back
+    there[slow ? k : R.later_stride - 1u - k] = i;
+}
+template <class T>
+__device__ __forceinline__ uint32_t run_put(const RunLate& l, const RunBufs<T>& R, uint32_t k, bool slow) {
+  const uint32_t* there = R.later + (size_t)blockIdx.x * R.later_stride;
+  return k < RUN_LATE_HERE ? (slow ? l.slow[k] : l.near[k]) : there[slow ? k : R.later_stride - 1u - k];
+}
+
+// Triangle container of a sphere from the triangles listed at the build, by
+// half a warp: the lanes test a triangle each, and the hits, which come in
+// ascending index, are added in turn.  The other half may have another
+// sphere (or none: nt = 0).
+template <class T>
+__device__ __forceinline__ void run_mesh_half(vec4_t<T>& P, vec4_t<T>& V, uint32_t nt, uint32_t t, const StepBufs<T>& b,
+                                              const SceneParams<T>& sp, const MeshView& mv) {
+  using A = Ar<T>;
+  static_assert(RUN_TRI_CAP == 16, "a triangle per lane of half a warp");
+  const unsigned sub = threadIdx.x & 15u;
+  const T r = P.w;
+  const V3<T> c = {P.x, P.y, P.z};
+  const V3<T> lo = {A::sub(c.x, r), A::sub(c.y, r), A::sub(c.z, r)};
+  const V3<T> hi = {A::add(c.x, r), A::add(c.y, r), A::add(c.z, r)};
+  bool hit = sub < nt && in_bounds(t, mv.n_tri, b.err);
+  Triangle<T> g = {};
+  if (hit) {
+    g = triangle<T>(mv, t);  // (with the box, not after it)
+    hit = in_box<T>(mv, t, lo, hi) && mesh_hit<T>(g, c, r, sp);
+  }
+  // what the hit adds (mesh_add's operations)
+  const V3<T> n = g.n;
+  const T vn2 = A::mul(T(2), dot3<T>(V.x, V.y, V.z, n.x, n.y, n.z));
+  const V3<T> refl = {A::fma(-vn2, n.x, V.x), A::fma(-vn2, n.y, V.y), A::fma(-vn2, n.z, V.z)};
+  const T sc = A::sub(r, dot3<T>(-n.x, -n.y, -n.z, A::sub(c.x, g.a.x), A::sub(c.y, g.a.y), A::sub(c.z, g.a.z)));
+  const uint32_t who = __ballot_sync(0xffffffffu, hit);
+  const uint32_t ours = (threadIdx.x & 16u) ? who >> 16 : who & 0xffffu;
+  MeshSums<T> m = {};
+  for (uint32_t left = (who | (who >> 16)) & 0xffffu; left != 0u; left &= left - 1u) {
+    const int k = __ffs(left) - 1;
+    const V3<T> rk = {__shfl_sync(0xffffffffu, refl.x, k, 16), __shfl_sync(0xffffffffu, refl.y, k, 16),
+                      __shfl_sync(0xffffffffu, refl.z, k, 16)};
+    const V3<T> nk = {__shfl_sync(0xffffffffu, n.x, k, 16), __shfl_sync(0xffffffffu, n.y, k, 16),
+                      __shfl_sync(0xffffffffu, n.z, k, 16)};
+    const T sk = __shfl_sync(0xffffffffu, sc, k, 16);
+    if ((ours >> k) & 1u) {
+      m.v = {A::fma(sp.e_poly, rk.x, m.v.x), A::fma(sp.e_poly, rk.y, m.v.y), A::fma(sp.e_poly, rk.z, m.v.z)};
+      m.x = {A::fma(-sk, nk.x, m.x.x), A::fma(-sk, nk.y, m.x.y), A::fma(-sk, nk.z, m.x.z)};
+      ++m.hits;
+    }
+  }
+  mesh_apply<T>(m, c, P, V);
+}
+
+// The step of the spheres put aside: a warp to each that needs run_slow's
+// order, half a warp to each near a triangle.
 template <class T, bool MULTI, bool MESH>
 __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
-                                       const RunBufs<T>& R, int cur, float frac, bool last, uint32_t n_slow,
-                                       uint32_t n_mesh) {
+                                       const RunBufs<T>& R, const RunLate& l, int cur, float frac, bool last) {
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
   vec4_t<T>* Vd = R.v(1 - cur);
-  const uint32_t* later = R.later + (size_t)blockIdx.x * R.later_stride;
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t n_slow = l.n_slow, n_near = MESH ? l.n_near : 0u;
   float m = 0.0f;
   for (uint32_t k = threadIdx.x >> 5; k < n_slow; k += STEP_THREADS / 32) {
-    const uint32_t i = later[k];
+    const uint32_t i = run_put<T>(l, R, k, true);
     const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
     const uint32_t word = R.cnt[i];
+    uint32_t mine = lane < R.cap ? R.list[(size_t)lane * b.n + i] & ~RUN_FAR_CELL : i;
     vec4_t<T> old = Ps[i];
-    vec4_t<T> V = run_slow<T>(i, word, b, sp, R, Ps, Vs, (T)frac, old, Vs[i]);
+    if (lane >= (word & RUN_COUNT) || !in_bounds(mine, b.n, b.err)) mine = i;
+    vec4_t<T> V = run_slow<T>(i, word, mine, b, sp, Ps, Vs, (T)frac, old, Vs[i]);
     old.w = fabs(old.w);
     vec4_t<T> P = old;
     if (!last) {
       integrate<T>(P, V, sp);
-      run_advance<T, MESH, true>(P, V, i, word, b, sp, mv, old, m);
+      if constexpr (MESH) {
+        if (sp.mesh_tris > 0)
+          mesh_contacts<T>(P, V, sp, *mv, b.err);
+        else
+          walls<T>(P, V, sp);
+      } else {
+        walls<T>(P, V, sp);
+      }
+      run_finish<T>(P, i, word, b, sp, old, m);
     }
     __syncwarp();
-    if ((threadIdx.x & 31u) == 0u) {
+    if (lane == 0u) {
       Pd[i] = P;
       Vd[i] = V;
     }
   }
   if constexpr (MESH) {
-    for (uint32_t k = threadIdx.x; k < n_mesh; k += STEP_THREADS) {
-      const uint32_t i = later[R.later_stride - 1u - k];
+    for (uint32_t k0 = (threadIdx.x >> 5) * 2u; k0 < n_near; k0 += STEP_THREADS / 16) {
+      const uint32_t k = k0 + ((threadIdx.x >> 4) & 1u);
+      const bool on = k < n_near;
+      const uint32_t i = run_put<T>(l, R, on ? k : k0, false);
+      const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
+      const uint32_t word = R.cnt[i], nt = word >> RUN_TRIS;
+      const uint32_t t = R.tris[(size_t)(lane & 15u) * b.n + i];
+      const vec4_t<T> old = Ps[i];
       vec4_t<T> P = Pd[i], V = Vd[i];
-      run_advance<T, MESH, true>(P, V, i, R.cnt[i], b, scene_of<T, MULTI>(i, sp0, b), mv, Ps[i], m);
-      Pd[i] = P;
-      Vd[i] = V;
+      // a sphere beyond its list walks its bin instead
+      const bool walk = on && (nt > RUN_TRI_CAP || run_near_mesh<T>(P, old, 0u, (T)frac * sp.interval));
+      vec4_t<T> Pw = P, Vw = V;
+      if (walk) mesh_contacts<T>(Pw, Vw, sp, *mv, b.err);
+      __syncwarp();
+      run_mesh_half<T>(P, V, on && !walk ? nt : 0u, t, b, sp, *mv);
+      if (walk) P = Pw, V = Vw;
+      run_finish<T>(P, i, word, b, sp, old, m);
+      __syncwarp();
+      if (on && (lane & 15u) == 0u) {
+        Pd[i] = P;
+        Vd[i] = V;
+      }
     }
   }
   return m;
 }
 
+// A thread's own sphere, kept in registers from step to step when the grid
+// has a thread for every sphere.
+template <class T>
+struct RunOwn {
+  vec4_t<T> P, V;
+  uint32_t word;
+  uint32_t head[run_batch<T>()];  // first entries of its list
+};
+
+template <class T, bool OWN>
+__device__ __forceinline__ void run_load_own(RunOwn<T>& o, uint32_t i, const StepBufs<T>& b, const RunBufs<T>& R,
+                                             int cur) {
+  o.P = R.p(cur)[i];
+  o.V = R.v(cur)[i];
+  o.word = R.cnt[i];
+  if constexpr (!OWN) return;
+#pragma unroll
+  for (int u = 0; u < run_batch<T>(); ++u)
+    o.head[u] = (uint32_t)u < (o.word & RUN_COUNT) ? R.list[(size_t)u * b.n + i] : i;
+}
+
 // One step on the lists: contacts of the state in buffer `cur`, then, unless
 // it is the call's last step, the next step's integration and container.
-template <class T, bool MULTI, bool MESH>
+// OWN: each thread has one sphere at most, and `own` holds it (loaded when
+// `fresh`), so that a step waits for its neighbours' positions alone.
+template <class T, bool MULTI, bool MESH, bool OWN>
 __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
-                                               const RunBufs<T>& R, int cur, float frac, bool last) {
-  __shared__ uint32_t s_slow, s_mesh;
-  if (threadIdx.x == 0) s_slow = s_mesh = 0u;
-  __syncthreads();
+                                               const RunBufs<T>& R, int cur, float frac, bool last, RunOwn<T>& own,
+                                               bool fresh) {
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
   vec4_t<T>* Vd = R.v(1 - cur);
+  constexpr int NB = run_batch<T>();
+  __shared__ RunLate late;
+  if (threadIdx.x == 0) late.n_slow = late.n_near = 0u;
+  __syncthreads();
   float m = 0.0f;
+  bool odd = false, near = false;
   for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += gridDim.x * STEP_THREADS) {
-    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
-    vec4_t<T> P = Ps[i];
-    const vec4_t<T> Vi = Vs[i];
-    const uint32_t word = R.cnt[i];
-    vec4_t<T> V = Vi;
-    const uint32_t nl = word & RUN_COUNT;
-    bool odd = (word & RUN_OVERFLOW) != 0u;
-    constexpr int NB = run_batch<T>();
-    for (uint32_t k0 = 0; k0 < nl; k0 += NB) {
-      uint32_t jj[NB];
-      vec4_t<T> Q[NB];
+    odd = near = false;
+    {
+      const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
+      if (!OWN || fresh) run_load_own<T, OWN>(own, i, b, R, cur);
+      const vec4_t<T> Vi = own.V;
+      const uint32_t nl = own.word & RUN_COUNT;
+      // Partners that have left their cell of the build may change the order,
+      // if there are two; a pair as wide as a cell may be of cells that are
+      // not adjacent, by the rounding of the hash (below a thousandth of a
+      // cell up to 4,096 cells on an axis), and is marked or was so at the build.
+      uint32_t touching = 0;
+      bool moved = false, wide = (own.word & RUN_OVERFLOW) != 0u;
+      uint32_t next[NB];
+      if constexpr (OWN) {
 #pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        jj[u] = k0 + u < nl ? R.list[(size_t)(k0 + u) * b.n + i] : i;
-        if (!in_bounds(jj[u] & ~RUN_FAR_CELL, b.n, b.err)) jj[u] = i;
+        for (int u = 0; u < NB; ++u) next[u] = own.head[u];
       }
+      for (uint32_t k0 = 0; k0 < nl; k0 += NB) {
+        uint32_t jj[NB];
+        vec4_t<T> Q[NB];
 #pragma unroll
-      for (int u = 0; u < NB; ++u) Q[u] = Ps[jj[u] & ~RUN_FAR_CELL];
+        for (int u = 0; u < NB; ++u) {
+          jj[u] = OWN ? next[u] : (k0 + u < nl ? R.list[(size_t)(k0 + u) * b.n + i] : i);
+          if (!in_bounds(jj[u] & ~RUN_FAR_CELL, b.n, b.err)) jj[u] = i;
+        }
 #pragma unroll
-      for (int u = 0; u < NB; ++u)
-        if (k0 + u < nl &&
-            contact_one<T, true>(Vs, jj[u] & ~RUN_FAR_CELL, P, Vi, Q[u], sp.k_spring, sp.e_sphere, V.x, V.y, V.z))
-          odd |= (jj[u] & RUN_FAR_CELL) != 0u || marked<T>(Q[u].w) || marked<T>(P.w);
-    }
-    P.w = fabs(P.w);
-    bool mesh = false;
-    if (!last && !odd) {
-      const vec4_t<T> old = P;
-      integrate<T>(P, V, sp);
-      if constexpr (MESH) {
-        // near a triangle at the build, or moving a good part of the skin now
-        const T lim = T(0.25) * (T)frac * sp.interval;
-        const T ex = P.x - old.x, ey = P.y - old.y, ez = P.z - old.z;
-        mesh = sp.mesh_tris > 0 && ((word & RUN_NEAR_MESH) || !(ex * ex + ey * ey + ez * ez <= lim * lim));
+        for (int u = 0; u < NB; ++u) Q[u] = Ps[jj[u] & ~RUN_FAR_CELL];
+        if constexpr (OWN) {  // (64 registers, of the other form, do not hold them)
+#pragma unroll
+          for (int u = 0; u < NB; ++u) next[u] = k0 + NB + u < nl ? R.list[(size_t)(k0 + NB + u) * b.n + i] : i;
+        }
+#pragma unroll
+        for (int u = 0; u < NB; ++u)
+          if (k0 + u < nl && contact_one<T, true>(Vs, jj[u] & ~RUN_FAR_CELL, own.P, Vi, Q[u], sp.k_spring, sp.e_sphere,
+                                                  own.V.x, own.V.y, own.V.z)) {
+            ++touching;
+            moved |= marked<T>(Q[u].w);
+            wide |= (jj[u] & RUN_FAR_CELL) != 0u ||
+                    ((marked<T>(Q[u].w) || marked<T>(own.P.w)) &&
+                     (fabs(own.P.w) + fabs(Q[u].w) > T(0.999) * sp.interval ||
+                      max(sp.nb[0], max(sp.nb[1], sp.nb[2])) > 4096));
+          }
       }
-      if (!mesh) run_advance<T, MESH, false>(P, V, i, word, b, sp, mv, old, m);
+      odd = wide || (moved && touching > 1u);
+      own.P.w = fabs(own.P.w);
+      if (!last && !odd) {
+        const vec4_t<T> old = own.P;
+        integrate<T>(own.P, own.V, sp);
+        bool box = true;
+        if constexpr (MESH) {
+          if (sp.mesh_tris > 0) {
+            box = false;
+            near = run_near_mesh<T>(own.P, old, own.word, (T)frac * sp.interval);
+            if (!near) {  // the container adds a zero correction
+              own.P.x = Ar<T>::add(own.P.x, T(0));
+              own.P.y = Ar<T>::add(own.P.y, T(0));
+              own.P.z = Ar<T>::add(own.P.z, T(0));
+            }
+          }
+        }
+        if (box) walls<T>(own.P, own.V, sp);
+        if (!near) run_finish<T>(own.P, i, own.word, b, sp, old, m);
+      }
+      Pd[i] = own.P;
+      Vd[i] = own.V;
     }
-    if (odd || mesh) {
-      uint32_t* later = R.later + (size_t)blockIdx.x * R.later_stride;
-      later[odd ? atomicAdd(&s_slow, 1u) : R.later_stride - 1u - atomicAdd(&s_mesh, 1u)] = i;
-    }
-    Pd[i] = P;
-    Vd[i] = V;
+    if (odd || near) run_put_aside<T>(late, R, i, odd);
   }
   __syncthreads();
-  const uint32_t n_slow = s_slow, n_mesh = s_mesh;
-  if (n_slow + n_mesh > 0u) m = fmaxf(m, run_late<T, MULTI, MESH>(b, sp0, mv, R, cur, frac, last, n_slow, n_mesh));
+  if (late.n_slow + late.n_near > 0u) {
+    m = fmaxf(m, run_late<T, MULTI, MESH>(b, sp0, mv, R, late, cur, frac, last));
+    if constexpr (OWN) {
+      __syncthreads();
+      if (odd || near) {
+        const uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x;
+        own.P = Pd[i];
+        own.V = Vd[i];
+      }
+    }
+  }
   return m;
 }
 
 // `steps` steps from the at-rest state (P0, V1, orig), which is also where
 // the state ends.
-template <class T, bool MULTI, bool MESH>
-__global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 2)
+// OWN: the grid has a thread for every sphere.
+//
+// CTAs per SM: with more spheres than threads the warps in flight hide the
+// latency, and four CTAs leave 64 registers (FP32); with a thread for every
+// sphere there are no more warps to have, and half the CTAs leave room for
+// the sphere's state.
+template <class T, bool OWN>
+__host__ __device__ constexpr int run_ctas() {
+  return (sizeof(T) == 4 ? 4 : 2) / (OWN ? 2 : 1);
+}
+
+template <class T, bool MULTI, bool MESH, bool OWN>
+__global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     k_run(const __grid_constant__ StepBufs<T> b, const __grid_constant__ SceneParams<T> sp0, const MeshView* mv,
           const __grid_constant__ RunBufs<T> R, uint32_t steps, int64_t n_cells, uint32_t scatter_blocks,
           uint32_t move_blocks, uint32_t run_id) {
@@ -644,14 +802,18 @@ __global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 2)
   bool counted = true;   // the state's cells are counted already
   float D = 0.0f;        // motion since the last build, in cells
   float frac = 0.0f;     // skin of the last build, in cells
-  uint32_t unsettled = 0;
-  float before = INFINITY;  // the last step's m
+  uint32_t rebuilds = 0;
+  // the last step's m, of an earlier run if need be
+  float before = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_BEFORE));
+  if (!(before > 0.0f)) before = INFINITY;
+  RunOwn<T> own;
   for (uint32_t s = 0; s < steps; ++s) {
     if (!run_barrier(R.ctl, b.err)) return;
     const float m = sqrtf(__uint_as_float(*reinterpret_cast<volatile uint32_t*>(maxd + s % 3u)));
     if (blockIdx.x == 0 && threadIdx.x == 0) maxd[(s + 2u) % 3u] = 0u;
     streak = m <= RUN_CALM_MAX ? (streak < RUN_CALM_STEPS ? streak + 1u : streak) : 0u;
     D = D * 1.000001f + m;
+    bool fresh = false;
     if (!lists || !(D <= 0.49f * frac)) {
       lists = streak >= RUN_CALM_STEPS;
       // (a single fast step, a sphere pushed out of a wall, is no measure)
@@ -659,13 +821,14 @@ __global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 2)
       if (!run_rebuild<T, MULTI, MESH>(b, sp0, mv, R, cur, counted, frac, n_cells, scatter_blocks, move_blocks)) return;
       cur = 1 - cur;
       D = 0.0f;
-      unsettled += lists ? 0u : 1u;
+      fresh = true;
+      ++rebuilds;
     }
     before = m;
     const bool last = s + 1u == steps;
     float mm;
     if (lists)
-      mm = run_list_step<T, MULTI, MESH>(b, sp0, mv, R, cur, frac, last);
+      mm = run_list_step<T, MULTI, MESH, OWN>(b, sp0, mv, R, cur, frac, last, own, fresh);
     else
       mm = run_grid_step<T, MULTI, MESH>(b, sp0, mv, R, cur, last);
     if (!last) publish_max(mm, maxd + (s + 1u) % 3u);
@@ -685,7 +848,8 @@ __global__ void __launch_bounds__(STEP_THREADS, sizeof(T) == 4 ? 4 : 2)
   if (blockIdx.x == 0 && threadIdx.x == 0u) {
     R.ctl[RUN_STREAK] = streak;
     R.report[0] = run_id;
-    R.report[1] = 2u * unsettled > steps ? 1u : 0u;
+    R.ctl[RUN_BEFORE] = __float_as_uint(before);
+    R.report[1] = (steps >= 64u ? 4u : 2u) * rebuilds > steps ? 1u : 0u;
   }
 }
 

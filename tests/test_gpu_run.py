@@ -48,7 +48,9 @@ SCENES = {
                       scenes.pile(64, seed=17, k_spring=1e4)],
     "box mesh": lambda: [scenes.box_mesh_scene()],
     "funnel": lambda: [scenes.funnel_wall_scene(1500)],
-    "fan": lambda: [scenes.fan_floor_scene()],
+    "fan": lambda: [scenes.fan_floor_scene()],                                    # more triangles than a sphere's list
+    "fine mesh": lambda: [scenes.box_mesh_scene(100, seed=46).copy(tri=scenes.box_container(n=16))],
+    "more than a CTA's share aside": lambda: [faster(scenes.pile(70000, seed=34, k_spring=1.0), 20.0)],
     "batch with a mesh": lambda: [scenes.pile(300, seed=28, k_spring=1.0), scenes.box_mesh_scene(),
                                   scenes.pile(500, seed=29, k_spring=1.0)],
 }
