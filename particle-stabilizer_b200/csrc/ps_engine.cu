@@ -518,15 +518,17 @@ void enqueue_regrid(ps_sim* s) {
   const unsigned gb = blocks_for(s->n_total);
   const unsigned gp = blocks_for(s->n_total);
   cudaStream_t st = s->stream;
-  k_begin<T, MULTI, false, false><<<gb, STEP_THREADS, 0, st>>>(b, sp0, s->d_mesh_view);
-  k_tile_sums<<<(unsigned)step_scan_tiles(n_scan(s)), STEP_THREADS, 0, st>>>(s->count, n_scan(s), s->tile_sum,
-                                                                              step_scan_shift(n_scan(s)));
-  step_scan_kernel(n_scan(s))<<<(unsigned)step_scan_tiles(n_scan(s)), SCAN_THREADS, 0, st>>>(s->count, s->offset, n_scan(s),
-                                                                                     s->tile_sum);
-  k_scatter<<<move_blocks(s->n_total, b.n_tiles), STEP_THREADS, 0, st>>>(s->cell, s->slot, s->orig, s->offset, s->tmp,
-                                                                       s->count, (uint32_t)s->n_total, s->tile_sum, b.n_tiles, s->err);
-  k_rank_move<T><<<move_blocks(s->n_total, 0), STEP_THREADS, 0, st>>>(b);
-  k_copy_vel<T><<<gp, STEP_THREADS, 0, st>>>(b);
+  const int64_t nsc = n_scan(s);
+  const unsigned gs = (unsigned)step_scan_tiles(nsc);
+  pdl_launch(k_begin<T, MULTI, false, false>, gb, STEP_THREADS, st, b, sp0, (const MeshView*)s->d_mesh_view);
+  pdl_launch(k_tile_sums, gs, STEP_THREADS, st, (const uint32_t*)s->count, nsc, s->tile_sum, step_scan_shift(nsc));
+  pdl_launch(step_scan_kernel(nsc), gs, SCAN_THREADS, st, (const uint32_t*)s->count, s->offset, nsc,
+             (const uint32_t*)s->tile_sum);
+  pdl_launch(k_scatter, move_blocks(s->n_total, b.n_tiles), STEP_THREADS, st, (const uint32_t*)s->cell, s->slot,
+             (const uint32_t*)s->orig, (const uint32_t*)s->offset, s->tmp, s->count, (uint32_t)s->n_total, s->tile_sum,
+             b.n_tiles, s->err);
+  pdl_launch(k_rank_move<T>, move_blocks(s->n_total, 0), STEP_THREADS, st, b);
+  pdl_launch(k_copy_vel<T>, gp, STEP_THREADS, st, b);
 }
 
 int regrid(ps_sim* s) {
@@ -547,6 +549,7 @@ int regrid(ps_sim* s) {
 // index, and the last run's report (its number, and 1 when it rebuilt the
 // grid in more than every fourth step; of a short run, in every second).
 constexpr int ERR_BITS = 0, ERR_BAD = 8, ERR_RUN = 16, ERR_WORDS = 18;
+constexpr int ERR_TICKET = 24;  // blocks of k_stats that have finished (zero between launches)
 
 // After a run that rebuilt so often, the next
 // RUN_BACKOFF_MIN steps (doubling up to RUN_BACKOFF_MAX while that repeats)
@@ -1485,8 +1488,7 @@ extern "C" int ps_get_state(ps_sim* s, double* out, int64_t n_total) {
                                                           static_cast<vec4_t<double>*>(s->V1), s->orig, (uint32_t)n_total);
   PS_CUDA(cudaGetLastError());
   PS_CUDA(cudaMemcpyAsync(out, s->staging, 64 * (size_t)n_total, cudaMemcpyDeviceToHost, s->stream));
-  PS_CUDA(cudaStreamSynchronize(s->stream));
-  return check_device_error(s);
+  return check_device_error(s);  // waits for the stream
 }
 
 namespace {
@@ -2242,16 +2244,18 @@ extern "C" int ps_stats_get(ps_sim* s, int32_t scene, ps_stats* out) {
     if (rc != PS_OK) return rc;
   }
   const uint32_t first = (uint32_t)s->pbase[scene];
-  if (s->precision == PS_FP32) {
-    k_stats<float><<<kStatsBlocks, kStatsThreads, 0, s->stream>>>(bufs<float>(s), s->sp32[scene], first, (uint32_t)n, s->d_stats);
-  } else {
-    k_stats<double><<<kStatsBlocks, kStatsThreads, 0, s->stream>>>(bufs<double>(s), s->sp64[scene], first, (uint32_t)n, s->d_stats);
-  }
-  k_stats_final<<<1, 32, 0, s->stream>>>(s->d_stats, s->d_stats_out);
+  const unsigned g = std::min<unsigned>(kStatsBlocks, (unsigned)((n + kStatsThreads - 1) / kStatsThreads));
+  if (s->precision == PS_FP32)
+    pdl_launch(k_stats<float>, g, kStatsThreads, s->stream, bufs<float>(s), s->sp32[scene], first, (uint32_t)n, s->d_stats,
+               s->d_stats_out, s->err + ERR_TICKET);
+  else
+    pdl_launch(k_stats<double>, g, kStatsThreads, s->stream, bufs<double>(s), s->sp64[scene], first, (uint32_t)n,
+               s->d_stats, s->d_stats_out, s->err + ERR_TICKET);
   PS_CUDA(cudaGetLastError());
   StatsPartial h{};
   PS_CUDA(cudaMemcpyAsync(&h, s->d_stats_out, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
-  PS_CUDA(cudaStreamSynchronize(s->stream));
+  const int rc = check_device_error(s);  // waits for the stream
+  if (rc != PS_OK) return rc;
   out->kinetic_energy = h.ke;
   for (int a = 0; a < 3; ++a) {
     out->min_pos[a] = h.mn[a];
@@ -2259,7 +2263,7 @@ extern "C" int ps_stats_get(ps_sim* s, int32_t scene, ps_stats* out) {
   }
   out->n_collided = (int64_t)h.collided;
   out->max_overlap = h.max_overlap;
-  return check_device_error(s);
+  return PS_OK;
 }
 
 extern "C" int ps_destroy(ps_sim* s) {

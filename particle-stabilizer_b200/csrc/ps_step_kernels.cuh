@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_begin(StepBufs<T> b, ScenePara
 __global__ void __launch_bounds__(STEP_THREADS) k_tile_sums(const uint32_t* __restrict__ count, int64_t n,
                                                            uint32_t* __restrict__ tile_sum, uint32_t tile_shift) {
   __shared__ uint32_t s_red[STEP_THREADS / 32];
+  pdl_wait();
   const int64_t base = (int64_t)blockIdx.x << tile_shift;
   const int64_t end = base + (int64_t(1) << tile_shift);
   uint32_t sum = 0;
@@ -718,6 +719,7 @@ __global__ void __launch_bounds__(BLOCK, contact_min_blocks<T, BLOCK>()) k_conta
 // Copy V0 -> V1 (restores the at-rest layout after a regrid).
 template <class T>
 __global__ void __launch_bounds__(STEP_THREADS) k_copy_vel(StepBufs<T> b) {
+  pdl_wait();
   const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
   if (p < b.n) b.V1[p] = b.V0[p];
 }

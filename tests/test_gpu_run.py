@@ -115,3 +115,21 @@ def test_adjoint_of_runs_whose_order_is_an_earlier_grids(need_gpu, skin):
     # the same sums in the same order, whatever the blocks
     assert np.array_equal(out[0][2], out[1][2])
     np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-9)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("n", [1, 31, 255, 257, 2000])
+def test_statistics_at_the_edges_of_the_reduction(need_gpu, prec, n):
+    sc = scenes.pile(max(n, 8), seed=60 + n, k_spring=1.0)
+    sc = sc.copy(state=sc.state[:n])
+    with psb200.Simulation([scenes.pile(300, seed=61), sc], prec) as sim:
+        sim.set_state()
+        sim.step(9)
+        got = [sim.stats(1) for _ in range(2)]
+        state = sim.get_state()[300:]
+    o = O.stats(state)
+    for s in got:
+        assert s.n_collided == o.n_collided
+        assert s.max_overlap == pytest.approx(o.max_overlap, rel=1e-12, abs=0)
+        assert s.kinetic_energy == pytest.approx(o.kinetic_energy, rel=1e-12)
+        assert list(s.min_pos) == list(o.min_pos) and list(s.max_pos) == list(o.max_pos)
