@@ -262,25 +262,42 @@ __global__ void k_tape_write(StepBufs<T> b, TapeRow<T> row) {
 
 
 // Per-scene sums of the parameter partials (acc: ADJ_NACC rows of n), in a
-// fixed order.
-__global__ void k_adj_reduce(const double* acc, const uint32_t* pbase, int n_scenes, uint32_t n, double* out) {
-  const int s = blockIdx.x;
-  if (s >= n_scenes) return;
-  const uint32_t p0 = pbase[s], p1 = s + 1 < n_scenes ? pbase[s + 1] : n;
-  __shared__ double red[ADJ_NACC][128];
-  double loc[ADJ_NACC];
-  for (int c = 0; c < ADJ_NACC; ++c) loc[c] = 0.0;
-  for (uint32_t p = p0 + threadIdx.x; p < p1; p += blockDim.x)
-    for (int c = 0; c < ADJ_NACC; ++c) loc[c] += acc[(size_t)c * n + p];
-  for (int c = 0; c < ADJ_NACC; ++c) red[c][threadIdx.x] = loc[c];
+// fixed order: block (q, c) of a scene adds row c's q-th share, and
+// k_adj_reduce_shares the shares.  One block per scene, as this was at first,
+// left the GPU idle: 65,536 spheres of one scene took 1.64 ms.
+constexpr int ADJ_REDUCE_THREADS = 256;
+
+__device__ __forceinline__ double adj_block_sum(double v, double (&red)[ADJ_REDUCE_THREADS / 32]) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+  if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int w = 64; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-      for (int c = 0; c < ADJ_NACC; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + w];
-    __syncthreads();
-  }
   if (threadIdx.x == 0)
-    for (int c = 0; c < ADJ_NACC; ++c) out[ADJ_NACC * s + c] = red[c][0];
+    for (int w = 1; w < ADJ_REDUCE_THREADS / 32; ++w) v += red[w];
+  return v;
+}
+
+// grid (shares, ADJ_NACC, scenes up to 65,535 at a time, the first being s0)
+__global__ void __launch_bounds__(ADJ_REDUCE_THREADS) k_adj_reduce(const double* __restrict__ acc,
+                                                                  const uint32_t* __restrict__ pbase, int s0,
+                                                                  int n_scenes, uint32_t n, double* part) {
+  __shared__ double red[ADJ_REDUCE_THREADS / 32];
+  const int s = s0 + (int)blockIdx.z, c = blockIdx.y;
+  const uint32_t p0 = pbase[s], p1 = s + 1 < n_scenes ? pbase[s + 1] : n;
+  double v = 0.0;
+  for (uint64_t p = p0 + blockIdx.x * ADJ_REDUCE_THREADS + threadIdx.x; p < p1;
+       p += (uint64_t)gridDim.x * ADJ_REDUCE_THREADS)
+    v += acc[(size_t)c * n + p];
+  v = adj_block_sum(v, red);
+  if (threadIdx.x == 0) part[((size_t)s * ADJ_NACC + c) * gridDim.x + blockIdx.x] = v;
+}
+
+__global__ void k_adj_reduce_shares(const double* __restrict__ part, int shares, int n_sums, double* out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n_sums) return;
+  double v = 0.0;
+  for (int q = 0; q < shares; ++q) v += part[(size_t)k * shares + q];
+  out[k] = v;
 }
 
 }  // namespace psb

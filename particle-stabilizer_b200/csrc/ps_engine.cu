@@ -1246,7 +1246,13 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
   const size_t adj_b = align_up(sizeof(vec4_t<T>) * (size_t)n, 256);
   const size_t acc_b = align_up(ADJ_NACC * sizeof(double) * (size_t)n, 256);
   const size_t io_b = align_up(6 * sizeof(double) * (size_t)n, 256);
-  const size_t red_b = align_up(ADJ_NACC * sizeof(double) * (size_t)s->n_scenes, 256);
+  // shares of a scene's sum: a block's worth of partials each, about 2,048 in all
+  int64_t most = 0;
+  for (int sc = 0; sc < s->n_scenes; ++sc) most = std::max(most, s->pbase[sc + 1] - s->pbase[sc]);
+  const int shares = (int)std::max<int64_t>(
+      1, std::min<int64_t>((most + ADJ_REDUCE_THREADS - 1) / ADJ_REDUCE_THREADS, 256 / std::min(s->n_scenes, 256)));
+  const size_t n_sums = (size_t)ADJ_NACC * (size_t)s->n_scenes;
+  const size_t red_b = align_up(sizeof(double) * n_sums, 256) + align_up(sizeof(double) * n_sums * (size_t)shares, 256);
   const size_t inv_b = align_up(sizeof(uint32_t) * (size_t)n, 256);
   const size_t need = tape_b + offs_b + 4 * adj_b + inv_b + acc_b + io_b + red_b;
   if (s->adj_bytes < need) {
@@ -1314,7 +1320,11 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
       PS_CUDA(cudaGetLastError());
     }
   }
-  k_adj_reduce<<<s->n_scenes, 128, 0, st>>>(a.acc, s->d_pbase, s->n_scenes, (uint32_t)n, red);
+  double* share_sums = red + align_up(sizeof(double) * n_sums, 256) / sizeof(double);
+  for (int s0 = 0; s0 < s->n_scenes; s0 += 65535)
+    k_adj_reduce<<<dim3((unsigned)shares, ADJ_NACC, (unsigned)std::min(65535, s->n_scenes - s0)), ADJ_REDUCE_THREADS, 0,
+                   st>>>(a.acc, s->d_pbase, s0, s->n_scenes, (uint32_t)n, share_sums);
+  k_adj_reduce_shares<<<(unsigned)((n_sums + 255) / 256), 256, 0, st>>>(share_sums, shares, (int)n_sums, red);
   std::vector<double> h((size_t)ADJ_NACC * s->n_scenes);
   PS_CUDA(cudaMemcpyAsync(h.data(), red, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
   if (dl_dstate0 != nullptr) {
