@@ -154,7 +154,9 @@ struct ps_sim {
   bool l2_limit_set = false;
   // differentiation
   int64_t fwd_steps = 0, fwd_every = 0;   // last ps_forward_checkpointed
-  std::vector<void*> fwd_ckpt;            // state at the start of each block, + final state last
+  std::vector<void*> fwd_ckpt;            // state at the start of each block, + final state last (in fwd_arena)
+  void* fwd_arena = nullptr;
+  size_t fwd_bytes = 0;
   void* adj_arena = nullptr;              // tape, adjoint arrays, partials
   size_t adj_bytes = 0;
   // neighbour-list mode (ps_set_neighbor_lists); off when list_skin <= 0
@@ -174,6 +176,8 @@ struct ps_sim {
   // the kernel of many steps (ps_run.cuh)
   uint32_t* d_chunk_scene = nullptr;      // scene of every SCENE_CHUNK-th slot (several scenes only)
   void* run_arena = nullptr;              // lists, count words, control words
+  bool run_arena_own = false;             // an allocation of its own, not a part of part_arena
+  size_t run_bytes = 0;
   unsigned run_grid = 0;                  // CTAs: one wave, or fewer for a small scene
   bool run_own = false;                   // those CTAs have a thread for every sphere
   bool run_off = false;                   // ps_autotune times the step kernels
@@ -759,23 +763,46 @@ bool axis_bounds(T lo, T iv, int32_t nb, std::vector<T>& out) {
   return true;
 }
 
+// Cell boundaries of every scene and axis; sets the scenes' bnd_base.
 template <class T>
-int upload_bounds(ps_sim* s) {
-  std::vector<T> all;
+int collect_bounds(ps_sim* s, std::vector<SceneParams<T>>& sps, std::vector<T>& all) {
   for (int sc = 0; sc < s->n_scenes; ++sc) {
     const GridHost& g = s->grids[sc];
     for (int a = 0; a < 3; ++a) {
-      const uint32_t base = (uint32_t)all.size();
+      sps[sc].bnd_base[a] = (uint32_t)all.size();
       if (!axis_bounds<T>((T)g.min[a], (T)g.interval, g.nb[a], all))
         return fail(PS_ERR_INVALID, "cell boundary table is not monotonic on axis " + std::to_string(a));
-      if (s->precision == PS_FP32)
-        s->sp32[sc].bnd_base[a] = base;
-      else
-        s->sp64[sc].bnd_base[a] = base;
     }
   }
-  PS_CUDA(cudaMalloc(&s->d_bounds, sizeof(T) * all.size()));
-  PS_CUDA(cudaMemcpy(s->d_bounds, all.data(), sizeof(T) * all.size(), cudaMemcpyHostToDevice));
+  return PS_OK;
+}
+
+// The arrays that belong to a grid, in one allocation: counts, offsets and
+// tile totals (zeroed), then the boundaries and the scene parameters.
+template <class T>
+int upload_grids(ps_sim* s, std::vector<SceneParams<T>>& sps) {
+  sps.clear();
+  for (int sc = 0; sc < s->n_scenes; ++sc)
+    sps.push_back(make_params<T>(s->desc[sc], s->grids[sc], s->pbase[sc], s->pbase[sc + 1] - s->pbase[sc]));
+  std::vector<T> bounds;
+  const int rc = collect_bounds<T>(s, sps, bounds);
+  if (rc != PS_OK) return rc;
+  const size_t cells_b = align_up(sizeof(uint32_t) * (size_t)(s->c_total + 1), 256);
+  const size_t tiles_b = align_up(sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), 256);
+  const size_t bounds_b = align_up(sizeof(T) * bounds.size(), 256), scenes_b = sizeof(SceneParams<T>) * sps.size();
+  s->cell_bytes = 2 * cells_b + tiles_b;
+  PS_CUDA(cudaMalloc(&s->cell_arena, s->cell_bytes + bounds_b + scenes_b));
+  char* c = static_cast<char*>(s->cell_arena);
+  s->count = reinterpret_cast<uint32_t*>(c);
+  s->offset = reinterpret_cast<uint32_t*>(c + cells_b);
+  s->tile_sum = reinterpret_cast<uint32_t*>(c + 2 * cells_b);
+  s->d_bounds = c + s->cell_bytes;
+  s->d_scenes = c + s->cell_bytes + bounds_b;
+  PS_CUDA(cudaMemset(s->cell_arena, 0, s->cell_bytes));
+  std::vector<char> host(bounds_b + scenes_b);
+  std::memcpy(host.data(), bounds.data(), sizeof(T) * bounds.size());
+  std::memcpy(host.data() + bounds_b, sps.data(), scenes_b);
+  PS_CUDA(cudaMemcpy(s->d_bounds, host.data(), host.size(), cudaMemcpyHostToDevice));
   return PS_OK;
 }
 
@@ -949,6 +976,18 @@ void apply_l2_window(ps_sim* s, cudaGraph_t g, bool clear = false) {
   cudaGetLastError();
 }
 
+// The lists' memory (134 B per sphere, 198 B with triangles).  Up to
+// RUN_WITH_PARTICLES it is a part of the particles' allocation, more is one of
+// its own, unless it would be more than a quarter of what the device has left;
+// without it every call takes the step kernels.
+constexpr size_t RUN_WITH_PARTICLES = (size_t)64 << 20;
+
+size_t run_need(const ps_sim* s, int sms) {
+  const size_t n = (size_t)s->n_total, threads = (size_t)sms * 2048;  // the grid's threads at most
+  return 256 + align_up(2 * n, 256) + align_up(4 * n * RUN_LIST_CAP, 256) + align_up(4 * (n + threads), 256) +
+         (s->has_mesh ? 4 * n * RUN_TRI_CAP : 0);
+}
+
 void run_alloc(ps_sim* s);
 cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes);
 
@@ -1052,41 +1091,16 @@ int size_grids(ps_sim* s, const double* aos) {
   s->bins_total = bin_base;
   s->tri_total = tri_base;
 
-  // per-cell arrays and scan scratch
-  const size_t cells_b = align_up(sizeof(uint32_t) * (size_t)(s->c_total + 1), 256);
-  const size_t tiles_b = align_up(sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), 256);
-  PS_CUDA(cudaMalloc(&s->cell_arena, 2 * cells_b + tiles_b));
-  char* c = static_cast<char*>(s->cell_arena);
-  s->count = reinterpret_cast<uint32_t*>(c);
-  s->offset = reinterpret_cast<uint32_t*>(c + cells_b);
-  s->tile_sum = reinterpret_cast<uint32_t*>(c + 2 * cells_b);
-  PS_CUDA(cudaMemset(s->cell_arena, 0, 2 * cells_b + tiles_b));
-  s->cell_bytes = 2 * cells_b + tiles_b;
-
   {
     std::vector<double> iv((size_t)s->n_scenes);
     for (int sc = 0; sc < s->n_scenes; ++sc) iv[(size_t)sc] = s->grids[sc].interval;
     PS_CUDA(cudaMemcpy(s->d_interval, iv.data(), 8 * iv.size(), cudaMemcpyHostToDevice));
   }
 
-  // scene parameter tables
-  s->sp32.clear();
-  s->sp64.clear();
-  for (int sc = 0; sc < s->n_scenes; ++sc) {
-    const int64_t pc = s->pbase[sc + 1] - s->pbase[sc];
-    s->sp32.push_back(make_params<float>(s->desc[sc], s->grids[sc], s->pbase[sc], pc));
-    s->sp64.push_back(make_params<double>(s->desc[sc], s->grids[sc], s->pbase[sc], pc));
-  }
   {
-    const int rc = s->precision == PS_FP32 ? upload_bounds<float>(s) : upload_bounds<double>(s);
+    const int rc = s->precision == PS_FP32 ? upload_grids<float>(s, s->sp32) : upload_grids<double>(s, s->sp64);
     if (rc != PS_OK) return rc;
   }
-  const size_t spb = s->precision == PS_FP32 ? sizeof(SceneParams<float>) : sizeof(SceneParams<double>);
-  PS_CUDA(cudaMalloc(&s->d_scenes, spb * s->n_scenes));
-  if (s->precision == PS_FP32)
-    PS_CUDA(cudaMemcpy(s->d_scenes, s->sp32.data(), spb * s->n_scenes, cudaMemcpyHostToDevice));
-  else
-    PS_CUDA(cudaMemcpy(s->d_scenes, s->sp64.data(), spb * s->n_scenes, cudaMemcpyHostToDevice));
   if (s->has_mesh) {
     const int rc = s->precision == PS_FP32 ? upload_mesh<float>(s) : upload_mesh<double>(s);
     if (rc != PS_OK) return rc;
@@ -1097,12 +1111,11 @@ int size_grids(ps_sim* s, const double* aos) {
 }
 
 void free_sim(ps_sim* s) {
-  for (void* p : s->fwd_ckpt) cudaFree(p);
-  s->fwd_ckpt.clear();
+  cudaFree(s->fwd_arena);
   cudaFree(s->adj_arena);
   cudaFree(s->list_arena);
   cudaFree(s->list_ckpt);
-  cudaFree(s->run_arena);
+  if (s->run_arena_own) cudaFree(s->run_arena);
   if (s->l2_window_on) {
     cudaStreamAttrValue v{};
     v.accessPolicyWindow.num_bytes = 0;
@@ -1120,8 +1133,6 @@ void free_sim(ps_sim* s) {
   s->graphs.clear();
   cudaFree(s->part_arena);
   cudaFree(s->cell_arena);
-  cudaFree(s->d_scenes);
-  cudaFree(s->d_bounds);
   cudaFree(s->d_tri);
   cudaFree(s->d_aabb);
   cudaFree(s->d_bin_offset);
@@ -1389,8 +1400,13 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   const size_t b4 = align_up(vb * n, 256), bu = align_up(4 * n, 256), bs = align_up(64 * n, 256);
   const size_t bp = align_up(4 * (size_t)(n_scenes + 1), 256), bi = align_up(8 * (size_t)n_scenes, 256);
   const size_t chunks = s->multi ? n / SCENE_CHUNK + 2 : 0, bc = align_up(4 * chunks, 256);
-  cudaError_t e = cudaMalloc(&s->part_arena,
-                             4 * b4 + 5 * bu + bs + 256 + bp + bi + bc + 2 * sizeof(StatsPartial) * kStatsBlocks + 256);
+  int sms = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  s->run_bytes = s->n_total > 0 ? run_need(s, sms) : 0;
+  const size_t br = s->run_bytes <= RUN_WITH_PARTICLES ? align_up(s->run_bytes, 256) : 0;
+  if (e == cudaSuccess)
+    e = cudaMalloc(&s->part_arena,
+                   4 * b4 + 5 * bu + bs + 256 + bp + bi + bc + br + 2 * sizeof(StatsPartial) * kStatsBlocks + 256);
   if (e != cudaSuccess) {
     delete s;
     return fail(e == cudaErrorMemoryAllocation ? PS_ERR_NOMEM : PS_ERR_CUDA, std::string("ps_create: ") + cudaGetErrorString(e));
@@ -1410,6 +1426,8 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   s->d_pbase = reinterpret_cast<uint32_t*>(p); p += bp;
   s->d_interval = reinterpret_cast<double*>(p); p += bi;
   s->d_chunk_scene = reinterpret_cast<uint32_t*>(p); p += bc;
+  if (br > 0) s->run_arena = p;
+  p += br;
   s->d_stats = reinterpret_cast<StatsPartial*>(p); p += sizeof(StatsPartial) * kStatsBlocks;
   s->d_stats_out = reinterpret_cast<StatsPartial*>(p);
   std::vector<uint32_t> pb(n_scenes + 1);
@@ -1625,34 +1643,32 @@ int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
   return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false>(s, steps);
 }
 
-// The lists' memory (134 B per sphere, 198 B with triangles), unless it would be more than a
-// quarter of what the device has left (asked only where it is large: the
-// question takes as long as the allocation); without it every call takes the
-// step kernels.
 void run_alloc(ps_sim* s) {
   const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, 0, true) : run_dispatch<double>(s, 0, true);
-  if (rc != PS_OK) return;
-  const size_t n = (size_t)s->n_total;
-  const size_t need = 256 + align_up(2 * n, 256) + align_up(4 * n * RUN_LIST_CAP, 256) +
-                      align_up(4 * (size_t)s->run_grid * run_share(s), 256) + (s->has_mesh ? 4 * n * RUN_TRI_CAP : 0);
-  size_t left = 4 * need, total = 0;
-  if ((need > ((size_t)1 << 30) && cudaMemGetInfo(&left, &total) != cudaSuccess) || need > left / 4 ||
-      cudaMalloc(&s->run_arena, need) != cudaSuccess) {
-    cudaGetLastError();
-    s->run_arena = nullptr;
-    return;
+  if (rc == PS_OK && s->run_arena == nullptr && s->run_bytes > 0) {
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess || s->run_bytes > left / 4 ||
+        cudaMalloc(&s->run_arena, s->run_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      s->run_arena = nullptr;
+    }
+    s->run_arena_own = s->run_arena != nullptr;
   }
+  if (rc != PS_OK && !s->run_arena_own) s->run_arena = nullptr;
+  if (s->run_arena == nullptr) return;
   cudaMemsetAsync(s->run_arena, 0, 256, s->stream);
 }
 
 // For the library's own later allocations: the lists give way to them.
 cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && s->run_arena != nullptr) {
+  if (e == cudaErrorMemoryAllocation && s->run_arena_own) {
     cudaGetLastError();
     cudaStreamSynchronize(s->stream);
     cudaFree(s->run_arena);
     s->run_arena = nullptr;
+    s->run_arena_own = false;
+    s->run_bytes = 0;
     e = cudaMalloc(p, bytes);
   }
   return e;
@@ -1895,7 +1911,7 @@ namespace {
 int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
-  void** bufs_to_free[] = {&s->cell_arena, &s->d_scenes, &s->d_bounds, &s->d_tri, &s->d_aabb, &s->adj_arena};
+  void** bufs_to_free[] = {&s->cell_arena, &s->d_tri, &s->d_aabb, &s->adj_arena};
   for (void** b : bufs_to_free) {
     cudaFree(*b);
     *b = nullptr;
@@ -1907,8 +1923,6 @@ int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   s->d_mesh_view = nullptr;
   s->adj_bytes = 0;
   s->run_grid = 0;
-  cudaFree(s->run_arena);
-  s->run_arena = nullptr;
   s->run_seen = s->run_id;
   s->run_settled = s->run_known = false;
   s->fwd_steps = 0;
@@ -2156,8 +2170,18 @@ extern "C" int ps_forward_checkpointed(ps_sim* s, int64_t n_steps, int64_t every
   if (s->has_mesh) return fail(PS_ERR_INVALID, "ps_forward_checkpointed: differentiation supports box containers only");
   DeviceGuard guard(s->device);
   const int64_t n_blocks = (n_steps + every - 1) / every;
-  for (size_t k = (size_t)n_blocks + 1; k < s->fwd_ckpt.size(); ++k) cudaFree(s->fwd_ckpt[k]);
-  s->fwd_ckpt.resize((size_t)n_blocks + 1, nullptr);
+  const size_t ckpt_b = align_up(2 * state_bytes(s) + 4 * (size_t)s->n_total, 256);
+  const size_t need = std::max<size_t>(ckpt_b * (size_t)(n_blocks + 1), 256);
+  if (s->fwd_bytes < need || s->fwd_bytes / 2 > need) {  // (a much shorter pass gives the rest back)
+    s->fwd_steps = 0;
+    cudaFree(s->fwd_arena);
+    s->fwd_arena = nullptr;
+    s->fwd_bytes = 0;
+    PS_CUDA(dev_alloc(s, &s->fwd_arena, need));
+    s->fwd_bytes = need;
+  }
+  s->fwd_ckpt.assign((size_t)n_blocks + 1, nullptr);
+  for (size_t k = 0; k < s->fwd_ckpt.size(); ++k) s->fwd_ckpt[k] = static_cast<char*>(s->fwd_arena) + ckpt_b * k;
   for (int64_t blk = 0; blk < n_blocks; ++blk) {
     int rc = save_state(s, s->fwd_ckpt[(size_t)blk]);
     if (rc == PS_OK) rc = ps_step(s, std::min(every, n_steps - blk * every));
