@@ -1521,6 +1521,13 @@ extern "C" int ps_get_state(ps_sim* s, double* out, int64_t n_total) {
 
 namespace {
 
+// Spheres from which the step kernels of a block shorter than graph_block
+// are launched one by one: each then runs for longer than its launch takes,
+// so that a graph gains nothing, and capturing one takes 1.5 ms per hundred
+// steps (first 100 steps of a 1M-sphere scene FIRST_NOW).  Longer calls use
+// graphs, which also keep the call asynchronous.
+constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
+
 // Run n_steps as CUDA graphs of up to graph_block steps (grid path, or the
 // neighbour-list path when `lists`), asynchronously.
 int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
@@ -1531,6 +1538,13 @@ int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
   int64_t left = n_steps;
   while (left > 0) {
     const int64_t L = std::min(left, s->graph_block);
+    if (!lists && L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES) {
+      s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
+      PS_CUDA(cudaGetLastError());
+      s->last_launches += 1 + 4 * L;
+      left -= L;
+      continue;
+    }
     const int64_t key = lists ? (L | (int64_t(1) << 62)) : L;
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
