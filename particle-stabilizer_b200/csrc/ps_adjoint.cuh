@@ -28,21 +28,12 @@
 // forward values; radii and masses are constants.
 #pragma once
 
-#include "ps_step_kernels.cuh"
+#include "ps_run.cuh"
 
 namespace psb {
 
 enum : int { ADJ_K = 0, ADJ_E = 1, ADJ_WALL = 2 };  // acc rows: k, e_sphere, e_wall[6] (zMin..yMax)
 constexpr int ADJ_NACC = 8;
-
-template <class T>
-struct TapeRow {
-  vec4_t<T>* p;     // (x, r) per sorted slot
-  vec4_t<T>* v;     // (v, m)
-  vec4_t<T>* vpre;  // (v, m) before the contacts of the step that wrote the row
-  uint32_t* o;      // original id
-  uint32_t* cell;   // sorted cell id of that step's grid
-};
 
 template <class T>
 struct AdjBufs {
@@ -109,6 +100,50 @@ __device__ __forceinline__ bool pair_active(const vec4_t<T>& P, const vec4_t<T>&
   return A::sub(s, A::sqrt(d2)) > T(0);
 }
 
+// Both directions of the active pair (i, j): what j's part in the pair adds
+// to the adjoints (xo, vo) of i's position and velocity, G and H being the
+// adjoints of the two output velocities; the parameter partials of the
+// direction in which i receives (those of the other belong to j's thread).
+template <class T>
+__device__ __forceinline__ void adj_pair(const vec4_t<T>& P, const vec4_t<T>& V, const vec4_t<T>& G,
+                                         const vec4_t<T>& Pj, const vec4_t<T>& Vj, const vec4_t<T>& H, T k, T e,
+                                         vec4_t<T>& xo, vec4_t<T>& vo, double& dk, double& de) {
+  PairGeom<T> g;
+  g.dx = P.x - Pj.x;
+  g.dy = P.y - Pj.y;
+  g.dz = P.z - Pj.z;
+  g.ux = V.x - Vj.x;
+  g.uy = V.y - Vj.y;
+  g.uz = V.z - Vj.z;
+  g.R = P.w + Pj.w;
+  const T L2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
+  g.L = sqrt(L2);
+  g.iL = T(1) / g.L;
+  g.iL2 = T(1) / L2;
+  g.ov = g.R - g.L;
+  g.ud = g.ux * g.dx + g.uy * g.dy + g.uz * g.dz;
+  const T inv_msum = T(1) / (V.w + Vj.w);
+  T ddx, ddy, ddz, dux, duy, duz;
+  // i receives from j
+  pair_adjoint<T>(g, T(1), V.w, Vj.w, inv_msum, k, e, G.x, G.y, G.z, ddx, ddy, ddz, dux, duy, duz, dk, de);
+  xo.x += ddx;
+  xo.y += ddy;
+  xo.z += ddz;
+  vo.x += dux;
+  vo.y += duy;
+  vo.z += duz;
+  // j receives from i: that direction's d and u are -d and -u, so its
+  // adjoints with respect to the stored d and u come back sign-mapped
+  double dk2 = 0.0, de2 = 0.0;
+  pair_adjoint<T>(g, T(-1), Vj.w, V.w, inv_msum, k, e, H.x, H.y, H.z, ddx, ddy, ddz, dux, duy, duz, dk2, de2);
+  xo.x += ddx;
+  xo.y += ddy;
+  xo.z += ddz;
+  vo.x += dux;
+  vo.y += duy;
+  vo.z += duz;
+}
+
 template <class T, bool MULTI>
 __global__ void __launch_bounds__(STEP_THREADS) k_adj_contacts(StepBufs<T> b, AdjBufs<T> a, SceneParams<T> sp0) {
   // one wave of CTAs (occupancy x SMs, the host's choice) loops over the particles
@@ -119,9 +154,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_contacts(StepBufs<T> b, Ad
     const uint32_t oi = b.orig[i];
     a.inv[oi] = i;
     const vec4_t<T> G = a.av[i], X = a.ax[i];
-    const T gx = G.x, gy = G.y, gz = G.z;
-    T xb0 = X.x, xb1 = X.y, xb2 = X.z;
-    T vb0 = gx, vb1 = gy, vb2 = gz;
+    vec4_t<T> xo = X, vo = G;
     double dk = 0.0, de = 0.0;
     int32_t cx, cy, cz;
     cell_coords<T>(b.scell[i], sp, cx, cy, cz);
@@ -145,51 +178,8 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_contacts(StepBufs<T> b, Ad
         if (q == 4 && j == i) continue;  // only the own column holds the sphere itself
         const vec4_t<T> Pj = ld4<T>(b.P0 + j);
         if (!pair_active<T>(P, Pj)) continue;
-        const vec4_t<T> Vj = b.V0[j];
-        const vec4_t<T> H = a.av[j];
-        PairGeom<T> g;
-        g.dx = P.x - Pj.x;
-        g.dy = P.y - Pj.y;
-        g.dz = P.z - Pj.z;
-        g.ux = V.x - Vj.x;
-        g.uy = V.y - Vj.y;
-        g.uz = V.z - Vj.z;
-        g.R = P.w + Pj.w;
-        const T L2 = g.dx * g.dx + g.dy * g.dy + g.dz * g.dz;
-        g.L = sqrt(L2);
-        g.iL = T(1) / g.L;
-        g.iL2 = T(1) / L2;
-        g.ov = g.R - g.L;
-        g.ud = g.ux * g.dx + g.uy * g.dy + g.uz * g.dz;
-        const T inv_msum = T(1) / (V.w + Vj.w);
-        T ddx, ddy, ddz, dux, duy, duz;
-        // i receives from j
-        pair_adjoint<T>(g, T(1), V.w, Vj.w, inv_msum, k, e, gx, gy, gz, ddx, ddy, ddz, dux, duy, duz, dk, de);
-        xb0 += ddx;
-        xb1 += ddy;
-        xb2 += ddz;
-        vb0 += dux;
-        vb1 += duy;
-        vb2 += duz;
-        // j receives from i: that direction's d and u are -d and -u, so its
-        // adjoints with respect to the stored d and u come back sign-mapped;
-        // its parameter partials belong to j's own thread
-        double dk2 = 0.0, de2 = 0.0;
-        pair_adjoint<T>(g, T(-1), Vj.w, V.w, inv_msum, k, e, H.x, H.y, H.z, ddx, ddy, ddz, dux, duy, duz, dk2, de2);
-        xb0 += ddx;
-        xb1 += ddy;
-        xb2 += ddz;
-        vb0 += dux;
-        vb1 += duy;
-        vb2 += duz;
+        adj_pair<T>(P, V, G, Pj, b.V0[j], a.av[j], k, e, xo, vo, dk, de);
       }
-    vec4_t<T> xo = X, vo = G;
-    xo.x = xb0;
-    xo.y = xb1;
-    xo.z = xb2;
-    vo.x = vb0;
-    vo.y = vb1;
-    vo.z = vb2;
     a.ax2[i] = xo;
     a.av2[i] = vo;
     a.acc[(size_t)ADJ_K * a.n + i] += dk;
@@ -197,16 +187,13 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_contacts(StepBufs<T> b, Ad
   }
 }
 
-// Walls + integrate adjoint over the tape row's sorted slots.  The step
-// input (x, v) comes from the tape; x' and v' and the clamp events are
+// Walls + integrate adjoint of slot p of the tape row: (x, v) come in as the
+// adjoints of the post-wall state and leave as those of the step's input.
+// The input comes from the tape; x' and v' and the clamp events are
 // recomputed from it with the forward's operations.
-template <class T, bool MULTI>
-__global__ void __launch_bounds__(STEP_THREADS) k_adj_walls_integrate(StepBufs<T> b, AdjBufs<T> a,
-                                                                      SceneParams<T> sp0) {
-  const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
-  if (p >= b.n) return;
-  const SceneParams<T>& sp = scene_of<T, MULTI>(p, sp0, b);
-  const uint32_t o = a.tape.o[p];
+template <class T>
+__device__ __forceinline__ void adj_walls_integrate(const AdjBufs<T>& a, const SceneParams<T>& sp, uint32_t p,
+                                                    vec4_t<T>& x, vec4_t<T>& v) {
   vec4_t<T> P = a.tape.p[p];
   vec4_t<T> V = a.tape.v[p];
   integrate<T>(P, V, sp);  // x', v'
@@ -215,9 +202,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_walls_integrate(StepBufs<T
   const T xs[3] = {P.x, P.y, P.z}, vs[3] = {V.x, V.y, V.z};
   const int lo_idx[3] = {PS_XMIN, PS_YMIN, PS_ZMIN}, hi_idx[3] = {PS_XMAX, PS_YMAX, PS_ZMAX};
   double* acc = a.acc + p;  // row c at acc[c * n]
-  const uint32_t i = a.inv[o];  // this particle's slot in step t's grid
-  const vec4_t<T> X2 = a.ax2[i], V2 = a.av2[i];
-  const T xb2[3] = {X2.x, X2.y, X2.z}, vb2[3] = {V2.x, V2.y, V2.z};
+  const T xb2[3] = {x.x, x.y, x.z}, vb2[3] = {v.x, v.y, v.z};
   T xo[3], vo[3];
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
@@ -239,15 +224,96 @@ __global__ void __launch_bounds__(STEP_THREADS) k_adj_walls_integrate(StepBufs<T
     xo[ax] = xb;
     vo[ax] = vb + sp.dt * xb;
   }
-  vec4_t<T> xw = X2, vw = V2;
-  xw.x = xo[0];
-  xw.y = xo[1];
-  xw.z = xo[2];
-  vw.x = vo[0];
-  vw.y = vo[1];
-  vw.z = vo[2];
-  a.ax[p] = xw;
-  a.av[p] = vw;
+  x.x = xo[0];
+  x.y = xo[1];
+  x.z = xo[2];
+  v.x = vo[0];
+  v.y = vo[1];
+  v.z = vo[2];
+}
+
+// The same over all of the tape row's slots, from the order of step t's grid.
+template <class T, bool MULTI>
+__global__ void __launch_bounds__(STEP_THREADS) k_adj_walls_integrate(StepBufs<T> b, AdjBufs<T> a,
+                                                                      SceneParams<T> sp0) {
+  pdl_wait();
+  const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (p >= b.n) return;
+  const uint32_t i = a.inv[a.tape.o[p]];  // this particle's slot in step t's grid
+  vec4_t<T> x = a.ax2[i], v = a.av2[i];
+  adj_walls_integrate<T>(a, scene_of<T, MULTI>(p, sp0, b), p, x, v);
+  a.ax[p] = x;
+  a.av[p] = v;
+}
+
+// The reverse of a step that a recorded run took on lists (ps_run.cuh): row
+// t + 1 holds what its contacts read, in the order of the build `list`
+// belongs to, and the list's pairs take the place of the 27-cell walk (65,536
+// spheres in contact, FP32: 19.1 us as a walk).  FUSED: row t is in the same order, so
+// the walls and the integration follow at once and (ax, av) goes to
+// (ax2, av2); else (ax2, av2) and inv are for k_adj_walls_integrate.
+template <class T, bool MULTI, bool FUSED>
+__global__ void __launch_bounds__(STEP_THREADS) k_adj_list(StepBufs<T> b, AdjBufs<T> a, SceneParams<T> sp0,
+                                                           const uint32_t* __restrict__ list,
+                                                           const uint16_t* __restrict__ cnt) {
+  pdl_wait();
+  const uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (i >= b.n) return;
+  const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
+  const vec4_t<T> P = b.P0[i], V = b.V0[i], G = a.av[i], X = a.ax[i];
+  const uint32_t nl = cnt[i] & RUN_COUNT;
+  if (!FUSED) a.inv[b.orig[i]] = i;
+  vec4_t<T> xo = X, vo = G;
+  double dk = 0.0, de = 0.0;
+  constexpr int NB = 4;  // pairs whose loads go together
+  for (uint32_t k0 = 0; k0 < nl; k0 += NB) {
+    uint32_t jj[NB];
+    vec4_t<T> Q[NB];
+    bool act[NB];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) jj[u] = k0 + u < nl ? list[(size_t)(k0 + u) * b.n + i] : i;
+#pragma unroll
+    for (int u = 0; u < NB; ++u) Q[u] = ld4<T>(b.P0 + (jj[u] & ~RUN_FAR_CELL));
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      act[u] = k0 + u < nl && pair_active<T>(P, Q[u]);
+      if (act[u] && (jj[u] & RUN_FAR_CELL)) {  // the walk's own condition, which rounding can make stricter
+        int32_t cx, cy, cz, jx, jy, jz;
+        cell_of<T>(P.x, P.y, P.z, sp, cx, cy, cz);
+        cell_of<T>(Q[u].x, Q[u].y, Q[u].z, sp, jx, jy, jz);
+        act[u] = abs(jx - cx) <= 1 && abs(jy - cy) <= 1 && abs(jz - cz) <= 1;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u)
+      if (act[u]) {
+        const uint32_t j = jj[u] & ~RUN_FAR_CELL;
+        adj_pair<T>(P, V, G, Q[u], ld4<T>(b.V0 + j), ld4<T>(a.av + j), sp.k_spring, sp.e_sphere, xo, vo, dk, de);
+      }
+  }
+  a.acc[(size_t)ADJ_K * a.n + i] += dk;
+  a.acc[(size_t)ADJ_E * a.n + i] += de;
+  if constexpr (FUSED) adj_walls_integrate<T>(a, sp, i, xo, vo);
+  a.ax2[i] = xo;
+  a.av2[i] = vo;
+}
+
+// Adjoints from the order of one state (inverse permutation `inv` of its
+// original ids) to that of another (`o`).
+template <class T>
+__global__ void k_adj_reorder(const vec4_t<T>* __restrict__ ax, const vec4_t<T>* __restrict__ av,
+                              const uint32_t* __restrict__ inv, const uint32_t* __restrict__ o, vec4_t<T>* ax2,
+                              vec4_t<T>* av2, uint32_t n) {
+  const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (p >= n) return;
+  const uint32_t i = inv[o[p]];
+  ax2[p] = ax[i];
+  av2[p] = av[i];
+}
+
+__global__ void k_adj_invert(const uint32_t* __restrict__ o, uint32_t* inv, uint32_t n) {
+  const uint32_t p = blockIdx.x * STEP_THREADS + threadIdx.x;
+  if (p < n) inv[o[p]] = p;
 }
 
 // Copy the at-rest state (P0, V1, orig) into a tape row.

@@ -158,6 +158,7 @@ struct ps_sim {
   void* fwd_arena = nullptr;
   size_t fwd_bytes = 0;
   void* adj_arena = nullptr;              // tape, adjoint arrays, partials
+  int record_skip = 0;                    // backward passes left that do not record runs
   size_t adj_bytes = 0;
   // neighbour-list mode (ps_set_neighbor_lists); off when list_skin <= 0
   double list_skin = 0.0;                 // skin as a fraction of the cell edge
@@ -1141,6 +1142,92 @@ void free_sim(ps_sim* s) {
   if (s->stream) cudaStreamDestroy(s->stream);
 }
 
+// ---- many steps in one launch ------------------------------------------------
+// Steps a launch covers: a launch starts with a rebuild (0.2 ms at 1M
+// spheres, 1 us a step over 512), and stays below a second or so.
+int64_t run_block(const ps_sim* s) {
+  return std::min<int64_t>(512, std::max<int64_t>(32, (int64_t)2000000000 / std::max<int64_t>(s->n_total, 1)));
+}
+
+// Spheres of one CTA of the run kernel.
+uint32_t run_share(const ps_sim* s) {
+  const int64_t stride = (int64_t)s->run_grid * STEP_THREADS;
+  return (uint32_t)((s->n_total + stride - 1) / stride) * STEP_THREADS;
+}
+
+template <class T>
+RunBufs<T> run_bufs(ps_sim* s) {
+  const size_t n = (size_t)s->n_total;
+  RunBufs<T> R;
+  R.P[0] = static_cast<vec4_t<T>*>(s->P0);
+  R.P[1] = static_cast<vec4_t<T>*>(s->P1);
+  R.V[0] = static_cast<vec4_t<T>*>(s->V0);
+  R.V[1] = static_cast<vec4_t<T>*>(s->V1);
+  char* p = static_cast<char*>(s->run_arena);
+  R.ctl = reinterpret_cast<uint32_t*>(p);
+  p += 256;
+  R.cnt = reinterpret_cast<uint16_t*>(p);
+  p += align_up(2 * n, 256);
+  R.list = reinterpret_cast<uint32_t*>(p);
+  p += align_up(4 * n * RUN_LIST_CAP, 256);
+  R.later = reinterpret_cast<uint32_t*>(p);
+  R.later_stride = run_share(s);
+  p += align_up(4 * (size_t)s->run_grid * R.later_stride, 256);
+  R.tris = s->has_mesh ? reinterpret_cast<uint32_t*>(p) : nullptr;
+  R.cap = RUN_LIST_CAP;
+  R.tape = nullptr;
+  R.tape_row_bytes = 0;
+  R.tape_build = nullptr;
+  R.max_builds = 0;
+  R.report = s->err + ERR_RUN;
+  return R;
+}
+
+template <class T, bool MULTI, bool MESH>
+int run_prepare(ps_sim* s) {
+  int per_sm = 0, sms = 0;
+  PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, true, false>, STEP_THREADS, 0));
+  s->run_own = (int64_t)blocks_for(s->n_total) <= (int64_t)per_sm * sms;
+  if (!s->run_own)
+    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, false, false>, STEP_THREADS, 0));
+  if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_step: the run kernel cannot be resident");
+  s->run_grid = std::min<unsigned>((unsigned)(per_sm * sms),
+                                   std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
+  return PS_OK;
+}
+
+template <class T, bool MULTI, bool MESH, bool TAPE>
+int run_launch(ps_sim* s, uint32_t steps, const RunBufs<T>& R, uint32_t run_id) {
+  const StepBufs<T> b = bufs<T>(s);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(s->run_grid);
+  cfg.blockDim = dim3(STEP_THREADS);
+  cfg.stream = s->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  // the cell arrays are read by rebuilds alone: not the stream's window, which keeps them in L2
+  at[1].id = cudaLaunchAttributeAccessPolicyWindow;
+  at[1].val.accessPolicyWindow = cudaAccessPolicyWindow{};
+  cfg.attrs = at;
+  cfg.numAttrs = s->l2_window_on ? 2 : 1;
+  PS_CUDA(cudaLaunchKernelEx(&cfg, s->run_own ? k_run<T, MULTI, MESH, true, TAPE> : k_run<T, MULTI, MESH, false, TAPE>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
+                             R, steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
+                             (uint32_t)move_blocks(s->n_total, 0), run_id));
+  return PS_OK;
+}
+
+template <class T>
+int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
+  if (s->multi) {
+    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+  }
+  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+}
+
 // ---- differentiation -----------------------------------------------------------
 size_t state_bytes(const ps_sim* s) { return (size_t)(s->precision == PS_FP32 ? 16 : 32) * (size_t)s->n_total; }
 
@@ -1190,20 +1277,6 @@ __global__ void k_adj_download(const vec4_t<T>* ax, const vec4_t<T>* av, const u
   q[3] = (double)v.x; q[4] = (double)v.y; q[5] = (double)v.z;
 }
 
-// Tape row t of a block: the at-rest state after t steps in sorted order;
-// rows t >= 1 also hold step t-1's grid (pre-contact velocities, cell ids).
-template <class T>
-TapeRow<T> tape_row(char* base, size_t row_bytes, int64_t n, int64_t t) {
-  TapeRow<T> r;
-  char* p = base + row_bytes * (size_t)t;
-  r.p = reinterpret_cast<vec4_t<T>*>(p);
-  r.v = r.p + n;
-  r.vpre = r.v + n;
-  r.o = reinterpret_cast<uint32_t*>(r.vpre + n);
-  r.cell = r.o + n;
-  return r;
-}
-
 size_t tape_row_bytes(size_t vec_bytes, int64_t n) {
   return align_up((3 * vec_bytes + 2 * sizeof(uint32_t)) * (size_t)n, 256);
 }
@@ -1247,13 +1320,45 @@ int enqueue_steps_taped(ps_sim* s, int64_t steps, char* tape, size_t row_bytes, 
   return PS_OK;
 }
 
+// Recording a block on lists: builds a block may make (its lists are kept,
+// 130 B per sphere each).  A block that needs more, or moves too fast for
+// lists, is recomputed step by step on the grid (enqueue_steps_taped).
+// After a pass with such a block the next RECORD_SKIP passes do not try.
+constexpr uint32_t TAPE_BUILDS = 3;
+constexpr int RECORD_SKIP = 8;
+
+// Recompute `steps` steps of a block as a recorded run; false if it gave up.
+template <class T, bool MULTI>
+int record_run(ps_sim* s, int64_t steps, char* tape, size_t row_bytes, char* lists, std::vector<uint32_t>& build, bool& ok) {
+  const size_t n = (size_t)s->n_total;
+  RunBufs<T> R = run_bufs<T>(s);
+  R.tape = tape;
+  R.tape_row_bytes = row_bytes;
+  R.max_builds = TAPE_BUILDS;
+  R.tape_build = reinterpret_cast<uint32_t*>(lists);
+  lists += align_up(4 * (size_t)(steps + 1), 256);
+  R.cnt = reinterpret_cast<uint16_t*>(lists);
+  R.list = reinterpret_cast<uint32_t*>(lists + align_up(2 * n * TAPE_BUILDS, 256));
+  PS_CUDA(cudaMemsetAsync(R.tape_build + steps, 0, sizeof(uint32_t), s->stream));
+  const int rc = run_launch<T, MULTI, false, true>(s, (uint32_t)steps, R, s->run_id);
+  if (rc != PS_OK) return rc;
+  build.resize((size_t)steps + 1);
+  PS_CUDA(cudaMemcpyAsync(build.data(), R.tape_build, 4 * build.size(), cudaMemcpyDeviceToHost, s->stream));
+  PS_CUDA(cudaStreamSynchronize(s->stream));
+  ok = build[(size_t)steps] == 1u;
+  if (!ok) {  // what the run left in the middle: counts and control words
+    PS_CUDA(cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)n_scan(s), s->stream));
+    PS_CUDA(cudaMemsetAsync(s->tile_sum, 0, sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), s->stream));
+    PS_CUDA(cudaMemsetAsync(R.ctl, 0, 256, s->stream));
+  }
+  return PS_OK;
+}
+
 template <class T, bool MULTI>
 int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl_dstate0) {
-  const int64_t n = s->n_total, K = s->fwd_every;
+  const int64_t n = s->n_total, K = std::min(s->fwd_every, s->fwd_steps);
   const size_t row_b = tape_row_bytes(sizeof(vec4_t<T>), n);
   const size_t tape_b = row_b * (size_t)(K + 1);                 // rows 0..K
-  const size_t offs_stride = align_up(sizeof(uint32_t) * (size_t)n_scan(s), 256) / sizeof(uint32_t);
-  const size_t offs_b = sizeof(uint32_t) * offs_stride * (size_t)K;  // cell offsets of each step's grid
   const size_t adj_b = align_up(sizeof(vec4_t<T>) * (size_t)n, 256);
   const size_t acc_b = align_up(ADJ_NACC * sizeof(double) * (size_t)n, 256);
   const size_t io_b = align_up(6 * sizeof(double) * (size_t)n, 256);
@@ -1265,30 +1370,30 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
   const size_t n_sums = (size_t)ADJ_NACC * (size_t)s->n_scenes;
   const size_t red_b = align_up(sizeof(double) * n_sums, 256) + align_up(sizeof(double) * n_sums * (size_t)shares, 256);
   const size_t inv_b = align_up(sizeof(uint32_t) * (size_t)n, 256);
-  const size_t need = tape_b + offs_b + 4 * adj_b + inv_b + acc_b + io_b + red_b;
-  if (s->adj_bytes < need) {
+  const size_t lists_b = align_up(4 * (size_t)(K + 1), 256) + align_up(2 * (size_t)n * TAPE_BUILDS, 256) +
+                         align_up(4 * (size_t)n * RUN_LIST_CAP * TAPE_BUILDS, 256);
+  // The lists of recorded runs, or the cell offsets of every step's grid;
+  // the second only when a block needs them.
+  const size_t offs_stride = align_up(sizeof(uint32_t) * (size_t)n_scan(s), 256) / sizeof(uint32_t);
+  const size_t offs_b = sizeof(uint32_t) * offs_stride * (size_t)K;
+  bool record = s->run_arena != nullptr && !s->run_off && K >= RUN_MIN_STEPS && s->record_skip == 0;
+  if (s->record_skip > 0) --s->record_skip;
+  const size_t base = tape_b + 4 * adj_b + inv_b + acc_b + io_b + red_b;
+  auto reserve = [&](size_t need) -> cudaError_t {
+    if (s->adj_bytes >= need) return cudaSuccess;
     cudaFree(s->adj_arena);
     s->adj_arena = nullptr;
     s->adj_bytes = 0;
-    PS_CUDA(dev_alloc(s, &s->adj_arena, need));
-    s->adj_bytes = need;
+    const cudaError_t e = dev_alloc(s, &s->adj_arena, need);
+    if (e == cudaSuccess) s->adj_bytes = need;
+    return e;
+  };
+  if (record && reserve(base + lists_b) != cudaSuccess) {
+    cudaGetLastError();
+    record = false;
   }
-  char* p = static_cast<char*>(s->adj_arena);
-  char* tape = p;
-  p += tape_b;
-  uint32_t* offs = reinterpret_cast<uint32_t*>(p);
-  p += offs_b;
-  AdjBufs<T> a;
-  a.tape = tape_row<T>(tape, row_b, n, 0);
-  a.ax = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
-  a.av = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
-  a.ax2 = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
-  a.av2 = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
-  a.inv = reinterpret_cast<uint32_t*>(p); p += inv_b;
-  a.acc = reinterpret_cast<double*>(p); p += acc_b;
-  a.n = (uint32_t)n;
-  double* io = reinterpret_cast<double*>(p); p += io_b;
-  double* red = reinterpret_cast<double*>(p);
+  record = record && s->run_arena != nullptr;  // (the allocation may have taken the lists' memory)
+  if (!record) PS_CUDA(reserve(base + offs_b));
   cudaStream_t st = s->stream;
   const unsigned gp = blocks_for(n);
   unsigned adj_grid = 0;  // one wave of k_adj_contacts, which loops over the particles
@@ -1299,23 +1404,67 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
     if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_backward: the adjoint contact kernel cannot be resident");
     adj_grid = (unsigned)(per_sm * sms);
   }
-  // the final state's order (recomputing the last block reproduces it exactly)
-  int rc0 = load_state(s, s->fwd_ckpt.back());
-  if (rc0 != PS_OK) return rc0;
+  char* p = static_cast<char*>(s->adj_arena);
+  char* tape = p;
+  p += tape_b;
+  AdjBufs<T> a;
+  a.ax = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
+  a.av = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
+  a.ax2 = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
+  a.av2 = reinterpret_cast<vec4_t<T>*>(p); p += adj_b;
+  a.inv = reinterpret_cast<uint32_t*>(p); p += inv_b;
+  a.acc = reinterpret_cast<double*>(p); p += acc_b;
+  a.n = (uint32_t)n;
+  double* io = reinterpret_cast<double*>(p); p += io_b;
+  double* red = reinterpret_cast<double*>(p); p += red_b;
+  char* lists = p;                                      // of a recorded block, or
+  uint32_t* offs = reinterpret_cast<uint32_t*>(p);      // the cell offsets of a block's steps
+  void* offs_own = nullptr;                             // where the arena is laid out for lists
+  struct FreeOffs {
+    void*& p;
+    ~FreeOffs() { cudaFree(p); }
+  } free_offs{offs_own};
   PS_CUDA(cudaMemcpyAsync(io, dl_dstate, 6 * sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, st));
-  k_adj_upload<T><<<gp, STEP_THREADS, 0, st>>>(io, s->orig, a.ax, a.av, (uint32_t)n);
   PS_CUDA(cudaMemsetAsync(a.acc, 0, acc_b, st));
   const SceneParams<T> sp0 = params<T>(s)[0];
   const int64_t n_blocks = (s->fwd_steps + K - 1) / K;
+  std::vector<uint32_t> build;
   for (int64_t blk = n_blocks - 1; blk >= 0; --blk) {
     const int64_t kb = std::min(K, s->fwd_steps - blk * K);
-    int rc = load_state(s, s->fwd_ckpt[(size_t)blk]);
-    if (rc != PS_OK) return rc;
-    // recompute the block, recording each step's input and grid (row 0 = block start)
-    k_tape_write<T><<<gp, STEP_THREADS, 0, st>>>(bufs<T>(s), tape_row<T>(tape, row_b, n, 0));
-    rc = enqueue_steps_taped<T, MULTI>(s, kb, tape, row_b, offs, offs_stride);
-    if (rc != PS_OK) return rc;
-    PS_CUDA(cudaGetLastError());
+    // recompute the block, recording each step's input and pairs (row 0 = block start)
+    bool on_lists = false;
+    for (int attempt = record ? 0 : 1; attempt < 2 && !on_lists; ++attempt) {
+      int rc = load_state(s, s->fwd_ckpt[(size_t)blk]);
+      if (rc != PS_OK) return rc;
+      k_tape_write<T><<<gp, STEP_THREADS, 0, st>>>(bufs<T>(s), tape_row<T>(tape, row_b, n, 0));
+      if (attempt == 0) {
+        rc = record_run<T, MULTI>(s, kb, tape, row_b, lists, build, on_lists);
+      } else {
+        if (record && offs_own == nullptr && s->adj_bytes < base + offs_b) {
+          PS_CUDA(dev_alloc(s, &offs_own, offs_b));
+          offs = static_cast<uint32_t*>(offs_own);
+        }
+        rc = enqueue_steps_taped<T, MULTI>(s, kb, tape, row_b, offs, offs_stride);
+        if (record) s->record_skip = RECORD_SKIP;
+        record = record && s->run_arena != nullptr;
+      }
+      if (rc != PS_OK) return rc;
+      PS_CUDA(cudaGetLastError());
+    }
+    // the adjoints in the order in which the block ends
+    const uint32_t* end_order = tape_row<T>(tape, row_b, n, kb).o;
+    if (blk == n_blocks - 1) {
+      k_adj_upload<T><<<gp, STEP_THREADS, 0, st>>>(io, end_order, a.ax, a.av, (uint32_t)n);
+    } else {
+      const char* ck = static_cast<const char*>(s->fwd_ckpt[(size_t)blk + 1]);
+      k_adj_invert<<<gp, STEP_THREADS, 0, st>>>(reinterpret_cast<const uint32_t*>(ck + 2 * state_bytes(s)), a.inv, (uint32_t)n);
+      k_adj_reorder<T><<<gp, STEP_THREADS, 0, st>>>(a.ax, a.av, a.inv, end_order, a.ax2, a.av2, (uint32_t)n);
+      std::swap(a.ax, a.ax2);
+      std::swap(a.av, a.av2);
+    }
+    const uint16_t* cnt0 = reinterpret_cast<const uint16_t*>(lists + align_up(4 * (size_t)(kb + 1), 256));
+    const uint32_t* list0 = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(cnt0) +
+                                                              align_up(2 * (size_t)n * TAPE_BUILDS, 256));
     for (int64_t t = kb - 1; t >= 0; --t) {
       // step t's sorted post-wall state and grid: row t + 1 and offsets t
       const TapeRow<T> g = tape_row<T>(tape, row_b, n, t + 1);
@@ -1324,12 +1473,25 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
       b.V0 = g.vpre;
       b.orig = g.o;
       b.scell = g.cell;
-      b.offset = offs + offs_stride * (size_t)t;
       a.tape = tape_row<T>(tape, row_b, n, t);
-      k_adj_contacts<T, MULTI><<<std::min(gp, adj_grid), STEP_THREADS, 0, st>>>(b, a, sp0);
-      k_adj_walls_integrate<T, MULTI><<<gp, STEP_THREADS, 0, st>>>(b, a, sp0);
-      PS_CUDA(cudaGetLastError());
+      if (on_lists) {
+        const size_t e = build[(size_t)t];
+        const uint32_t* list = list0 + e * RUN_LIST_CAP * (size_t)n;
+        const uint16_t* cnt = cnt0 + e * (size_t)n;
+        if (t > 0 && build[(size_t)t - 1] == build[(size_t)t]) {
+          pdl_launch(k_adj_list<T, MULTI, true>, gp, STEP_THREADS, st, b, a, sp0, list, cnt);
+          std::swap(a.ax, a.ax2);
+          std::swap(a.av, a.av2);
+          continue;
+        }
+        pdl_launch(k_adj_list<T, MULTI, false>, gp, STEP_THREADS, st, b, a, sp0, list, cnt);
+      } else {
+        b.offset = offs + offs_stride * (size_t)t;
+        k_adj_contacts<T, MULTI><<<std::min(gp, adj_grid), STEP_THREADS, 0, st>>>(b, a, sp0);
+      }
+      pdl_launch(k_adj_walls_integrate<T, MULTI>, gp, STEP_THREADS, st, b, a, sp0);
     }
+    PS_CUDA(cudaGetLastError());
   }
   double* share_sums = red + align_up(sizeof(double) * n_sums, 256) / sizeof(double);
   for (int s0 = 0; s0 < s->n_scenes; s0 += 65535)
@@ -1524,7 +1686,8 @@ namespace {
 // Spheres from which the step kernels of a block shorter than graph_block
 // are launched one by one: each then runs for longer than its launch takes,
 // so that a graph gains nothing, and capturing one takes 1.5 ms per hundred
-// steps (first 100 steps of a 1M-sphere scene FIRST_NOW).  Longer calls use
+// steps (first 100 steps of a 1M-sphere scene
+// and download: 11.6 ms with a graph, 10.3 ms without).  Longer calls use
 // graphs, which also keep the call asynchronous.
 constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
 
@@ -1573,88 +1736,6 @@ int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
     left -= L;
   }
   return PS_OK;
-}
-
-// ---- many steps in one launch ------------------------------------------------
-// Steps a launch covers: a launch starts with a rebuild (0.2 ms at 1M
-// spheres, 1 us a step over 512), and stays below a second or so.
-int64_t run_block(const ps_sim* s) {
-  return std::min<int64_t>(512, std::max<int64_t>(32, (int64_t)2000000000 / std::max<int64_t>(s->n_total, 1)));
-}
-
-// Spheres of one CTA of the run kernel.
-uint32_t run_share(const ps_sim* s) {
-  const int64_t stride = (int64_t)s->run_grid * STEP_THREADS;
-  return (uint32_t)((s->n_total + stride - 1) / stride) * STEP_THREADS;
-}
-
-template <class T>
-RunBufs<T> run_bufs(ps_sim* s) {
-  const size_t n = (size_t)s->n_total;
-  RunBufs<T> R;
-  R.P[0] = static_cast<vec4_t<T>*>(s->P0);
-  R.P[1] = static_cast<vec4_t<T>*>(s->P1);
-  R.V[0] = static_cast<vec4_t<T>*>(s->V0);
-  R.V[1] = static_cast<vec4_t<T>*>(s->V1);
-  char* p = static_cast<char*>(s->run_arena);
-  R.ctl = reinterpret_cast<uint32_t*>(p);
-  p += 256;
-  R.cnt = reinterpret_cast<uint16_t*>(p);
-  p += align_up(2 * n, 256);
-  R.list = reinterpret_cast<uint32_t*>(p);
-  p += align_up(4 * n * RUN_LIST_CAP, 256);
-  R.later = reinterpret_cast<uint32_t*>(p);
-  R.later_stride = run_share(s);
-  p += align_up(4 * (size_t)s->run_grid * R.later_stride, 256);
-  R.tris = s->has_mesh ? reinterpret_cast<uint32_t*>(p) : nullptr;
-  R.cap = RUN_LIST_CAP;
-  R.report = s->err + ERR_RUN;
-  return R;
-}
-
-template <class T, bool MULTI, bool MESH>
-int run_prepare(ps_sim* s) {
-  int per_sm = 0, sms = 0;
-  PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, true>, STEP_THREADS, 0));
-  s->run_own = (int64_t)blocks_for(s->n_total) <= (int64_t)per_sm * sms;
-  if (!s->run_own)
-    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, false>, STEP_THREADS, 0));
-  if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_step: the run kernel cannot be resident");
-  s->run_grid = std::min<unsigned>((unsigned)(per_sm * sms),
-                                   std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
-  return PS_OK;
-}
-
-template <class T, bool MULTI, bool MESH>
-int run_launch(ps_sim* s, uint32_t steps) {
-  const StepBufs<T> b = bufs<T>(s);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(s->run_grid);
-  cfg.blockDim = dim3(STEP_THREADS);
-  cfg.stream = s->stream;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  // the cell arrays are read by rebuilds alone: not the stream's window, which keeps them in L2
-  at[1].id = cudaLaunchAttributeAccessPolicyWindow;
-  at[1].val.accessPolicyWindow = cudaAccessPolicyWindow{};
-  cfg.attrs = at;
-  cfg.numAttrs = s->l2_window_on ? 2 : 1;
-  PS_CUDA(cudaLaunchKernelEx(&cfg, s->run_own ? k_run<T, MULTI, MESH, true> : k_run<T, MULTI, MESH, false>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
-                             run_bufs<T>(s), steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
-                             (uint32_t)move_blocks(s->n_total, 0), ++s->run_id));
-  return PS_OK;
-}
-
-template <class T>
-int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
-  if (s->multi) {
-    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true>(s, steps);
-    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false>(s, steps);
-  }
-  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true>(s, steps);
-  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false>(s, steps);
 }
 
 void run_alloc(ps_sim* s) {

@@ -52,7 +52,7 @@ constexpr uint32_t RUN_LIST_CAP = 32;
 constexpr float RUN_CALM_MAX = 0.05f;
 constexpr uint32_t RUN_CALM_STEPS = 2;
 constexpr float RUN_STEPS_PER_BUILD = 64.0f;
-constexpr float RUN_SKIN_MIN = 0.02f, RUN_SKIN_MAX = 0.25f;
+constexpr float RUN_SKIN_MIN = 0.02f, RUN_SKIN_MAX = 0.25f, RUN_SKIN_FIRST = 0.06f;
 
 // count word of a sphere: list length and what its step needs besides
 enum : uint32_t {
@@ -73,6 +73,7 @@ enum : int {
   RUN_STREAK = 5,   // calm steps up to now
   RUN_RMAX = 6,     // largest radius, in cells of its scene
   RUN_BEFORE = 7,   // largest displacement of the last step, in cells (0: none yet)
+  RUN_FULL = 8,     // a recorded run met a sphere with more neighbours than a list holds
 };
 
 template <class T>
@@ -84,11 +85,27 @@ struct RunBufs {
   uint32_t* tris;       // [k][slot]: triangles within reach (triangle containers)
   uint32_t* later;      // per CTA: the slots of its RunLate beyond what fits in shared memory
   uint32_t* ctl;
+  // recording for the backward pass (null otherwise): rows of the tape, one
+  // list and count array per build (max_builds of them), the build of every
+  // step, and after them 1 when the run is complete
+  char* tape;
+  size_t tape_row_bytes;
+  uint32_t* tape_build;
+  uint32_t max_builds;
   uint32_t* report;     // number of the last run, and whether it rebuilt too often
   uint32_t cap;
   uint32_t later_stride;  // entries of `later` per CTA
   __device__ __forceinline__ vec4_t<T>* p(int k) const { return k ? P[1] : P[0]; }
   __device__ __forceinline__ vec4_t<T>* v(int k) const { return k ? V[1] : V[0]; }
+  // list and count words of build `build` (one only unless recording)
+  template <bool TAPE>
+  __device__ __forceinline__ uint32_t* lists(uint32_t build, uint32_t n) const {
+    return TAPE ? list + (size_t)build * cap * n : list;
+  }
+  template <bool TAPE>
+  __device__ __forceinline__ uint16_t* counts(uint32_t build, uint32_t n) const {
+    return TAPE ? cnt + (size_t)build * n : cnt;
+  }
 };
 
 // One phase's end for the whole grid.  Arrivals only ever count up, by
@@ -186,6 +203,17 @@ __device__ __forceinline__ Span<T> reach_span(const vec4_t<T>& P, T reach, const
   return s;
 }
 
+// Row s + 1 of the tape: sphere i's state after step s's contacts.
+template <class T>
+__device__ __forceinline__ void run_record(const RunBufs<T>& R, const StepBufs<T>& b, uint32_t s, uint32_t i,
+                                           const vec4_t<T>& P, const vec4_t<T>& V, const vec4_t<T>& Vi) {
+  const TapeRow<T> row = tape_row<T>(R.tape, R.tape_row_bytes, b.n, (int64_t)s + 1);
+  row.p[i] = P;
+  row.v[i] = V;
+  row.vpre[i] = Vi;
+  row.o[i] = b.orig[i];
+}
+
 // Candidates whose positions are fetched together.
 template <class T>
 __host__ __device__ constexpr int run_batch() {
@@ -195,10 +223,11 @@ __host__ __device__ constexpr int run_batch() {
 // List and count word of slot i of the sorted state (positions P, sorted
 // cell ids scell); columns are visited in ascending cell id, so a list is in
 // ascending (cell, original index).
-template <class T, bool MULTI, bool MESH>
+template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, const SceneParams<T>& sp,
                                               const MeshView* mv, const RunBufs<T>& R, const vec4_t<T>* Ps, T frac,
-                                              T rmax) {
+                                              T rmax, uint32_t build) {
+  uint32_t* const list = R.template lists<TAPE>(build, b.n);
   const vec4_t<T> P = Ps[i];
   const T skin = frac * sp.interval;
   uint32_t k = 0, word = 0;
@@ -220,7 +249,7 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
             cell_coords<T>(b.scell[j], sp, jx, jy, jz);
             if (abs(jx - cx) > 1 || abs(jy - cy) > 1 || abs(jz - cz) > 1) entry |= RUN_FAR_CELL;
           }
-          R.list[(size_t)k * b.n + i] = entry;
+          list[(size_t)k * b.n + i] = entry;
         }
         ++k;
       }
@@ -267,8 +296,11 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
       }
     }
   }
-  if (k > R.cap) word |= RUN_OVERFLOW, k = 0;
-  R.cnt[i] = (uint16_t)(word | k);
+  if (k > R.cap) {
+    word |= RUN_OVERFLOW, k = 0;
+    if (TAPE) R.ctl[RUN_FULL] = 1u;
+  }
+  R.template counts<TAPE>(build, b.n)[i] = (uint16_t)(word | k);
 }
 
 // Contacts of slot i in the exact order whatever has moved: the overlapping
@@ -391,10 +423,10 @@ __device__ __noinline__ void run_begin(const StepBufs<T>& b, const SceneParams<T
 
 // Grid of the state in buffer `cur`, sorted into the other one, and with
 // frac > 0 its lists.  False: a barrier gave up.
-template <class T, bool MULTI, bool MESH>
+template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
-                                         const RunBufs<T>& R, int cur, bool counted, float frac, int64_t n_cells,
-                                         uint32_t scatter_blocks, uint32_t move_blocks) {
+                                         const RunBufs<T>& R, int cur, bool counted, float frac, uint32_t build,
+                                         int64_t n_cells, uint32_t scatter_blocks, uint32_t move_blocks) {
   const uint32_t stride = gridDim.x * STEP_THREADS;
   if (!counted) {
     vec4_t<T>* Ps = R.p(cur);
@@ -436,7 +468,7 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
     const vec4_t<T>* Ps = R.p(1 - cur);
     const T rmax = (T)__uint_as_float(R.ctl[RUN_RMAX]) * T(1.0001);
     for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += stride)
-      run_build_one<T, MULTI, MESH>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax);
+      run_build_one<T, MULTI, MESH, TAPE>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax, build);
   }
   return true;
 }
@@ -587,9 +619,10 @@ __device__ __forceinline__ void run_mesh_half(vec4_t<T>& P, vec4_t<T>& V, uint32
 
 // The step of the spheres put aside: a warp to each that needs run_slow's
 // order, half a warp to each near a triangle.
-template <class T, bool MULTI, bool MESH>
+template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
-                                       const RunBufs<T>& R, const RunLate& l, int cur, float frac, bool last) {
+                                       const RunBufs<T>& R, const RunLate& l, int cur, float frac, uint32_t build,
+                                       uint32_t s, bool last) {
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
@@ -600,13 +633,15 @@ __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T
   for (uint32_t k = threadIdx.x >> 5; k < n_slow; k += STEP_THREADS / 32) {
     const uint32_t i = run_put<T>(l, R, k, true);
     const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
-    const uint32_t word = R.cnt[i];
-    uint32_t mine = lane < R.cap ? R.list[(size_t)lane * b.n + i] & ~RUN_FAR_CELL : i;
+    const uint32_t word = R.template counts<TAPE>(build, b.n)[i];
+    uint32_t mine = lane < R.cap ? R.template lists<TAPE>(build, b.n)[(size_t)lane * b.n + i] & ~RUN_FAR_CELL : i;
     vec4_t<T> old = Ps[i];
+    const vec4_t<T> Vi = Vs[i];
     if (lane >= (word & RUN_COUNT) || !in_bounds(mine, b.n, b.err)) mine = i;
-    vec4_t<T> V = run_slow<T>(i, word, mine, b, sp, Ps, Vs, (T)frac, old, Vs[i]);
+    vec4_t<T> V = run_slow<T>(i, word, mine, b, sp, Ps, Vs, (T)frac, old, Vi);
     old.w = fabs(old.w);
     vec4_t<T> P = old;
+    if (TAPE && lane == 0u) run_record<T>(R, b, s, i, P, V, Vi);
     if (!last) {
       integrate<T>(P, V, sp);
       if constexpr (MESH) {
@@ -631,7 +666,7 @@ __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T
       const bool on = k < n_near;
       const uint32_t i = run_put<T>(l, R, on ? k : k0, false);
       const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
-      const uint32_t word = R.cnt[i], nt = word >> RUN_TRIS;
+      const uint32_t word = R.template counts<TAPE>(build, b.n)[i], nt = word >> RUN_TRIS;
       const uint32_t t = R.tris[(size_t)(lane & 15u) * b.n + i];
       const vec4_t<T> old = Ps[i];
       vec4_t<T> P = Pd[i], V = Vd[i];
@@ -663,25 +698,27 @@ struct RunOwn {
 };
 
 template <class T, bool OWN>
-__device__ __forceinline__ void run_load_own(RunOwn<T>& o, uint32_t i, const StepBufs<T>& b, const RunBufs<T>& R,
-                                             int cur) {
-  o.P = R.p(cur)[i];
-  o.V = R.v(cur)[i];
-  o.word = R.cnt[i];
+__device__ __forceinline__ void run_load_own(RunOwn<T>& o, uint32_t i, const StepBufs<T>& b, const vec4_t<T>* Ps,
+                                             const vec4_t<T>* Vs, const uint32_t* list, const uint16_t* cnt) {
+  o.P = Ps[i];
+  o.V = Vs[i];
+  o.word = cnt[i];
   if constexpr (!OWN) return;
 #pragma unroll
   for (int u = 0; u < run_batch<T>(); ++u)
-    o.head[u] = (uint32_t)u < (o.word & RUN_COUNT) ? R.list[(size_t)u * b.n + i] : i;
+    o.head[u] = (uint32_t)u < (o.word & RUN_COUNT) ? list[(size_t)u * b.n + i] : i;
 }
 
 // One step on the lists: contacts of the state in buffer `cur`, then, unless
 // it is the call's last step, the next step's integration and container.
 // OWN: each thread has one sphere at most, and `own` holds it (loaded when
 // `fresh`), so that a step waits for its neighbours' positions alone.
-template <class T, bool MULTI, bool MESH, bool OWN>
+template <class T, bool MULTI, bool MESH, bool OWN, bool TAPE>
 __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
-                                               const RunBufs<T>& R, int cur, float frac, bool last, RunOwn<T>& own,
-                                               bool fresh) {
+                                               const RunBufs<T>& R, int cur, float frac, uint32_t build, uint32_t s,
+                                               bool last, RunOwn<T>& own, bool fresh) {
+  const uint32_t* list = R.template lists<TAPE>(build, b.n);
+  const uint16_t* cnt = R.template counts<TAPE>(build, b.n);
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
@@ -696,7 +733,7 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
     odd = near = false;
     {
       const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
-      if (!OWN || fresh) run_load_own<T, OWN>(own, i, b, R, cur);
+      if (!OWN || fresh) run_load_own<T, OWN>(own, i, b, Ps, Vs, list, cnt);
       const vec4_t<T> Vi = own.V;
       const uint32_t nl = own.word & RUN_COUNT;
       // Partners that have left their cell of the build may change the order,
@@ -715,14 +752,14 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
         vec4_t<T> Q[NB];
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
-          jj[u] = OWN ? next[u] : (k0 + u < nl ? R.list[(size_t)(k0 + u) * b.n + i] : i);
+          jj[u] = OWN ? next[u] : (k0 + u < nl ? list[(size_t)(k0 + u) * b.n + i] : i);
           if (!in_bounds(jj[u] & ~RUN_FAR_CELL, b.n, b.err)) jj[u] = i;
         }
 #pragma unroll
         for (int u = 0; u < NB; ++u) Q[u] = Ps[jj[u] & ~RUN_FAR_CELL];
         if constexpr (OWN) {  // (64 registers, of the other form, do not hold them)
 #pragma unroll
-          for (int u = 0; u < NB; ++u) next[u] = k0 + NB + u < nl ? R.list[(size_t)(k0 + NB + u) * b.n + i] : i;
+          for (int u = 0; u < NB; ++u) next[u] = k0 + NB + u < nl ? list[(size_t)(k0 + NB + u) * b.n + i] : i;
         }
 #pragma unroll
         for (int u = 0; u < NB; ++u)
@@ -738,6 +775,7 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
       }
       odd = wide || (moved && touching > 1u);
       own.P.w = fabs(own.P.w);
+      if (TAPE && !odd) run_record<T>(R, b, s, i, own.P, own.V, Vi);
       if (!last && !odd) {
         const vec4_t<T> old = own.P;
         integrate<T>(own.P, own.V, sp);
@@ -763,7 +801,7 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
   }
   __syncthreads();
   if (late.n_slow + late.n_near > 0u) {
-    m = fmaxf(m, run_late<T, MULTI, MESH>(b, sp0, mv, R, late, cur, frac, last));
+    m = fmaxf(m, run_late<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, frac, build, s, last));
     if constexpr (OWN) {
       __syncthreads();
       if (odd || near) {
@@ -778,7 +816,8 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
 
 // `steps` steps from the at-rest state (P0, V1, orig), which is also where
 // the state ends.
-// OWN: the grid has a thread for every sphere.
+// OWN: the grid has a thread for every sphere.  TAPE: recording for the
+// backward pass.
 //
 // CTAs per SM: with more spheres than threads the warps in flight hide the
 // latency, and four CTAs leave 64 registers (FP32); with a thread for every
@@ -789,7 +828,7 @@ __host__ __device__ constexpr int run_ctas() {
   return (sizeof(T) == 4 ? 4 : 2) / (OWN ? 2 : 1);
 }
 
-template <class T, bool MULTI, bool MESH, bool OWN>
+template <class T, bool MULTI, bool MESH, bool OWN, bool TAPE>
 __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     k_run(const __grid_constant__ StepBufs<T> b, const __grid_constant__ SceneParams<T> sp0, const MeshView* mv,
           const __grid_constant__ RunBufs<T> R, uint32_t steps, int64_t n_cells, uint32_t scatter_blocks,
@@ -802,10 +841,10 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   bool counted = true;   // the state's cells are counted already
   float D = 0.0f;        // motion since the last build, in cells
   float frac = 0.0f;     // skin of the last build, in cells
-  uint32_t rebuilds = 0;
+  uint32_t rebuilds = 0, build = 0;
   // the last step's m, of an earlier run if need be
   float before = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_BEFORE));
-  if (!(before > 0.0f)) before = INFINITY;
+  if (!(before > 0.0f) || TAPE) before = INFINITY;
   RunOwn<T> own;
   for (uint32_t s = 0; s < steps; ++s) {
     if (!run_barrier(R.ctl, b.err)) return;
@@ -815,20 +854,32 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     D = D * 1.000001f + m;
     bool fresh = false;
     if (!lists || !(D <= 0.49f * frac)) {
+      if (TAPE) {  // a recorded run has lists in every step, or gives up
+        if (m > RUN_CALM_MAX || rebuilds == R.max_builds) return;
+        build = rebuilds;
+        streak = RUN_CALM_STEPS;
+      }
       lists = streak >= RUN_CALM_STEPS;
       // (a single fast step, a sphere pushed out of a wall, is no measure)
-      frac = lists ? fminf(fmaxf(fminf(m, before) * (RUN_STEPS_PER_BUILD / 0.49f), RUN_SKIN_MIN), RUN_SKIN_MAX) : 0.0f;
-      if (!run_rebuild<T, MULTI, MESH>(b, sp0, mv, R, cur, counted, frac, n_cells, scatter_blocks, move_blocks)) return;
+      // (A recorded run depends on its starting state alone, for the backward
+      // pass to give the same sums every time; its builds have to last for
+      // the block, and the first, of unknown speed, is kept thin.)
+      const float last_for = TAPE ? fmaxf(RUN_STEPS_PER_BUILD, 0.7f * (float)steps) : RUN_STEPS_PER_BUILD;
+      const float widest = TAPE && s == 0u ? RUN_SKIN_FIRST : RUN_SKIN_MAX;
+      frac = lists ? fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest) : 0.0f;
+      if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, n_cells, scatter_blocks, move_blocks))
+        return;
       cur = 1 - cur;
       D = 0.0f;
       fresh = true;
       ++rebuilds;
     }
     before = m;
+    if (TAPE && blockIdx.x == 0 && threadIdx.x == 0) R.tape_build[s] = build;
     const bool last = s + 1u == steps;
     float mm;
     if (lists)
-      mm = run_list_step<T, MULTI, MESH, OWN>(b, sp0, mv, R, cur, frac, last, own, fresh);
+      mm = run_list_step<T, MULTI, MESH, OWN, TAPE>(b, sp0, mv, R, cur, frac, build, s, last, own, fresh);
     else
       mm = run_grid_step<T, MULTI, MESH>(b, sp0, mv, R, cur, last);
     if (!last) publish_max(mm, maxd + (s + 1u) % 3u);
@@ -846,6 +897,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   if (blockIdx.x == 0 && threadIdx.x < 3u) maxd[threadIdx.x] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 3u) R.ctl[RUN_RMAX] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0u) {
+    if (TAPE) R.tape_build[steps] = R.ctl[RUN_FULL] == 0u ? 1u : 0u;
     R.ctl[RUN_STREAK] = streak;
     R.report[0] = run_id;
     R.ctl[RUN_BEFORE] = __float_as_uint(before);

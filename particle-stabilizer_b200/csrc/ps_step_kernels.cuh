@@ -184,6 +184,30 @@ __device__ __forceinline__ const SceneParams<T>& scene_of(uint32_t p, const Scen
   return b.scenes[lo];
 }
 
+// One row of the backward pass's tape (ps_adjoint.cuh).
+template <class T>
+struct TapeRow {
+  vec4_t<T>* p;     // (x, r) per sorted slot
+  vec4_t<T>* v;     // (v, m)
+  vec4_t<T>* vpre;  // (v, m) before the contacts of the step that wrote the row
+  uint32_t* o;      // original id
+  uint32_t* cell;   // sorted cell id of that step's grid
+};
+
+// Row t of a tape: the at-rest state after t steps; rows t >= 1 also hold
+// what step t - 1's contacts read.
+template <class T>
+__host__ __device__ inline TapeRow<T> tape_row(char* base, size_t row_bytes, int64_t n, int64_t t) {
+  TapeRow<T> r;
+  char* p = base + row_bytes * (size_t)t;
+  r.p = reinterpret_cast<vec4_t<T>*>(p);
+  r.v = r.p + n;
+  r.vpre = r.v + n;
+  r.o = reinterpret_cast<uint32_t*>(r.vpre + n);
+  r.cell = r.o + n;
+  return r;
+}
+
 // Container step + hash + count on an integrated state, shared by k_begin and
 // the fused epilogue of k_contacts.
 template <class T, bool MESH>

@@ -99,7 +99,8 @@ def test_run_equals_oracle(need_gpu):
 @pytest.mark.parametrize("skin", [None, 0.2])
 def test_adjoint_of_runs_whose_order_is_an_earlier_grids(need_gpu, skin):
     # spheres change cells inside the blocks, so a block does not end in the
-    # order of its last build; blocks of 5 steps take the step kernels
+    # order of its last build; blocks of 5 steps take the step kernels and
+    # their recording, whose sums differ in order alone
     sc = faster(scenes.pile(1000, seed=24, k_spring=1.0), 20.0)
     out = []
     for every in (5, 50):
@@ -112,9 +113,32 @@ def test_adjoint_of_runs_whose_order_is_an_earlier_grids(need_gpu, skin):
             grads, g0 = sim.backward(psb200.height_loss(final)[1])
             out.append((final, grads[0], g0))
     assert np.array_equal(out[0][0], out[1][0])
-    # the same sums in the same order, whatever the blocks
-    assert np.array_equal(out[0][2], out[1][2])
-    np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-9)
+    for k in (1, 2):
+        np.testing.assert_allclose(out[0][k], out[1][k], rtol=1e-9, atol=1e-10 * np.abs(out[0][k]).max())
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("name", ["pile", "fast", "crowd", "batch", "cells of 2 r_max"])
+def test_backward_on_recorded_runs(need_gpu, name, prec):
+    """The backward pass recomputes blocks as recorded runs, or on the grid
+    where lists do not last (fast) or overflow (crowd): blocks of 40 steps
+    against blocks of 7, which are always recomputed on the grid, and two
+    passes of the same against each other."""
+    scs = SCENES[name]()
+    if name == "batch":
+        scs = scs[:-1]  # without the scene that diverges
+    out = []
+    for every in (7, 40):
+        with psb200.Simulation(scs, prec) as sim:
+            sim.set_state()
+            sim.forward_checkpointed(84, every)
+            g = psb200.height_loss(sim.get_state())[1]
+            first, again = sim.backward(g), sim.backward(g)
+            assert all(np.array_equal(x, y) for x, y in zip(first[0], again[0])) and np.array_equal(first[1], again[1])
+            out.append(first)
+    tol = 1e-9 if prec == "f64" else 2e-4
+    for x, y in zip([*out[0][0], out[0][1]], [*out[1][0], out[1][1]]):
+        np.testing.assert_allclose(x, y, rtol=tol, atol=tol * max(np.abs(x).max(), 1e-300))
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
