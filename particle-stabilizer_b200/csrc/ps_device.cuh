@@ -170,8 +170,7 @@ enum : uint32_t {
   PS_DEVERR_SCAN_TIMEOUT = 1u << 0,   // decoupled look-back gave up waiting
   PS_DEVERR_MESH_OVERFLOW = 1u << 1,  // reserved: a sphere may touch any number of triangles
   PS_DEVERR_BAD_CELL = 1u << 2,       // a cell id fell outside its scene (never expected)
-  PS_DEVERR_LIST_OVERFLOW = 1u << 3,  // neighbour-list mode: a list or a sphere's overlap buffer was full
-  PS_DEVERR_LIST_BARRIER = 1u << 4,   // neighbour-list mode: a grid barrier of the rebuild gave up waiting
+  PS_DEVERR_LIST_BARRIER = 1u << 4,   // a grid barrier of the many-step kernel gave up waiting
   PS_DEVERR_BOUNDS = 1u << 5,         // bounds-checked build: an index fell outside its array
 };
 

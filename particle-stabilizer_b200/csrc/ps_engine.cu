@@ -23,7 +23,6 @@
 
 #include "particle_stabilizer_b200.h"
 #include "ps_adjoint.cuh"
-#include "ps_lists.cuh"
 #include "ps_run.cuh"
 #include "ps_scan.cuh"
 #include "ps_stats.cuh"
@@ -163,17 +162,14 @@ struct ps_sim {
   // neighbour-list mode (ps_set_neighbor_lists); off when list_skin <= 0
   double list_skin = 0.0;                 // skin as a fraction of the cell edge
   int32_t list_cap = 0;                   // list capacity per sphere
-  void* list_arena = nullptr;
+  void* list_arena = nullptr;             // as run_arena, with the program's capacity
   size_t list_bytes = 0;
-  void* list_ckpt = nullptr;              // state at the start of a list-mode call
-  int64_t list_fallbacks = 0;             // calls repeated on the grid path after an overflow
+  int64_t list_fallbacks = 0;             // calls in which a sphere had more neighbours than a list holds
   int64_t list_rebuilds = 0;              // grid + list rebuilds requested by the device
   int64_t list_grid_steps = 0;            // list-mode steps run on the grid path (backoff)
   // backoff: a window of list steps that rebuilt more than once per
   // LIST_BACKOFF_RATE steps sends the next `list_backoff` steps to the grid path
   int64_t list_win_steps = 0, list_win_rebuilds = 0, list_backoff = 0, list_backoff_len = 0;
-  unsigned list_rebuild_grid = 0;         // CTAs of the cooperative rebuild (one wave)
-  unsigned list_step_grid = 0;            // CTAs of the list step kernel (one wave)
   // the kernel of many steps (ps_run.cuh)
   uint32_t* d_chunk_scene = nullptr;      // scene of every SCENE_CHUNK-th slot (several scenes only)
   void* run_arena = nullptr;              // lists, count words, control words
@@ -397,113 +393,6 @@ void enqueue_steps_recorded_dispatch(ps_sim* s, int64_t steps, std::vector<Launc
     else
       enqueue_steps_recorded<T, false, false>(s, steps, rec);
   }
-}
-
-// ---- neighbour-list mode ---------------------------------------------------------
-size_t list_arena_bytes(const ps_sim* s) {
-  const size_t n = (size_t)std::max<int64_t>(s->n_total, 1), vb = s->precision == PS_FP32 ? 16 : 32;
-  return 5 * align_up(vb * n, 256) + 3 * align_up(4 * n, 256) + align_up(4 * n * (size_t)s->list_cap, 256) +
-         align_up(4 * LIST_FLAG_WORDS, 256);
-}
-
-template <class T>
-ListBufs<T> list_bufs(ps_sim* s) {
-  const size_t n = (size_t)std::max<int64_t>(s->n_total, 1);
-  const size_t b4 = align_up(sizeof(vec4_t<T>) * n, 256), bu = align_up(4 * n, 256);
-  char* p = static_cast<char*>(s->list_arena);
-  ListBufs<T> L;
-  L.P[0] = reinterpret_cast<vec4_t<T>*>(p); p += b4;
-  L.P[1] = reinterpret_cast<vec4_t<T>*>(p); p += b4;
-  L.V[0] = reinterpret_cast<vec4_t<T>*>(p); p += b4;
-  L.V[1] = reinterpret_cast<vec4_t<T>*>(p); p += b4;
-  L.ref = reinterpret_cast<vec4_t<T>*>(p); p += b4;
-  L.cell[0] = reinterpret_cast<uint32_t*>(p); p += bu;
-  L.cell[1] = reinterpret_cast<uint32_t*>(p); p += bu;
-  L.cnt = reinterpret_cast<uint32_t*>(p); p += bu;
-  L.list = reinterpret_cast<uint32_t*>(p); p += align_up(4 * n * (size_t)s->list_cap, 256);
-  L.flag = reinterpret_cast<uint32_t*>(p);
-  L.cap = (uint32_t)s->list_cap;
-  L.skin_frac = (T)s->list_skin;
-  return L;
-}
-
-// `steps` steps on neighbour lists: a full rebuild from the at-rest state,
-// then per step the gated cooperative rebuild and the list step kernel.
-// Every graph starts from zeroed counts, whatever an earlier rebuild left.
-template <class T, bool MULTI, bool MESH>
-cudaError_t enqueue_steps_list(ps_sim* s, int64_t steps) {
-  const StepBufs<T> b = bufs<T>(s);
-  const ListBufs<T> L = list_bufs<T>(s);
-  const SceneParams<T> sp0 = params<T>(s)[0];
-  const unsigned gp = blocks_for(s->n_total);
-  const unsigned gs = (unsigned)step_scan_tiles(n_scan(s));
-  const unsigned gm0 = move_blocks(s->n_total, b.n_tiles), gm1 = move_blocks(s->n_total, 0);
-  cudaStream_t st = s->stream;
-  const MeshView* mv = s->d_mesh_view;
-  const int64_t nsc = n_scan(s);
-  const uint32_t nt = (uint32_t)s->n_total;
-  cudaMemsetAsync(L.flag, 0, LIST_RESET_WORDS * sizeof(uint32_t), st);
-  cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)nsc, st);
-  cudaMemsetAsync(s->tile_sum, 0, sizeof(uint32_t) * (size_t)b.n_tiles, st);
-  pdl_launch(k_begin<T, MULTI, MESH, true>, gp, STEP_THREADS, st, b, sp0, mv);
-  pdl_launch(step_scan_kernel(n_scan(s)), gs, SCAN_THREADS, st, (const uint32_t*)s->count, s->offset, nsc,
-             (const uint32_t*)s->tile_sum);
-  pdl_launch(k_scatter, gm0, STEP_THREADS, st, (const uint32_t*)s->cell, s->slot, (const uint32_t*)s->orig,
-             (const uint32_t*)s->offset, s->tmp, s->count, nt, s->tile_sum, b.n_tiles, s->err);
-  pdl_launch(k_rank_move<T>, gm1, STEP_THREADS, st, b);
-  pdl_launch(k_list_build<T, MULTI>, gp, STEP_THREADS, st, b, sp0, L, 0);
-  for (int64_t k = 0; k < steps; ++k) {
-    const int par = (int)(k & 1);
-    if (k > 0) {
-      // the rebuild works on state buffer `par`, in the order of the previous build
-      StepBufs<T> br = b;
-      br.P1 = L.P[par];
-      br.V1 = L.V[par];
-      br.cell = L.cell[par];
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(s->list_rebuild_grid);
-      cfg.blockDim = dim3(STEP_THREADS);
-      cfg.stream = st;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeCooperative;
-      at[0].val.cooperative = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      const cudaError_t e = cudaLaunchKernelEx(&cfg, k_list_rebuild<T, MULTI>, br, sp0, L, par, nsc, (uint32_t)gs,
-                                               (uint32_t)gm0, (uint32_t)gm1);
-      if (e != cudaSuccess) return e;
-    }
-    const unsigned gl = std::min(gp, s->list_step_grid);
-    if (k + 1 < steps)
-      pdl_launch(k_contacts_list<T, MULTI, MESH, true>, gl, STEP_THREADS, st, b, sp0, mv, L, par);
-    else
-      pdl_launch(k_contacts_list<T, MULTI, MESH, false>, gl, STEP_THREADS, st, b, sp0, mv, L, par);
-  }
-  return cudaGetLastError();
-}
-
-// CTAs of one wave of k_list_rebuild, which its grid barriers need resident,
-// and of one wave of the list step kernel, which loops over the spheres.
-template <class T, bool MULTI, bool MESH>
-int list_grids(ps_sim* s) {
-  int per_sm = 0, step_per_sm = 0, sms = 0;
-  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_list_rebuild<T, MULTI>, STEP_THREADS, 0));
-  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&step_per_sm, k_contacts_list<T, MULTI, MESH, true>,
-                                                        STEP_THREADS, 0));
-  PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-  if (per_sm < 1 || step_per_sm < 1 || sms < 1)
-    return fail(PS_ERR_CUDA, "ps_step: the list kernels cannot be resident");
-  s->list_rebuild_grid = (unsigned)(per_sm * sms);
-  s->list_step_grid = (unsigned)(step_per_sm * sms);
-  return PS_OK;
-}
-
-template <class T>
-cudaError_t enqueue_steps_list_dispatch(ps_sim* s, int64_t steps) {
-  if (s->multi) {
-    return s->has_mesh ? enqueue_steps_list<T, true, true>(s, steps) : enqueue_steps_list<T, true, false>(s, steps);
-  }
-  return s->has_mesh ? enqueue_steps_list<T, false, true>(s, steps) : enqueue_steps_list<T, false, false>(s, steps);
 }
 
 template <class T>
@@ -958,9 +847,7 @@ void ensure_l2_limit(ps_sim* s) {
 }
 
 // Captured kernel nodes carry the window explicitly.
-// `clear` gives the nodes an empty window instead (neighbour-list graphs:
-// their steps do not touch the cell arrays, which only a rebuild reads).
-void apply_l2_window(ps_sim* s, cudaGraph_t g, bool clear = false) {
+void apply_l2_window(ps_sim* s, cudaGraph_t g) {
   if (!s->l2_window_on) return;
   size_t n = 0;
   if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess || n == 0) return;
@@ -968,7 +855,6 @@ void apply_l2_window(ps_sim* s, cudaGraph_t g, bool clear = false) {
   cudaGraphGetNodes(g, nodes.data(), &n);
   cudaKernelNodeAttrValue v{};
   v.accessPolicyWindow = s->l2_window;
-  if (clear) v.accessPolicyWindow.num_bytes = 0;
   for (auto nd : nodes) {
     cudaGraphNodeType t;
     if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel)
@@ -983,9 +869,9 @@ void apply_l2_window(ps_sim* s, cudaGraph_t g, bool clear = false) {
 // without it every call takes the step kernels.
 constexpr size_t RUN_WITH_PARTICLES = (size_t)64 << 20;
 
-size_t run_need(const ps_sim* s, int sms) {
+size_t run_need(const ps_sim* s, int sms, size_t cap) {
   const size_t n = (size_t)s->n_total, threads = (size_t)sms * 2048;  // the grid's threads at most
-  return 256 + align_up(2 * n, 256) + align_up(4 * n * RUN_LIST_CAP, 256) + align_up(4 * (n + threads), 256) +
+  return 256 + align_up(2 * n, 256) + align_up(4 * n * cap, 256) + align_up(4 * (n + threads), 256) +
          (s->has_mesh ? 4 * n * RUN_TRI_CAP : 0);
 }
 
@@ -1115,7 +1001,6 @@ void free_sim(ps_sim* s) {
   cudaFree(s->fwd_arena);
   cudaFree(s->adj_arena);
   cudaFree(s->list_arena);
-  cudaFree(s->list_ckpt);
   if (s->run_arena_own) cudaFree(s->run_arena);
   if (s->l2_window_on) {
     cudaStreamAttrValue v{};
@@ -1149,37 +1034,45 @@ int64_t run_block(const ps_sim* s) {
   return std::min<int64_t>(512, std::max<int64_t>(32, (int64_t)2000000000 / std::max<int64_t>(s->n_total, 1)));
 }
 
+int run_sms(const ps_sim* s) {
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+  return sms;
+}
+
 // Spheres of one CTA of the run kernel.
 uint32_t run_share(const ps_sim* s) {
   const int64_t stride = (int64_t)s->run_grid * STEP_THREADS;
   return (uint32_t)((s->n_total + stride - 1) / stride) * STEP_THREADS;
 }
 
+// set: with the skin and the capacity of ps_set_neighbor_lists
 template <class T>
-RunBufs<T> run_bufs(ps_sim* s) {
+RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
   const size_t n = (size_t)s->n_total;
   RunBufs<T> R;
   R.P[0] = static_cast<vec4_t<T>*>(s->P0);
   R.P[1] = static_cast<vec4_t<T>*>(s->P1);
   R.V[0] = static_cast<vec4_t<T>*>(s->V0);
   R.V[1] = static_cast<vec4_t<T>*>(s->V1);
-  char* p = static_cast<char*>(s->run_arena);
+  char* p = static_cast<char*>(set ? s->list_arena : s->run_arena);
   R.ctl = reinterpret_cast<uint32_t*>(p);
+  R.cap = set ? (uint32_t)s->list_cap : RUN_LIST_CAP;
+  R.skin = set ? (float)s->list_skin : 0.0f;
   p += 256;
   R.cnt = reinterpret_cast<uint16_t*>(p);
   p += align_up(2 * n, 256);
   R.list = reinterpret_cast<uint32_t*>(p);
-  p += align_up(4 * n * RUN_LIST_CAP, 256);
+  p += align_up(4 * n * R.cap, 256);
   R.later = reinterpret_cast<uint32_t*>(p);
   R.later_stride = run_share(s);
   p += align_up(4 * (size_t)s->run_grid * R.later_stride, 256);
   R.tris = s->has_mesh ? reinterpret_cast<uint32_t*>(p) : nullptr;
-  R.cap = RUN_LIST_CAP;
   R.tape = nullptr;
   R.tape_row_bytes = 0;
   R.tape_build = nullptr;
   R.max_builds = 0;
-  R.report = s->err + ERR_RUN;
+  R.report = set ? R.ctl + RUN_REPORT : s->err + ERR_RUN;
   return R;
 }
 
@@ -1219,13 +1112,13 @@ int run_launch(ps_sim* s, uint32_t steps, const RunBufs<T>& R, uint32_t run_id) 
 }
 
 template <class T>
-int run_dispatch(ps_sim* s, uint32_t steps, bool prepare) {
+int run_dispatch(ps_sim* s, uint32_t steps, bool prepare, bool set = false) {
   if (s->multi) {
-    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true, false>(s, steps, run_bufs<T>(s), ++s->run_id);
-    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
+    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
   }
-  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true, false>(s, steps, run_bufs<T>(s), ++s->run_id);
-  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false, false>(s, steps, run_bufs<T>(s), ++s->run_id);
+  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
+  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
 }
 
 // ---- differentiation -----------------------------------------------------------
@@ -1335,11 +1228,13 @@ int record_run(ps_sim* s, int64_t steps, char* tape, size_t row_bytes, char* lis
   R.tape = tape;
   R.tape_row_bytes = row_bytes;
   R.max_builds = TAPE_BUILDS;
+  R.report = R.ctl + RUN_REPORT;
   R.tape_build = reinterpret_cast<uint32_t*>(lists);
   lists += align_up(4 * (size_t)(steps + 1), 256);
   R.cnt = reinterpret_cast<uint16_t*>(lists);
   R.list = reinterpret_cast<uint32_t*>(lists + align_up(2 * n * TAPE_BUILDS, 256));
   PS_CUDA(cudaMemsetAsync(R.tape_build + steps, 0, sizeof(uint32_t), s->stream));
+  PS_CUDA(cudaMemsetAsync(R.ctl + RUN_FULL, 0, sizeof(uint32_t), s->stream));
   const int rc = run_launch<T, MULTI, false, true>(s, (uint32_t)steps, R, s->run_id);
   if (rc != PS_OK) return rc;
   build.resize((size_t)steps + 1);
@@ -1564,7 +1459,7 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   const size_t chunks = s->multi ? n / SCENE_CHUNK + 2 : 0, bc = align_up(4 * chunks, 256);
   int sms = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  s->run_bytes = s->n_total > 0 ? run_need(s, sms) : 0;
+  s->run_bytes = s->n_total > 0 ? run_need(s, sms, RUN_LIST_CAP) : 0;
   const size_t br = s->run_bytes <= RUN_WITH_PARTICLES ? align_up(s->run_bytes, 256) : 0;
   if (e == cudaSuccess)
     e = cudaMalloc(&s->part_arena,
@@ -1691,48 +1586,41 @@ namespace {
 // graphs, which also keep the call asynchronous.
 constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
 
-// Run n_steps as CUDA graphs of up to graph_block steps (grid path, or the
-// neighbour-list path when `lists`), asynchronously.
-int step_graphs(ps_sim* s, int64_t n_steps, bool lists) {
-  if (!lists) {
-    setup_l2_window(s);
-    ensure_l2_limit(s);
-  }
+// Run n_steps on the step kernels as CUDA graphs of up to graph_block steps,
+// asynchronously.
+int step_graphs(ps_sim* s, int64_t n_steps) {
+  setup_l2_window(s);
+  ensure_l2_limit(s);
   int64_t left = n_steps;
   while (left > 0) {
     const int64_t L = std::min(left, s->graph_block);
-    if (!lists && L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES) {
+    if (L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES) {
       s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
       PS_CUDA(cudaGetLastError());
       s->last_launches += 1 + 4 * L;
       left -= L;
       continue;
     }
-    const int64_t key = lists ? (L | (int64_t(1) << 62)) : L;
-    auto it = s->graphs.find(key);
+    auto it = s->graphs.find(L);
     if (it == s->graphs.end()) {
       cudaGraph_t graph = nullptr;
       PS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t ce = cudaSuccess;
-      if (lists)
-        ce = s->precision == PS_FP32 ? enqueue_steps_list_dispatch<float>(s, L) : enqueue_steps_list_dispatch<double>(s, L);
-      else
-        s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
-      if (ce == cudaSuccess) ce = cudaGetLastError();
+      s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
+      const cudaError_t ce = cudaGetLastError();
       const cudaError_t ee = cudaStreamEndCapture(s->stream, &graph);
       if (ce != cudaSuccess || ee != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return fail(PS_ERR_CUDA, std::string("ps_step: capture failed: ") + cudaGetErrorString(ce != cudaSuccess ? ce : ee));
       }
-      apply_l2_window(s, graph, lists);
+      apply_l2_window(s, graph);
       cudaGraphExec_t exec = nullptr;
       const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
       cudaGraphDestroy(graph);
       if (ie != cudaSuccess) return fail(PS_ERR_CUDA, std::string("ps_step: instantiate failed: ") + cudaGetErrorString(ie));
-      it = s->graphs.emplace(key, exec).first;
+      it = s->graphs.emplace(L, exec).first;
     }
     PS_CUDA(cudaGraphLaunch(it->second, s->stream));
-    s->last_launches += lists ? 5 + 2 * L - 1 : 1 + 4 * L;
+    s->last_launches += 1 + 4 * L;
     left -= L;
   }
   return PS_OK;
@@ -1786,7 +1674,7 @@ int step_run(ps_sim* s, int64_t n_steps) {
     if (s->run_backoff > 0 || waiting) {
       L = std::min(left, waiting ? RUN_BACKOFF_MIN : s->run_backoff);
       s->run_backoff = std::max<int64_t>(0, s->run_backoff - L);
-      rc = step_graphs(s, L, false);
+      rc = step_graphs(s, L);
       s->grid_valid = true;
     } else {
       L = std::min(left, s->run_settled ? run_block(s) : RUN_PROBE_STEPS);
@@ -1810,56 +1698,46 @@ int step_run(ps_sim* s, int64_t n_steps) {
 constexpr int64_t LIST_BACKOFF_WINDOW = 256, LIST_BACKOFF_RATE = 4, LIST_BACKOFF_MIN = 1024,
                   LIST_BACKOFF_MAX = 65536;
 
-// Neighbour-list path: exact as long as no list or overlap buffer overflows
-// (checked after the call); otherwise the call is repeated on the grid path
-// from the state it started from.
+// Runs with the program's skin and capacity; returns when they are done.
 int step_lists(ps_sim* s, int64_t n_steps) {
-  const size_t need = list_arena_bytes(s);
+  if (s->run_grid == 0) {
+    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, 0, true) : run_dispatch<double>(s, 0, true);
+    if (rc != PS_OK) return rc;
+  }
+  const size_t need = run_need(s, run_sms(s), (size_t)s->list_cap);
   if (s->list_arena == nullptr || s->list_bytes < need) {
     cudaFree(s->list_arena);
     s->list_arena = nullptr;
     s->list_bytes = 0;
-    for (auto it = s->graphs.begin(); it != s->graphs.end();) {  // list graphs hold the old buffers
-      if (it->first & (int64_t(1) << 62)) {
-        cudaGraphExecDestroy(it->second);
-        it = s->graphs.erase(it);
-      } else {
-        ++it;
-      }
-    }
     PS_CUDA(dev_alloc(s, &s->list_arena, need));
     s->list_bytes = need;
+    PS_CUDA(cudaMemsetAsync(s->list_arena, 0, 256, s->stream));
   }
-  if (s->list_rebuild_grid == 0) {
-    int g;
-    if (s->precision == PS_FP32)
-      g = s->multi ? (s->has_mesh ? list_grids<float, true, true>(s) : list_grids<float, true, false>(s))
-                   : (s->has_mesh ? list_grids<float, false, true>(s) : list_grids<float, false, false>(s));
-    else
-      g = s->multi ? (s->has_mesh ? list_grids<double, true, true>(s) : list_grids<double, true, false>(s))
-                   : (s->has_mesh ? list_grids<double, false, true>(s) : list_grids<double, false, false>(s));
-    if (g != PS_OK) return g;
+  uint32_t* ctl = static_cast<uint32_t*>(s->list_arena);
+  PS_CUDA(cudaMemsetAsync(ctl + RUN_FULL, 0, 2 * sizeof(uint32_t), s->stream));  // and RUN_BUILDS
+  for (int64_t left = n_steps; left > 0;) {
+    const int64_t L = std::min(left, run_block(s));
+    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, false, true)
+                                           : run_dispatch<double>(s, (uint32_t)L, false, true);
+    if (rc != PS_OK) return rc;
+    s->last_launches += 1;
+    left -= L;
   }
-  uint32_t* rebuilds = s->precision == PS_FP32 ? list_bufs<float>(s).flag + LIST_REBUILDS
-                                               : list_bufs<double>(s).flag + LIST_REBUILDS;
-  PS_CUDA(cudaMemsetAsync(rebuilds, 0, sizeof(uint32_t), s->stream));
-  // the grid path's persisting lines (cell counts and offsets) would hold
-  // L2 that the list steps stream through
-  if (s->l2_window_on) {
-    PS_CUDA(cudaStreamSynchronize(s->stream));
-    cudaCtxResetPersistingL2Cache();
-    cudaGetLastError();
+  s->grid_valid = false;  // the grid arrays are those of the last rebuild
+  uint32_t told[2] = {};
+  static_assert(RUN_BUILDS == RUN_FULL + 1, "read together");
+  PS_CUDA(cudaMemcpyAsync(told, ctl + RUN_FULL, sizeof(told), cudaMemcpyDeviceToHost, s->stream));
+  const int rc = check_device_error(s);  // waits for the stream
+  if (rc != PS_OK) {
+    cudaFree(s->list_arena);  // with what a run left in its control words
+    s->list_arena = nullptr;
+    s->list_bytes = 0;
+    return rc;
   }
-  int rc = save_state(s, s->list_ckpt);
-  if (rc == PS_OK) rc = step_graphs(s, n_steps, true);
-  if (rc != PS_OK) return rc;
-  uint32_t e = 0, nr = 0;
-  PS_CUDA(cudaMemcpyAsync(&e, s->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-  PS_CUDA(cudaMemcpyAsync(&nr, rebuilds, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-  PS_CUDA(cudaStreamSynchronize(s->stream));
-  s->list_rebuilds += nr;
+  s->list_fallbacks += told[0] != 0u;
+  s->list_rebuilds += told[1];
   s->list_win_steps += n_steps;
-  s->list_win_rebuilds += nr;
+  s->list_win_rebuilds += told[1];
   if (s->list_win_steps >= LIST_BACKOFF_WINDOW) {
     if (s->list_win_rebuilds * LIST_BACKOFF_RATE > s->list_win_steps) {
       s->list_backoff_len = std::min<int64_t>(std::max<int64_t>(2 * s->list_backoff_len, LIST_BACKOFF_MIN),
@@ -1870,19 +1748,7 @@ int step_lists(ps_sim* s, int64_t n_steps) {
     }
     s->list_win_steps = s->list_win_rebuilds = 0;
   }
-  constexpr uint32_t list_err = PS_DEVERR_LIST_OVERFLOW | PS_DEVERR_LIST_BARRIER;
-  if (e & list_err) {
-    // counts and tile totals may be left over from an interrupted rebuild
-    const uint32_t rest = e & ~list_err;
-    PS_CUDA(cudaMemcpyAsync(s->err, &rest, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
-    PS_CUDA(cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)n_scan(s), s->stream));
-    PS_CUDA(cudaMemsetAsync(s->tile_sum, 0, sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), s->stream));
-    PS_CUDA(cudaStreamSynchronize(s->stream));
-    ++s->list_fallbacks;
-    rc = load_state(s, s->list_ckpt);
-    if (rc == PS_OK) rc = step_graphs(s, n_steps, false);
-  }
-  return rc;
+  return PS_OK;
 }
 
 }  // namespace
@@ -1893,21 +1759,13 @@ extern "C" int ps_set_neighbor_lists(ps_sim* s, double skin_fraction, int32_t ma
     return fail(PS_ERR_INVALID,
                 "ps_set_neighbor_lists: skin_fraction must be 0 or in [0.01, 1], and max_neighbours in [1, 4096]");
   DeviceGuard guard(s->device);
-  if (max_neighbours != s->list_cap) {  // the arena and the list graphs are rebuilt on the next step
+  if (max_neighbours != s->list_cap) {  // the lists are laid out anew on the next step
     cudaFree(s->list_arena);
     s->list_arena = nullptr;
     s->list_bytes = 0;
   }
-  for (auto it = s->graphs.begin(); it != s->graphs.end();) {
-    if (it->first & (int64_t(1) << 62)) {
-      cudaGraphExecDestroy(it->second);
-      it = s->graphs.erase(it);
-    } else {
-      ++it;
-    }
-  }
   s->list_skin = skin_fraction;
-  s->list_cap = skin_fraction > 0.0 ? max_neighbours : 0;
+  s->list_cap = skin_fraction > 0.0 ? std::min<int32_t>(max_neighbours, (int32_t)RUN_LIST_CAP_MAX) : 0;
   s->list_rebuilds = 0;
   s->list_fallbacks = 0;
   s->list_grid_steps = 0;
@@ -1935,7 +1793,8 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
   int64_t left = n_steps;
   if (lists && s->list_backoff > 0) {
     const int64_t g = std::min(left, s->list_backoff);
-    rc = step_graphs(s, g, false);
+    rc = step_graphs(s, g);
+    s->grid_valid = true;
     s->list_backoff -= g;
     s->list_grid_steps += g;
     left -= g;
@@ -1943,8 +1802,8 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
   if (!lists && left >= RUN_MIN_STEPS && s->run_arena != nullptr && !s->run_off) {
     rc = step_run(s, left);
   } else if (rc == PS_OK && left > 0) {
-    rc = lists ? step_lists(s, left) : step_graphs(s, left, false);
-    s->grid_valid = !lists;  // after the list path the grid arrays do not describe the at-rest state
+    rc = lists ? step_lists(s, left) : step_graphs(s, left);
+    if (!lists) s->grid_valid = true;
   }
   if (rc != PS_OK) return rc;
   s->stepped = true;

@@ -37,13 +37,16 @@
 // cells, like the step kernels.  The skin of a build follows from the speed,
 // so that a build lasts about RUN_STEPS_PER_BUILD steps.
 //
+// ps_set_neighbor_lists sets the skin and the lists' capacity of the same
+// kernel, for every build.
+//
 // What bounds it: a list step moves 66 B per sphere in FP32 (position and
 // velocity in and out, one 2-byte count), mostly through L2 up to a million
 // spheres; what remains is the chain count -> list entry -> position ->
 // velocity of the touching pairs and the barrier (about 1.5 us).
 #pragma once
 
-#include "ps_lists.cuh"
+#include "ps_step_kernels.cuh"
 
 namespace psb {
 
@@ -56,15 +59,15 @@ constexpr float RUN_SKIN_MIN = 0.02f, RUN_SKIN_MAX = 0.25f, RUN_SKIN_FIRST = 0.0
 
 // count word of a sphere: list length and what its step needs besides
 enum : uint32_t {
-  RUN_COUNT = 0x3fu,
-  RUN_NEAR_FACE = 1u << 6,  // may leave its cell before the next build
-  RUN_OVERFLOW = 1u << 7,   // more neighbours than the list holds
-  RUN_TRIS = 8,             // shift: triangles that may come within reach, RUN_TRI_MANY if not all are listed
+  RUN_COUNT = 0xffu,
+  RUN_NEAR_FACE = 1u << 8,  // may leave its cell before the next build
+  RUN_OVERFLOW = 1u << 9,   // more neighbours than the list holds
+  RUN_TRIS = 10,            // shift: triangles that may come within reach, RUN_TRI_MANY if not all are listed
 };
 constexpr int RUN_TRI_CAP = 16;
 constexpr uint32_t RUN_TRI_MANY = RUN_TRI_CAP + 1;
 constexpr uint32_t RUN_FAR_CELL = 0x80000000u;  // list entry: cells not adjacent at the build
-static_assert(RUN_LIST_CAP <= 32 && RUN_LIST_CAP <= RUN_COUNT, "a list is at most an entry per lane, its length fits the word");
+constexpr uint32_t RUN_LIST_CAP_MAX = RUN_COUNT;  // list capacity that a program may ask for
 
 // control words
 enum : int {
@@ -73,7 +76,9 @@ enum : int {
   RUN_STREAK = 5,   // calm steps up to now
   RUN_RMAX = 6,     // largest radius, in cells of its scene
   RUN_BEFORE = 7,   // largest displacement of the last step, in cells (0: none yet)
-  RUN_FULL = 8,     // a recorded run met a sphere with more neighbours than a list holds
+  RUN_FULL = 8,     // a sphere had more neighbours than a list holds
+  RUN_BUILDS = 9,   // builds after a run's first
+  RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
 };
 
 template <class T>
@@ -94,6 +99,7 @@ struct RunBufs {
   uint32_t max_builds;
   uint32_t* report;     // number of the last run, and whether it rebuilt too often
   uint32_t cap;
+  float skin;           // skin of every build, as a fraction of the cell edge; 0: from the speed
   uint32_t later_stride;  // entries of `later` per CTA
   __device__ __forceinline__ vec4_t<T>* p(int k) const { return k ? P[1] : P[0]; }
   __device__ __forceinline__ vec4_t<T>* v(int k) const { return k ? V[1] : V[0]; }
@@ -110,8 +116,10 @@ struct RunBufs {
 
 // One phase's end for the whole grid.  Arrivals only ever count up, by
 // gridDim per barrier, so nothing is reset between barriers or launches.
-// Bounded like grid_barrier; the limit is longer because one phase of a
-// diverged scene (spheres crowded into one cell) may take long.
+// Every wait is bounded: a CTA that gives up records PS_DEVERR_LIST_BARRIER
+// and leaves the kernel, and no later barrier can then complete.  The limit
+// is seconds, because one phase of a diverged scene (spheres crowded into one
+// cell) may take long.
 constexpr uint32_t RUN_BARRIER_SPIN_LIMIT = 1u << 26;
 
 __device__ __forceinline__ bool run_barrier(uint32_t* ctl, uint32_t* err) {
@@ -187,6 +195,16 @@ __device__ __forceinline__ void cell_ranges(const StepBufs<T>& b, const ScenePar
     hi[q] = inb ? b.offset[col + z1] : 0u;
     if (!in_bounds(hi[q], b.n + 1u, b.err)) hi[q] = lo[q] = 0u;
   }
+}
+
+// Cells [c0, c1] of one axis that can hold a point within `reach` of x.
+// The hash is monotonic in x, so the cells of x - reach and x + reach bound
+// them; the pad covers the rounding of x +- reach.
+template <class T>
+__device__ __forceinline__ void axis_span(T x, T reach, T lo, T iv, int32_t nb, int32_t& c0, int32_t& c1) {
+  const T pad = reach + (fabs(x) + fabs(lo)) * T(1.0 / 1048576.0);
+  c0 = axis_cell<T>(x - pad, lo, iv, nb);
+  c1 = axis_cell<T>(x + pad, lo, iv, nb);
 }
 
 // Cells that can hold, at the last build, a partner of a sphere now at P.
@@ -298,7 +316,7 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
   }
   if (k > R.cap) {
     word |= RUN_OVERFLOW, k = 0;
-    if (TAPE) R.ctl[RUN_FULL] = 1u;
+    R.ctl[RUN_FULL] = 1u;
   }
   R.template counts<TAPE>(build, b.n)[i] = (uint16_t)(word | k);
 }
@@ -307,14 +325,15 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
 // partners whose cell is adjacent now, by ascending (cell now, original
 // index).  Every lane of the warp calls it with the same sphere.
 //
-// The lanes take the list's entries (`mine`) side by side, each forms its
-// pair's key and force, and the forces are added in the order of the keys.  With the
-// list overflowed the candidates are those of the cells of the last build,
-// and the smallest key above the last one is looked for in turn.
+// The lanes take the list's entries side by side (`mine`), each forms its
+// pair's key and force, and the forces are added in the order of the keys.
+// A list of more than an entry per lane, and the cells of the last build in
+// place of a list that overflowed, are gone through for the smallest key
+// above the last one in turn.
 template <class T>
-__device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_t mine, const StepBufs<T>& b,
-                                              const SceneParams<T>& sp, const vec4_t<T>* Ps, const vec4_t<T>* Vs,
-                                              T frac, const vec4_t<T>& P, const vec4_t<T>& Vi) {
+__device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_t mine, const uint32_t* list,
+                                              const StepBufs<T>& b, const SceneParams<T>& sp, const vec4_t<T>* Ps,
+                                              const vec4_t<T>* Vs, T frac, const vec4_t<T>& P, const vec4_t<T>& Vi) {
   using A = Ar<T>;
   const unsigned lane = threadIdx.x & 31u;
   vec4_t<T> V = Vi;
@@ -353,8 +372,9 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_
     V.y = A::fma(g, __shfl_sync(0xffffffffu, dy, from), V.y);
     V.z = A::fma(g, __shfl_sync(0xffffffffu, dz, from), V.z);
   };
-  if (!(word & RUN_OVERFLOW)) {
-    uint64_t key = lane < (word & RUN_COUNT) ? key_of(mine) : NONE;
+  const uint32_t nl = word & RUN_COUNT;
+  if (!(word & RUN_OVERFLOW) && nl <= 32u) {
+    uint64_t key = lane < nl ? key_of(mine) : NONE;
     for (uint64_t best = smallest(key); best != NONE; best = smallest(key)) {
       apply(__ffs(__ballot_sync(0xffffffffu, key == best)) - 1);
       if (key == best) key = NONE;
@@ -366,19 +386,27 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_
   for (uint64_t from = 0;;) {
     uint64_t best = NONE;
     T bf = T(0), bdx = T(0), bdy = T(0), bdz = T(0);
-    for (int32_t bx = s.x0; bx <= s.x1; ++bx)
-      for (int32_t by = s.y0; by <= s.y1; ++by) {
-        const uint32_t col = sp.cbase + ((uint32_t)bx * (uint32_t)sp.nb[1] + (uint32_t)by) * (uint32_t)sp.nb[2];
-        const uint32_t j1 = b.offset[col + (uint32_t)s.z1 + 1u];
-        if (!in_bounds(j1, (uint64_t)b.n + 1u, b.err)) continue;
-        for (uint32_t j = b.offset[col + (uint32_t)s.z0] + lane; j < j1; j += 32u) {
-          const uint64_t key = key_of(j);
-          if (key >= from && key < best) {
-            best = key;
-            bf = f, bdx = dx, bdy = dy, bdz = dz;
-          }
-        }
+    auto consider = [&](uint32_t j) {
+      const uint64_t key = key_of(j);
+      if (key >= from && key < best) {
+        best = key;
+        bf = f, bdx = dx, bdy = dy, bdz = dz;
       }
+    };
+    if (word & RUN_OVERFLOW) {
+      for (int32_t bx = s.x0; bx <= s.x1; ++bx)
+        for (int32_t by = s.y0; by <= s.y1; ++by) {
+          const uint32_t col = sp.cbase + ((uint32_t)bx * (uint32_t)sp.nb[1] + (uint32_t)by) * (uint32_t)sp.nb[2];
+          const uint32_t j1 = b.offset[col + (uint32_t)s.z1 + 1u];
+          if (!in_bounds(j1, (uint64_t)b.n + 1u, b.err)) continue;
+          for (uint32_t j = b.offset[col + (uint32_t)s.z0] + lane; j < j1; j += 32u) consider(j);
+        }
+    } else {
+      for (uint32_t k = lane; k < nl; k += 32u) {
+        const uint32_t j = list[(size_t)k * b.n + i] & ~RUN_FAR_CELL;
+        if (in_bounds(j, b.n, b.err)) consider(j);
+      }
+    }
     __syncwarp();
     f = bf, dx = bdx, dy = bdy, dz = bdz;
     const uint64_t next = smallest(best);
@@ -634,11 +662,12 @@ __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T
     const uint32_t i = run_put<T>(l, R, k, true);
     const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
     const uint32_t word = R.template counts<TAPE>(build, b.n)[i];
-    uint32_t mine = lane < R.cap ? R.template lists<TAPE>(build, b.n)[(size_t)lane * b.n + i] & ~RUN_FAR_CELL : i;
+    const uint32_t* list = R.template lists<TAPE>(build, b.n);
+    uint32_t mine = lane < R.cap ? list[(size_t)lane * b.n + i] & ~RUN_FAR_CELL : i;
     vec4_t<T> old = Ps[i];
     const vec4_t<T> Vi = Vs[i];
     if (lane >= (word & RUN_COUNT) || !in_bounds(mine, b.n, b.err)) mine = i;
-    vec4_t<T> V = run_slow<T>(i, word, mine, b, sp, Ps, Vs, (T)frac, old, Vi);
+    vec4_t<T> V = run_slow<T>(i, word, mine, list, b, sp, Ps, Vs, (T)frac, old, Vi);
     old.w = fabs(old.w);
     vec4_t<T> P = old;
     if (TAPE && lane == 0u) run_record<T>(R, b, s, i, P, V, Vi);
@@ -859,14 +888,15 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
         build = rebuilds;
         streak = RUN_CALM_STEPS;
       }
-      lists = streak >= RUN_CALM_STEPS;
+      lists = streak >= RUN_CALM_STEPS || R.skin > 0.0f;
       // (a single fast step, a sphere pushed out of a wall, is no measure)
       // (A recorded run depends on its starting state alone, for the backward
       // pass to give the same sums every time; its builds have to last for
       // the block, and the first, of unknown speed, is kept thin.)
       const float last_for = TAPE ? fmaxf(RUN_STEPS_PER_BUILD, 0.7f * (float)steps) : RUN_STEPS_PER_BUILD;
       const float widest = TAPE && s == 0u ? RUN_SKIN_FIRST : RUN_SKIN_MAX;
-      frac = lists ? fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest) : 0.0f;
+      frac = fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest);
+      frac = R.skin > 0.0f ? R.skin : (lists ? frac : 0.0f);
       if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, n_cells, scatter_blocks, move_blocks))
         return;
       cur = 1 - cur;
@@ -898,6 +928,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   if (blockIdx.x == 0 && threadIdx.x == 3u) R.ctl[RUN_RMAX] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0u) {
     if (TAPE) R.tape_build[steps] = R.ctl[RUN_FULL] == 0u ? 1u : 0u;
+    R.ctl[RUN_BUILDS] += rebuilds - 1u;
     R.ctl[RUN_STREAK] = streak;
     R.report[0] = run_id;
     R.ctl[RUN_BEFORE] = __float_as_uint(before);

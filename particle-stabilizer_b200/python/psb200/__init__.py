@@ -269,14 +269,14 @@ class Simulation:
         return self.list_stats_all()[:2]
 
     def list_stats_all(self) -> tuple[int, int, int]:
-        """(rebuilds, fallbacks, steps run on the grid path by the backoff)."""
+        """(rebuilds, calls in which a list overflowed, steps run on the step kernels by the backoff)."""
         r, f, g = C.c_int64(), C.c_int64(), C.c_int64()
         _check(lib().ps_list_stats(self.h, C.byref(r), C.byref(f), C.byref(g)), "ps_list_stats")
         return int(r.value), int(f.value), int(g.value)
 
     def tune_neighbor_lists(self, trial_steps: int = 100, skins=(0.0, 0.02, 0.05, 0.1, 0.2),
                             max_neighbours: int = 64) -> dict:
-        """ps_tune_neighbor_lists: the fastest skin fraction (0 = grid path)."""
+        """ps_tune_neighbor_lists: the fastest skin fraction (0 = the default path)."""
         sk = np.ascontiguousarray(skins, dtype=np.float64)
         table = np.zeros(len(sk), dtype=np.float64)
         best = C.c_double()
@@ -285,7 +285,7 @@ class Simulation:
         return {"skin_fraction": float(best.value), "skins": [float(x) for x in sk], "ms_table": table.tolist()}
 
     def list_fallbacks(self) -> int:
-        """ps_step calls repeated on the grid path after a list overflow."""
+        """ps_step calls in which some sphere had more neighbours than a list holds."""
         return self.list_stats()[1]
 
     def autotune(self, trial_steps: int = 20, cell_factors=(1.0, 1.05, 1.25, 1.5, 2.0),

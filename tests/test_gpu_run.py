@@ -157,3 +157,19 @@ def test_statistics_at_the_edges_of_the_reduction(need_gpu, prec, n):
         assert s.max_overlap == pytest.approx(o.max_overlap, rel=1e-12, abs=0)
         assert s.kinetic_energy == pytest.approx(o.kinetic_energy, rel=1e-12)
         assert list(s.min_pos) == list(o.min_pos) and list(s.max_pos) == list(o.max_pos)
+
+
+@pytest.mark.parametrize("cap", [1, 31, 33, 64, 255, 4000])
+def test_set_lists_of_any_capacity(need_gpu, cap):
+    # shorter than the lists, one entry per lane and more, beyond the count word
+    sc = faster(crowd(200), 30.0)
+    want, _ = both([sc], "f32", (90, 40))
+    with psb200.Simulation(sc, "f32") as sim:
+        sim.set_state()
+        sim.set_neighbor_lists(0.3, cap)
+        sim.step(90)
+        sim.step(40)
+        got = (sim.get_state(), *sim.buckets())
+        overflows = sim.list_stats()[1]
+    assert same(got, want)
+    assert (overflows > 0) == (cap < 200)  # all 200 small spheres are neighbours of the large one
