@@ -113,6 +113,7 @@ template <class T>
 struct SceneParams {
   T grid_lo[3];   // grid domain minimum
   T interval;     // cell edge
+  T inv_interval, inv_interval2;  // 1 / interval, approximately, and its square
   T box_lo[3];    // box walls
   T box_hi[3];
   T e_lo[3];      // restitution of the x/y/z min walls

@@ -561,6 +561,8 @@ SceneParams<T> make_params(const ps_scene_desc& d, const GridHost& g, int64_t pb
     sp.mesh_hi[a] = (T)g.mesh_hi[a];
   }
   sp.interval = (T)g.interval;
+  sp.inv_interval = (T)(1.0 / g.interval);
+  sp.inv_interval2 = sp.inv_interval * sp.inv_interval;
   sp.e_lo[0] = (T)d.e_wall[PS_XMIN];
   sp.e_lo[1] = (T)d.e_wall[PS_YMIN];
   sp.e_lo[2] = (T)d.e_wall[PS_ZMIN];
