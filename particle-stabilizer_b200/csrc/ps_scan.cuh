@@ -5,9 +5,9 @@
 //
 // One launch, one read and one write per element.  Each CTA takes a tile of
 // SCAN_TILE elements in ticket order (an atomic counter, so every
-// predecessor tile is already running), publishes its aggregate, then all
-// its threads look back over 256 predecessor status words per round until
-// one holds an inclusive prefix.  A status word packs (value << 32 | flag)
+// predecessor tile is already running), publishes its aggregate, then its
+// first warp looks back over 32 predecessor status words at a time until one
+// holds an inclusive prefix.  A status word packs (value << 32 | flag)
 // so value and flag travel in one 64-bit store.  Every wait on a predecessor
 // is bounded: after SCAN_SPIN_LIMIT polls the thread records
 // PS_DEVERR_SCAN_TIMEOUT in the error word and takes the missing value as 0,
@@ -58,130 +58,170 @@ __device__ __forceinline__ void scan_st(uint64_t* p, uint64_t v) {
   cuda::atomic_ref<uint64_t, cuda::thread_scope_device>(*p).store(v, cuda::memory_order_relaxed);
 }
 
-// in and out may alias.  `scratch` must be zeroed before the launch.
-__global__ void __launch_bounds__(SCAN_THREADS, 8) k_exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n,
-                                                                     uint64_t* scratch, uint32_t* err) {
-  __shared__ uint32_t s_warp[SCAN_THREADS / 32];
-  __shared__ uint32_t s_tile;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint64_t* status = scratch + 1;
-
-  if (tid == 0) s_tile = atomicAdd(reinterpret_cast<unsigned int*>(scratch), 1u);
-  __syncthreads();
-  const int64_t tile = s_tile;
-  const int64_t base = tile * SCAN_TILE + (int64_t)tid * SCAN_ITEMS;
-
-  // pass 1: per-thread sum only (values are re-read after the look-back, from
-  // L1/L2, so a CTA holds few registers and every tile is resident at once)
-  const bool vec = base + SCAN_ITEMS <= n && (((uintptr_t)(in + base)) & 15) == 0;
-  uint32_t local = 0;
-  if (vec) {
-    const uint4* q = reinterpret_cast<const uint4*>(in + base);
+// A warp's 32 x ITEMS contiguous elements from wbase, as rows of 32 uint4: in
+// row k lane l holds elements 4 * (32 k + l) .. + 3, so every load and store
+// of a warp covers 512 contiguous bytes.  VEC: all of them are there and
+// 16-byte aligned.
+template <int ROWS, bool VEC, class LD>
+__device__ __forceinline__ void scan_load(uint4 (&v)[ROWS], int64_t wbase, int64_t n, int lane, LD ld) {
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS / 4; ++k) {
-      const uint4 w = q[k];
-      local += w.x + w.y + w.z + w.w;
+  for (int k = 0; k < ROWS; ++k) {
+    const int64_t e = wbase + 4 * (32 * k + lane);
+    if (VEC) {
+      v[k] = ld.four(e);
+    } else {
+      v[k].x = e + 0 < n ? ld.one(e + 0) : 0u;
+      v[k].y = e + 1 < n ? ld.one(e + 1) : 0u;
+      v[k].z = e + 2 < n ? ld.one(e + 2) : 0u;
+      v[k].w = e + 3 < n ? ld.one(e + 3) : 0u;
     }
-  } else {
-    for (int k = 0; k < SCAN_ITEMS; ++k) local += (base + k < n) ? in[base + k] : 0u;
   }
+}
 
-  // warp-inclusive scan of the per-thread sums
-  uint32_t inc = local;
+// Exclusive prefixes of a warp's rows (excl[k]: of the lane's uint4 of row k,
+// within the warp); returns the warp's total.
+template <int ROWS>
+__device__ __forceinline__ uint32_t scan_rows(const uint4 (&v)[ROWS], uint32_t (&excl)[ROWS], int lane) {
+  uint32_t carry = 0;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
-    if (lane >= d) inc += t;
+  for (int k = 0; k < ROWS; ++k) {
+    const uint32_t sum = v[k].x + v[k].y + v[k].z + v[k].w;
+    uint32_t inc = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += t;
+    }
+    excl[k] = carry + inc - sum;
+    carry += __shfl_sync(0xffffffffu, inc, 31);
   }
-  if (lane == 31) s_warp[warp] = inc;
+  return carry;
+}
+
+template <int ROWS, bool VEC>
+__device__ __forceinline__ void scan_store(const uint4 (&v)[ROWS], const uint32_t (&excl)[ROWS], uint32_t off,
+                                           uint32_t* out, int64_t wbase, int64_t n, int lane) {
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    const int64_t e = wbase + 4 * (32 * k + lane);
+    uint4 y;
+    y.x = off + excl[k];
+    y.y = y.x + v[k].x;
+    y.z = y.y + v[k].y;
+    y.w = y.z + v[k].z;
+    if (VEC) {
+      *reinterpret_cast<uint4*>(out + e) = y;
+    } else {
+      if (e + 0 < n) out[e + 0] = y.x;
+      if (e + 1 < n) out[e + 1] = y.y;
+      if (e + 2 < n) out[e + 2] = y.z;
+      if (e + 3 < n) out[e + 3] = y.w;
+    }
+  }
+}
+
+constexpr int SCAN_WINDOWS = 4;
+
+struct ScanPlain {
+  const uint32_t* in;
+  __device__ __forceinline__ uint4 four(int64_t e) const { return *reinterpret_cast<const uint4*>(in + e); }
+  __device__ __forceinline__ uint32_t one(int64_t e) const { return in[e]; }
+};
+
+// Prefix of everything before `tile`, by the first warp: publishes the tile's
+// aggregate, then adds predecessors' words, 32 * SCAN_WINDOWS read together,
+// back to the nearest inclusive prefix, and publishes its own.  The tiles of a
+// wave publish their aggregates at about the same time, and prefixes reach
+// them a round's reach per round trip (1M counts: 9.4 us with 64 words a
+// round, 8.3 us with 128, 8.2 us with 256).
+__device__ __forceinline__ uint32_t scan_look_back(uint64_t* status, int64_t tile, uint32_t tile_sum, int lane,
+                                                   uint32_t* err) {
+  uint32_t prefix = 0;
+  if (tile == 0) {
+    if (lane == 0) scan_st(&status[0], ((uint64_t)tile_sum << 32) | SCAN_FLAG_PREFIX);
+    return 0u;
+  }
+  if (lane == 0) scan_st(&status[tile], ((uint64_t)tile_sum << 32) | SCAN_FLAG_AGG);
+  uint32_t spins = 0;
+  bool timed_out = false, done = false;
+  for (int64_t pred = tile - 1; !done; pred -= 32 * SCAN_WINDOWS) {
+    uint64_t s[SCAN_WINDOWS];
+#pragma unroll
+    for (int w = 0; w < SCAN_WINDOWS; ++w) {
+      const int64_t idx = pred - 32 * w - lane;
+      s[w] = idx >= 0 ? scan_ld(&status[idx]) : (uint64_t)SCAN_FLAG_PREFIX;
+    }
+#pragma unroll
+    for (int w = 0; w < SCAN_WINDOWS; ++w) {
+      if (done) break;
+      while (__any_sync(0xffffffffu, (s[w] & 3u) == SCAN_FLAG_NONE)) {
+        if (++spins > SCAN_SPIN_LIMIT) {
+          timed_out = true;
+          if ((s[w] & 3u) == SCAN_FLAG_NONE) s[w] = (uint64_t)SCAN_FLAG_PREFIX;  // give up: value 0
+          break;
+        }
+        if (spins > 8u) __nanosleep(spins < 64u ? 32 : 256);
+        if ((s[w] & 3u) == SCAN_FLAG_NONE) s[w] = scan_ld(&status[pred - 32 * w - lane]);
+      }
+      const unsigned pm = __ballot_sync(0xffffffffu, (s[w] & 3u) == SCAN_FLAG_PREFIX);
+      const int stop = pm ? (__ffs(pm) - 1) : 31;
+      prefix += __reduce_add_sync(0xffffffffu, (lane <= stop) ? (uint32_t)(s[w] >> 32) : 0u);
+      done = pm != 0u;
+    }
+  }
+  if (timed_out && lane == 0) atomicOr(err, PS_DEVERR_SCAN_TIMEOUT);
+  if (lane == 0) scan_st(&status[tile], ((uint64_t)(prefix + tile_sum) << 32) | SCAN_FLAG_PREFIX);
+  return prefix;
+}
+
+// in and out may alias.  `scratch` must be zeroed before the launch.
+//
+// What bounds it: memory, one read and one write, and for small inputs the
+// launch.  Values stay in registers between the two passes over a tile, four
+// CTAs of 256 threads per SM (five, or three or four of 512: 32 to 33 us at
+// 8M).  With the clearing of the scratch, 7,953,877 counts took 39.5 us and 64M
+// 221 us while a thread's 32 elements were contiguous (a warp's load touched
+// 32 lines) and read again after the look-back; in rows 30.5 us and 163 us.
+template <bool VEC>
+__device__ __forceinline__ void scan_tile_look_back(int64_t tile, const uint32_t* in, uint32_t* out, int64_t n,
+                                                    uint64_t* status, uint32_t* err) {
+  constexpr int ROWS = SCAN_ITEMS / 4;
+  __shared__ uint32_t s_warp[SCAN_THREADS / 32];
+  __shared__ uint32_t s_prefix;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t wbase = tile * SCAN_TILE + (int64_t)warp * (32 * SCAN_ITEMS);
+  uint4 v[ROWS];
+  scan_load<ROWS, VEC>(v, wbase, n, lane, ScanPlain{in});
+  uint32_t excl[ROWS];
+  const uint32_t total = scan_rows<ROWS>(v, excl, lane);
+  if (lane == 0) s_warp[warp] = total;
   __syncthreads();
-  uint32_t warp_excl = 0, tile_sum = 0;
+  uint32_t before = 0, tile_sum = 0;
 #pragma unroll
   for (int w = 0; w < SCAN_THREADS / 32; ++w) {
-    const uint32_t t = s_warp[w];
-    warp_excl += (w < warp) ? t : 0u;
-    tile_sum += t;
+    before += (w < warp) ? s_warp[w] : 0u;
+    tile_sum += s_warp[w];
   }
-
-  // publish the aggregate, then warp 0 looks back 32 predecessors per round
-  __shared__ uint32_t s_prefix;
   if (warp == 0) {
-    uint32_t prefix = 0;
-    if (tile == 0) {
-      if (lane == 0) scan_st(&status[0], ((uint64_t)tile_sum << 32) | SCAN_FLAG_PREFIX);
-    } else {
-      if (lane == 0) scan_st(&status[tile], ((uint64_t)tile_sum << 32) | SCAN_FLAG_AGG);
-      int64_t pred = tile - 1;  // predecessor read by lane 0 this round
-      uint32_t spins = 0;
-      bool timed_out = false;
-      while (true) {
-        const int64_t idx = pred - lane;
-        uint64_t s = (idx >= 0) ? scan_ld(&status[idx]) : (uint64_t)SCAN_FLAG_PREFIX;
-        unsigned ns = 32;
-        while (__any_sync(0xffffffffu, (s & 3u) == SCAN_FLAG_NONE)) {
-          if (++spins > SCAN_SPIN_LIMIT) {
-            timed_out = true;
-            if ((s & 3u) == SCAN_FLAG_NONE) s = (uint64_t)SCAN_FLAG_PREFIX;  // give up: value 0
-            break;
-          }
-          __nanosleep(ns);
-          ns = ns < 512 ? 2 * ns : 512;
-          if ((s & 3u) == SCAN_FLAG_NONE) s = scan_ld(&status[idx]);
-        }
-        const unsigned pm = __ballot_sync(0xffffffffu, (s & 3u) == SCAN_FLAG_PREFIX);
-        const int stop = pm ? (__ffs(pm) - 1) : 31;
-        uint32_t contrib = (lane <= stop) ? (uint32_t)(s >> 32) : 0u;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, d);
-        prefix += contrib;
-        if (pm) break;
-        pred -= 32;
-      }
-      if (timed_out && lane == 0) atomicOr(err, PS_DEVERR_SCAN_TIMEOUT);
-      if (lane == 0) scan_st(&status[tile], ((uint64_t)(prefix + tile_sum) << 32) | SCAN_FLAG_PREFIX);
-    }
+    const uint32_t prefix = scan_look_back(status, tile, tile_sum, lane, err);
     if (lane == 0) s_prefix = prefix;
   }
   __syncthreads();
-  const uint32_t prefix = s_prefix;
+  scan_store<ROWS, VEC>(v, excl, s_prefix + before, out, wbase, n, lane);
+}
 
-  // pass 2: re-read (in may alias out: each thread reads its own elements
-  // before writing them) and write the exclusive prefixes
-  asm volatile("" ::: "memory");
-  uint32_t run = prefix + warp_excl + (inc - local);
-  if (vec) {
-    const uint4* q = reinterpret_cast<const uint4*>(in + base);
-    uint4* w = reinterpret_cast<uint4*>(out + base);
-    const bool vec_out = (((uintptr_t)(out + base)) & 15) == 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS / 4; ++k) {
-      const uint4 x = q[k];
-      uint4 y;
-      y.x = run;
-      run += x.x;
-      y.y = run;
-      run += x.y;
-      y.z = run;
-      run += x.z;
-      y.w = run;
-      run += x.w;
-      if (vec_out) {
-        w[k] = y;
-      } else {
-        out[base + 4 * k + 0] = y.x;
-        out[base + 4 * k + 1] = y.y;
-        out[base + 4 * k + 2] = y.z;
-        out[base + 4 * k + 3] = y.w;
-      }
-    }
-  } else {
-    for (int k = 0; k < SCAN_ITEMS; ++k)
-      if (base + k < n) {
-        const uint32_t x = in[base + k];
-        out[base + k] = run;
-        run += x;
-      }
-  }
+__global__ void __launch_bounds__(SCAN_THREADS, 4) k_exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n,
+                                                                     uint64_t* scratch, uint32_t* err) {
+  __shared__ uint32_t s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(reinterpret_cast<unsigned int*>(scratch), 1u);
+  __syncthreads();
+  const int64_t tile = s_tile;
+  // 16-byte accesses where the tile is whole and both arrays are aligned (a
+  // tile's offset keeps the alignment)
+  if ((tile + 1) * SCAN_TILE <= n && ((((uintptr_t)in) | ((uintptr_t)out)) & 15) == 0)
+    scan_tile_look_back<true>(tile, in, out, n, scratch + 1, err);
+  else
+    scan_tile_look_back<false>(tile, in, out, n, scratch + 1, err);
 }
 
 // Exclusive scan whose per-tile totals are already known: tile_sum[t] holds
@@ -190,16 +230,22 @@ __global__ void __launch_bounds__(SCAN_THREADS, 8) k_exclusive_scan_u32(const ui
 // prefix from the totals before it and scans its own tile: one read and one
 // write per element, and no CTA waits on another.
 //
-// Layout: warp w of the CTA owns the contiguous 1024 elements
-// [w*1024, (w+1)*1024) of the tile as 8 rows of 32 uint4; in row k lane l
-// holds elements 4*(32k + l) .. +3, so every load and store instruction of a
-// warp covers 512 contiguous bytes.  Rows are scanned with warp shuffles and
-// carried from row to row; warps are combined through shared memory.
+// Layout: warp w of the CTA owns the contiguous 32 * ITEMS elements from
+// w * 32 * ITEMS of the tile in rows (scan_load).  Rows are scanned with warp
+// shuffles and carried from row to row; warps are combined through shared
+// memory.
 // One CTA scans tile `tile`; a CTA that scans several tiles in turn
 // synchronises its threads between them.
 // ITEMS elements per thread: STEP_SCAN_ITEMS_LARGE (8,192-cell tiles) for
 // large grids, STEP_SCAN_ITEMS_SMALL (2,048) where a grid would fill too few
 // CTAs with the large tile.
+template <bool COH>
+struct ScanCounts {
+  const uint32_t* in;
+  __device__ __forceinline__ uint4 four(int64_t e) const { return __ldcs(reinterpret_cast<const uint4*>(in + e)); }
+  __device__ __forceinline__ uint32_t one(int64_t e) const { return ld_pl<COH>(in + e); }
+};
+
 template <bool COH, int ITEMS>
 __device__ __forceinline__ void scan_tile_with_sums(int64_t tile, const uint32_t* __restrict__ in,
                                                     uint32_t* __restrict__ out, int64_t n,
@@ -219,55 +265,21 @@ __device__ __forceinline__ void scan_tile_with_sums(int64_t tile, const uint32_t
 
   const bool full = wbase + 32 * ITEMS <= n;
   uint4 v[ROWS];
-#pragma unroll
-  for (int k = 0; k < ROWS; ++k) {
-    const int64_t e = wbase + 4 * (32 * k + lane);
-    if (full) {
-      v[k] = __ldcs(reinterpret_cast<const uint4*>(in + e));
-    } else {
-      v[k].x = e + 0 < n ? ld_pl<COH>(in + e + 0) : 0u;
-      v[k].y = e + 1 < n ? ld_pl<COH>(in + e + 1) : 0u;
-      v[k].z = e + 2 < n ? ld_pl<COH>(in + e + 2) : 0u;
-      v[k].w = e + 3 < n ? ld_pl<COH>(in + e + 3) : 0u;
-    }
-  }
-  // scan row by row inside the warp; `carry` is the warp's running total
+  if (full)
+    scan_load<ROWS, true>(v, wbase, n, lane, ScanCounts<COH>{in});
+  else
+    scan_load<ROWS, false>(v, wbase, n, lane, ScanCounts<COH>{in});
   uint32_t excl[ROWS];
-  uint32_t carry = 0;
-#pragma unroll
-  for (int k = 0; k < ROWS; ++k) {
-    const uint32_t sum = v[k].x + v[k].y + v[k].z + v[k].w;
-    uint32_t inc = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += t;
-    }
-    excl[k] = carry + inc - sum;
-    carry += __shfl_sync(0xffffffffu, inc, 31);
-  }
-  if (lane == 0) s_warp[warp] = carry;
+  const uint32_t total = scan_rows<ROWS>(v, excl, lane);
+  if (lane == 0) s_warp[warp] = total;
   __syncthreads();
   uint32_t off = 0;
 #pragma unroll
   for (int w = 0; w < SCAN_THREADS / 32; ++w) off += s_pre[w] + ((w < warp) ? s_warp[w] : 0u);
-#pragma unroll
-  for (int k = 0; k < ROWS; ++k) {
-    const int64_t e = wbase + 4 * (32 * k + lane);
-    uint4 y;
-    y.x = off + excl[k];
-    y.y = y.x + v[k].x;
-    y.z = y.y + v[k].y;
-    y.w = y.z + v[k].z;
-    if (full) {
-      *reinterpret_cast<uint4*>(out + e) = y;
-    } else {
-      if (e + 0 < n) out[e + 0] = y.x;
-      if (e + 1 < n) out[e + 1] = y.y;
-      if (e + 2 < n) out[e + 2] = y.z;
-      if (e + 3 < n) out[e + 3] = y.w;
-    }
-  }
+  if (full)
+    scan_store<ROWS, true>(v, excl, off, out, wbase, n, lane);
+  else
+    scan_store<ROWS, false>(v, excl, off, out, wbase, n, lane);
 }
 
 template <int ITEMS>
