@@ -140,6 +140,7 @@ struct ps_sim {
   std::vector<SceneParams<double>> sp64;
 
   std::map<int64_t, cudaGraphExec_t> graphs;
+  std::map<int64_t, int> eager_uses;      // blocks of a length that were launched without a graph
   int64_t graph_block = 200;  // steps per captured CUDA graph (ps_autotune may change it)
   int32_t walk = WALK_ADAPTIVE;  // neighbour walk of the contact kernel (WALK_LANE / WALK_WARP / WALK_ADAPTIVE)
   int32_t contact_block = 256;    // threads per CTA of the contact kernel (WALK_LANE: 128, 256, 512; others: 256)
@@ -1580,13 +1581,16 @@ extern "C" int ps_get_state(ps_sim* s, double* out, int64_t n_total) {
 
 namespace {
 
-// Spheres from which the step kernels of a block shorter than graph_block
-// are launched one by one: each then runs for longer than its launch takes,
-// so that a graph gains nothing, and capturing one takes 1.5 ms per hundred
-// steps (first 100 steps of a 1M-sphere scene
-// and download: 11.6 ms with a graph, 10.3 ms without).  Longer calls use
-// graphs, which also keep the call asynchronous.
+// From EAGER_MIN_SPHERES the step kernels of a block shorter than graph_block
+// are launched one by one the first EAGER_USES times its length comes: each
+// kernel then runs for longer than its launch takes, and capturing a graph
+// takes 2 to 3 ms per hundred steps (first 100 steps of a 1M-sphere scene and
+// download: 13.1 to 13.9 ms with a graph, 10.4 to 10.9 ms without).  A length
+// that keeps coming is worth the graph: the same 100 steps repeated take 0.4
+// to 0.8 % longer one by one (9.38 to 9.66 ms against 9.45 to 9.73 ms).  The
+// odd lengths around a probe seldom come again.
 constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
+constexpr int EAGER_USES = 2;
 
 // Run n_steps on the step kernels as CUDA graphs of up to graph_block steps,
 // asynchronously.
@@ -1596,14 +1600,16 @@ int step_graphs(ps_sim* s, int64_t n_steps) {
   int64_t left = n_steps;
   while (left > 0) {
     const int64_t L = std::min(left, s->graph_block);
-    if (L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES) {
+    auto it = s->graphs.find(L);
+    if (it == s->graphs.end() && L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES &&
+        s->eager_uses[L] < EAGER_USES) {
+      s->eager_uses[L] += 1;
       s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
       PS_CUDA(cudaGetLastError());
       s->last_launches += 1 + 4 * L;
       left -= L;
       continue;
     }
-    auto it = s->graphs.find(L);
     if (it == s->graphs.end()) {
       cudaGraph_t graph = nullptr;
       PS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -1867,6 +1873,7 @@ namespace {
 int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
+  s->eager_uses.clear();
   void** bufs_to_free[] = {&s->cell_arena, &s->d_tri, &s->d_aabb, &s->adj_arena};
   for (void** b : bufs_to_free) {
     cudaFree(*b);
