@@ -17,6 +17,7 @@
 #include <cstring>
 #include <limits>
 #include <map>
+#include <set>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -140,7 +141,7 @@ struct ps_sim {
   std::vector<SceneParams<double>> sp64;
 
   std::map<int64_t, cudaGraphExec_t> graphs;
-  std::map<int64_t, int> eager_uses;      // blocks of a length that were launched without a graph
+  std::set<int64_t> eager_lengths;        // block lengths that were launched without a graph
   int64_t graph_block = 200;  // steps per captured CUDA graph (ps_autotune may change it)
   int32_t walk = WALK_ADAPTIVE;  // neighbour walk of the contact kernel (WALK_LANE / WALK_WARP / WALK_ADAPTIVE)
   int32_t contact_block = 256;    // threads per CTA of the contact kernel (WALK_LANE: 128, 256, 512; others: 256)
@@ -1582,15 +1583,15 @@ extern "C" int ps_get_state(ps_sim* s, double* out, int64_t n_total) {
 namespace {
 
 // From EAGER_MIN_SPHERES the step kernels of a block shorter than graph_block
-// are launched one by one the first EAGER_USES times its length comes: each
-// kernel then runs for longer than its launch takes, and capturing a graph
-// takes 2 to 3 ms per hundred steps (first 100 steps of a 1M-sphere scene and
-// download: 13.1 to 13.9 ms with a graph, 10.4 to 10.9 ms without).  A length
-// that keeps coming is worth the graph: the same 100 steps repeated take 0.4
-// to 0.8 % longer one by one (9.38 to 9.66 ms against 9.45 to 9.73 ms).  The
-// odd lengths around a probe seldom come again.
+// are launched one by one the first time its length comes: each kernel then
+// runs for longer than its launch takes, and capturing a graph takes 2 to 3 ms
+// per hundred steps (first 100 steps of a 1M-sphere scene and download: 13.1
+// to 13.9 ms with a graph, 10.4 to 10.9 ms without).  The second time, it is
+// captured, so that a program's warm-up still takes that: the same 100 steps
+// repeated take 0.4 to 0.8 % longer one by one (9.38 to 9.66 ms against 9.45
+// to 9.73 ms).  The odd lengths around a probe seldom come again.  The trials
+// of ps_autotune (run_off) warm up once and always use graphs.
 constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
-constexpr int EAGER_USES = 2;
 
 // Run n_steps on the step kernels as CUDA graphs of up to graph_block steps,
 // asynchronously.
@@ -1602,8 +1603,7 @@ int step_graphs(ps_sim* s, int64_t n_steps) {
     const int64_t L = std::min(left, s->graph_block);
     auto it = s->graphs.find(L);
     if (it == s->graphs.end() && L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES &&
-        s->eager_uses[L] < EAGER_USES) {
-      s->eager_uses[L] += 1;
+        !s->run_off && s->eager_lengths.insert(L).second) {
       s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
       PS_CUDA(cudaGetLastError());
       s->last_launches += 1 + 4 * L;
@@ -1873,7 +1873,7 @@ namespace {
 int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
-  s->eager_uses.clear();
+  s->eager_lengths.clear();
   void** bufs_to_free[] = {&s->cell_arena, &s->d_tri, &s->d_aabb, &s->adj_arena};
   for (void** b : bufs_to_free) {
     cudaFree(*b);
@@ -2059,6 +2059,7 @@ extern "C" int ps_tune_neighbor_lists(ps_sim* s, int64_t trial_steps, const doub
     if (r == PS_OK) r = ps_step(s, trial_steps);
     if (r == PS_OK) r = load_state(s, saved);
     if (r != PS_OK) return r;
+    s->eager_lengths.clear();  // no large scene's capture inside the timed call (the warm-up's probe changed its length)
     cudaEventRecord(ea, s->stream);
     r = ps_step(s, trial_steps);
     cudaEventRecord(eb, s->stream);
