@@ -337,10 +337,10 @@ def mesh_measure(psb200, scenes_mod, device, steps: int) -> dict:
 
 
 def lists_measure(psb200, scenes_mod, device, only=None, fixed_skin=None) -> dict:
-    """Neighbour-list mode against the grid path on the same steps from the
+    """Neighbour-list mode against the default path on the same steps from the
     same state (after 100 warm-up steps), with the final states compared
     bit for bit.  The skin fraction is chosen by ps_tune_neighbor_lists
-    (100 trial steps per candidate, 0 = grid path) from that state, unless
+    (100 trial steps per candidate, 0 = default path) from that state, unless
     `fixed_skin` gives it (profiling runs, where the tuner's timings mean
     nothing).
     Scenes: 1M spheres with a soft spring (FP32 and FP64), the 1M-sphere
@@ -455,8 +455,8 @@ def reference_cuda_measure(psb200, scenes_mod, device, steps: int = 200, warm: i
 # log-uniform in [0.25, 2.5]; all other draws identical).
 def walks_measure(psb200, scenes_mod, device) -> dict:
     """The contact kernel's neighbour walks on the same states: per launch of
-    the contact kernel (eager steps, CUDA events) and per graph step (best of
-    three), for the per-lane walk, the warp walk and the adaptive walk (the
+    the contact kernel (eager steps, CUDA events) and per step of ps_step (best of
+    three; calls of many steps do not use this kernel on settled scenes), for the per-lane walk, the warp walk and the adaptive walk (the
     default), each at 256 threads per CTA, with a hash of the final state
     (equal for every walk).  Scenes: this benchmark's 1M scene (steps 1-20),
     the soft 1M scene in FP32 and FP64 and the 1M dense pile after 100 steps,
