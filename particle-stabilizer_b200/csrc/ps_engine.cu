@@ -180,6 +180,7 @@ struct ps_sim {
   unsigned run_grid = 0;                  // CTAs: one wave, or fewer for a small scene
   bool run_own = false;                   // those CTAs have a thread for every sphere
   bool run_off = false;                   // ps_autotune times the step kernels
+  uint32_t run_turn = 0, list_turn = 0;   // launches on the control words of run_arena and of list_arena
   uint32_t run_id = 0, run_seen = 0;      // runs launched, and the last one whose report was read (run_read)
   bool run_settled = false;               // what that report said
   bool run_known = false;                 // a run was launched on this grid
@@ -1076,6 +1077,7 @@ RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
   R.tape_row_bytes = 0;
   R.tape_build = nullptr;
   R.max_builds = 0;
+  R.bar = R.bar_next = nullptr;  // (run_launch)
   R.report = set ? R.ctl + RUN_REPORT : s->err + ERR_RUN;
   return R;
 }
@@ -1095,7 +1097,10 @@ int run_prepare(ps_sim* s) {
 }
 
 template <class T, bool MULTI, bool MESH, bool TAPE>
-int run_launch(ps_sim* s, uint32_t steps, const RunBufs<T>& R, uint32_t run_id) {
+int run_launch(ps_sim* s, uint32_t steps, RunBufs<T> R, uint32_t run_id) {
+  uint32_t& turn = R.ctl == static_cast<uint32_t*>(s->list_arena) ? s->list_turn : s->run_turn;
+  R.bar = R.ctl + (turn & 1u ? RUN_BAR_ODD : RUN_BAR);
+  R.bar_next = R.ctl + (turn & 1u ? RUN_BAR : RUN_BAR_ODD);
   const StepBufs<T> b = bufs<T>(s);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(s->run_grid);
@@ -1112,6 +1117,7 @@ int run_launch(ps_sim* s, uint32_t steps, const RunBufs<T>& R, uint32_t run_id) 
   PS_CUDA(cudaLaunchKernelEx(&cfg, s->run_own ? k_run<T, MULTI, MESH, true, TAPE> : k_run<T, MULTI, MESH, false, TAPE>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
                              R, steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
                              (uint32_t)move_blocks(s->n_total, 0), run_id));
+  ++turn;  // (a launch that failed has cleared nothing)
   return PS_OK;
 }
 

@@ -71,7 +71,7 @@ constexpr uint32_t RUN_LIST_CAP_MAX = RUN_COUNT;  // list capacity that a progra
 
 // control words
 enum : int {
-  RUN_BAR = 0,      // grid barrier: arrivals so far (64 bits)
+  RUN_BAR = 0,      // grid barrier of even launches: arrivals so far (64 bits)
   RUN_MAXD = 2,     // largest squared displacement of a step, in cells (3 words, by step)
   RUN_STREAK = 5,   // calm steps up to now
   RUN_RMAX = 6,     // largest radius, in cells of its scene
@@ -79,6 +79,7 @@ enum : int {
   RUN_FULL = 8,     // a sphere had more neighbours than a list holds
   RUN_BUILDS = 9,   // builds after a run's first
   RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
+  RUN_BAR_ODD = 12, // grid barrier of odd launches
 };
 
 template <class T>
@@ -90,6 +91,7 @@ struct RunBufs {
   uint32_t* tris;       // [k][slot]: triangles within reach (triangle containers)
   uint32_t* later;      // per CTA: the slots of its RunLate beyond what fits in shared memory
   uint32_t* ctl;
+  uint32_t *bar, *bar_next;  // grid barrier of this launch, and of the next one on these control words
   // recording for the backward pass (null otherwise): rows of the tape, one
   // list and count array per build (max_builds of them), the build of every
   // step, and after them 1 when the run is complete
@@ -115,19 +117,21 @@ struct RunBufs {
 };
 
 // One phase's end for the whole grid.  Arrivals only ever count up, by
-// gridDim per barrier, so nothing is reset between barriers or launches.
+// gridDim per barrier, so nothing is reset between the barriers of a launch.
+// A launch's count starts at zero whatever the grid of the one before it and
+// however that ended: two words take turns, and a launch clears the other one.
 // Every wait is bounded: a CTA that gives up records PS_DEVERR_LIST_BARRIER
 // and leaves the kernel, and no later barrier can then complete.  The limit
 // is seconds, because one phase of a diverged scene (spheres crowded into one
 // cell) may take long.
 constexpr uint32_t RUN_BARRIER_SPIN_LIMIT = 1u << 26;
 
-__device__ __forceinline__ bool run_barrier(uint32_t* ctl, uint32_t* err) {
+__device__ __forceinline__ bool run_barrier(uint32_t* word, uint32_t* err) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(ctl + RUN_BAR);
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(word);
     unsigned long long seen;
     asm volatile("fence.acq_rel.gpu;" ::: "memory");  // the CTA's writes, gathered by the barrier above
     asm volatile("atom.add.release.gpu.global.u64 %0, [%1], 1;" : "=l"(seen) : "l"(bar) : "memory");
@@ -492,7 +496,7 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
       }
       count_cell(b.count, b.tile_sum, c, valid && in_bounds(c, b.n_scan - 1u, b.err), b.tile_shift);
     }
-    if (!run_barrier(R.ctl, b.err)) return false;
+    if (!run_barrier(R.bar, b.err)) return false;
   }
   for (uint32_t t = blockIdx.x; t < b.n_tiles; t += gridDim.x) {
     __syncthreads();  // the tile scan reuses its shared arrays
@@ -501,17 +505,17 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
     else
       scan_tile_with_sums<true, STEP_SCAN_ITEMS_SMALL>(t, b.count, b.offset, n_cells, b.tile_sum);
   }
-  if (!run_barrier(R.ctl, b.err)) return false;
+  if (!run_barrier(R.bar, b.err)) return false;
   for (uint32_t blk = blockIdx.x; blk < scatter_blocks; blk += gridDim.x)
     scatter_block<true>(blk, b.cell, b.slot, b.orig, b.offset, b.tmp, b.count, b.n, b.tile_sum, b.n_tiles, b.err);
-  if (!run_barrier(R.ctl, b.err)) return false;
+  if (!run_barrier(R.bar, b.err)) return false;
   StepBufs<T> mb = b;
   mb.P1 = R.p(cur);
   mb.V1 = R.v(cur);
   mb.P0 = R.p(1 - cur);
   mb.V0 = R.v(1 - cur);
   for (uint32_t blk = blockIdx.x; blk < move_blocks; blk += gridDim.x) rank_move_block<T, true>(blk, mb);
-  if (!run_barrier(R.ctl, b.err)) return false;
+  if (!run_barrier(R.bar, b.err)) return false;
   if (frac > 0.0f) {
     const vec4_t<T>* Ps = R.p(1 - cur);
     const T rmax = (T)__uint_as_float(R.ctl[RUN_RMAX]) * T(1.0001);
@@ -894,6 +898,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
           const __grid_constant__ RunBufs<T> R, uint32_t steps, int64_t n_cells, uint32_t scatter_blocks,
           uint32_t move_blocks, uint32_t run_id) {
   uint32_t* maxd = R.ctl + RUN_MAXD;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.bar_next) = 0ull;
   uint32_t streak = *reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_STREAK);
   run_begin<T, MULTI, MESH>(b, sp0, mv, R);
   int cur = 1;           // buffer with the state before the step's contacts
@@ -907,7 +912,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   if (!(before > 0.0f) || TAPE) before = INFINITY;
   RunOwn<T> own;
   for (uint32_t s = 0; s < steps; ++s) {
-    if (!run_barrier(R.ctl, b.err)) return;
+    if (!run_barrier(R.bar, b.err)) return;
     const float m = sqrtf(__uint_as_float(*reinterpret_cast<volatile uint32_t*>(maxd + s % 3u)));
     if (blockIdx.x == 0 && threadIdx.x == 0) maxd[(s + 2u) % 3u] = 0u;
     streak = m <= RUN_CALM_MAX ? (streak < RUN_CALM_STEPS ? streak + 1u : streak) : 0u;
@@ -948,7 +953,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     cur = 1 - cur;
   }
   // the state is in buffer `cur`; at rest the positions are in P0 and the velocities in V1
-  if (!run_barrier(R.ctl, b.err)) return;
+  if (!run_barrier(R.bar, b.err)) return;
   for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += gridDim.x * STEP_THREADS) {
     if (cur == 1)
       R.P[0][i] = R.P[1][i];
