@@ -707,7 +707,9 @@ int upload_grids(ps_sim* s, std::vector<SceneParams<T>>& sps) {
 // the bins are those that the triangle's box, widened by mesh_reach, covers;
 // and the point it touches lies in the triangle's plane, so bins further
 // than mesh_reach from the plane are left out (a third of the entries of a
-// slanted wall remain).
+// slanted wall remain).  The normal of a triangle without area is rounding
+// and its vertices need not lie in that "plane": such a triangle stays in
+// every bin around its box.
 template <class T>
 int upload_mesh(ps_sim* s) {
   std::vector<T> tri, aabb;
@@ -762,13 +764,19 @@ int upload_mesh(ps_sim* s) {
         const double* n = nrm.data() + 3 * gt;
         const double* v0 = s->tris[sc].data() + 9 * t;
         const double far = reach + (0.5 + 1e-3) * g.mesh_iv * (std::fabs(n[0]) + std::fabs(n[1]) + std::fabs(n[2])) + 1e-5 * size;
+        double off = 0.0;  // of its vertices from the plane (not a number for a triangle without a normal)
+        for (int k = 3; k < 9; k += 3) {
+          const double d = std::fabs(n[0] * (v0[k] - v0[0]) + n[1] * (v0[k + 1] - v0[1]) + n[2] * (v0[k + 2] - v0[2]));
+          if (!(d <= off)) off = d;
+        }
+        const bool flat = off <= 1e-6 * size;  // it is flat and its normal is good
         for (int32_t x = b0[0]; x <= b1[0]; ++x)
           for (int32_t y = b0[1]; y <= b1[1]; ++y)
             for (int32_t z = b0[2]; z <= b1[2]; ++z) {
               const double h = n[0] * (g.mesh_lo[0] + (x + 0.5) * g.mesh_iv - v0[0]) +
                                n[1] * (g.mesh_lo[1] + (y + 0.5) * g.mesh_iv - v0[1]) +
                                n[2] * (g.mesh_lo[2] + (z + 0.5) * g.mesh_iv - v0[2]);
-              if (std::fabs(h) > far) continue;  // (a triangle without a normal stays)
+              if (flat && std::fabs(h) > far) continue;
               const int64_t bin = g.bin_base + ((int64_t)x * g.mesh_nb[1] + y) * g.mesh_nb[2] + z;
               if (pass == 0)
                 bin_offset[bin + 1] += 1;

@@ -262,8 +262,11 @@ __device__ __forceinline__ uint32_t mesh_candidates(const vec4_t<T>& P, T skin, 
                [&](uint32_t t) {
                  if (n > CAP || !in_box<T>(mv, t, lo, hi)) return;
                  const Triangle<T> g = triangle<T>(mv, t);
+                 const V3<T> ab = v3sub(g.b, g.a), ac = v3sub(g.c, g.a);
                  const T h = (P.x - g.a.x) * g.n.x + (P.y - g.a.y) * g.n.y + (P.z - g.a.z) * g.n.z;
-                 if (fabs(h) > along) return;  // (a triangle without a normal stays)
+                 // vertices off the plane: the normal of a triangle without area is rounding
+                 const T off = fabs(v3dot(ab, g.n)) + fabs(v3dot(ac, g.n));
+                 if (fabs(h) > along + off) return;  // (a triangle without a normal stays)
                  uint32_t k = n;  // several bins: not in order, and not once
                  while (k > 0u && ids[k - 1] > t) --k;
                  if (k > 0u && ids[k - 1] == t) return;

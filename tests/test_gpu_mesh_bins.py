@@ -47,3 +47,38 @@ def test_coarse_and_fine_triangles(need_gpu, prec, n):
         sim.step(25)
         got = sim.get_state()
     assert same(got, O.run(sc, 25, prec), prec)
+
+
+def flat_triangles_scene(seed: int, kind: str, n: int = 200, length: float = 0.12) -> scenes.Scene:
+    """Triangles without area among a box's, and a small sphere on each."""
+    rng = np.random.default_rng(seed)
+    a = rng.uniform(-0.04, 0.04, (n, 3)) + (0.0, 0.0, 0.12)
+    d = rng.normal(size=(n, 3))
+    d *= length / 2 / np.linalg.norm(d, axis=1)[:, None]
+    a -= d / 2
+    third = {"collinear": a + 0.37 * d, "two equal corners": a, "sliver": a + 0.37 * d + rng.normal(0, 1e-12, (n, 3))}[kind]
+    off = rng.normal(size=(n, 3))
+    off *= 0.001 / np.linalg.norm(off, axis=1)[:, None]
+    base = scenes.box_mesh_scene()
+    st = np.zeros((n, 8))
+    st[:, :3] = a + rng.uniform(0.0, 1.0, n)[:, None] * d + off
+    st[:, 3:6] = rng.normal(0, 0.05, (n, 3))
+    st[:, 6] = 0.002
+    st[:, 7] = scenes.mass_of(st[:, 6], 1000.0)
+    return base.copy(state=st, tri=np.concatenate([base.tri, np.concatenate([a, a + d, third], axis=1)]), k_spring=1e-6,
+                     dt=1e-6)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("kind", ["collinear", "two equal corners", "sliver"])
+@pytest.mark.parametrize("steps,skin", [(1, 0.0), (12, 0.0), (12, 0.2)])
+def test_triangles_without_area(need_gpu, kind, steps, skin, prec):
+    # their normals are rounding, or not numbers, but their edges are touched all the same
+    sc = flat_triangles_scene(3, kind)
+    with psb200.Simulation(sc, prec) as sim:
+        sim.set_state()
+        sim.set_neighbor_lists(skin, 64)
+        sim.step(steps)
+        got = sim.get_state()
+    want = O.run(sc, steps, prec)
+    assert np.array_equal(got.astype(want.dtype), want, equal_nan=True)
