@@ -159,7 +159,7 @@ struct ps_sim {
   void* fwd_arena = nullptr;
   size_t fwd_bytes = 0;
   void* adj_arena = nullptr;              // tape, adjoint arrays, partials
-  int record_skip = 0;                    // backward passes left that do not record runs
+  int64_t fwd_lists_from = -1;            // blocks from here on are reversed on lists (-1: no backward pass yet)
   size_t adj_bytes = 0;
   // neighbour-list mode (ps_set_neighbor_lists); off when list_skin <= 0
   double list_skin = 0.0;                 // skin as a fraction of the cell edge
@@ -1233,10 +1233,12 @@ int enqueue_steps_taped(ps_sim* s, int64_t steps, char* tape, size_t row_bytes, 
 
 // Recording a block on lists: builds a block may make (its lists are kept,
 // 130 B per sphere each).  A block that needs more, or moves too fast for
-// lists, is recomputed step by step on the grid (enqueue_steps_taped).
-// After a pass with such a block the next RECORD_SKIP passes do not try.
+// lists, is recomputed step by step on the grid (enqueue_steps_taped), and so
+// are the blocks before it, which the pass comes to later.  The two orders of
+// summation differ, so the first pass after a forward pass decides
+// (fwd_lists_from) and the others repeat its choice: the same gradients bit
+// for bit, unless memory runs short between them.
 constexpr uint32_t TAPE_BUILDS = 3;
-constexpr int RECORD_SKIP = 8;
 
 // Recompute `steps` steps of a block as a recorded run; false if it gave up.
 template <class T, bool MULTI>
@@ -1289,8 +1291,10 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
   // the second only when a block needs them.
   const size_t offs_stride = align_up(sizeof(uint32_t) * (size_t)n_scan(s), 256) / sizeof(uint32_t);
   const size_t offs_b = sizeof(uint32_t) * offs_stride * (size_t)K;
-  bool record = s->run_arena != nullptr && !s->run_off && K >= RUN_MIN_STEPS && s->record_skip == 0;
-  if (s->record_skip > 0) --s->record_skip;
+  const int64_t n_blocks = (s->fwd_steps + K - 1) / K;
+  const bool known = s->fwd_lists_from >= 0;
+  int64_t lists_from = known ? s->fwd_lists_from : 0;
+  bool record = s->run_arena != nullptr && !s->run_off && K >= RUN_MIN_STEPS && lists_from < n_blocks;
   const size_t base = tape_b + 4 * adj_b + inv_b + acc_b + io_b + red_b;
   auto reserve = [&](size_t need) -> cudaError_t {
     if (s->adj_bytes >= need) return cudaSuccess;
@@ -1301,12 +1305,15 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
     if (e == cudaSuccess) s->adj_bytes = need;
     return e;
   };
-  if (record && reserve(base + lists_b) != cudaSuccess) {
+  if (record && reserve(base + (lists_from > 0 ? std::max(lists_b, offs_b) : lists_b)) != cudaSuccess) {
     cudaGetLastError();
     record = false;
   }
   record = record && s->run_arena != nullptr;  // (the allocation may have taken the lists' memory)
-  if (!record) PS_CUDA(reserve(base + offs_b));
+  if (!record) {
+    lists_from = n_blocks;
+    PS_CUDA(reserve(base + offs_b));
+  }
   cudaStream_t st = s->stream;
   const unsigned gp = blocks_for(n);
   unsigned adj_grid = 0;  // one wave of k_adj_contacts, which loops over the particles
@@ -1340,26 +1347,31 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
   PS_CUDA(cudaMemcpyAsync(io, dl_dstate, 6 * sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, st));
   PS_CUDA(cudaMemsetAsync(a.acc, 0, acc_b, st));
   const SceneParams<T> sp0 = params<T>(s)[0];
-  const int64_t n_blocks = (s->fwd_steps + K - 1) / K;
   std::vector<uint32_t> build;
   for (int64_t blk = n_blocks - 1; blk >= 0; --blk) {
     const int64_t kb = std::min(K, s->fwd_steps - blk * K);
     // recompute the block, recording each step's input and pairs (row 0 = block start)
     bool on_lists = false;
-    for (int attempt = record ? 0 : 1; attempt < 2 && !on_lists; ++attempt) {
+    for (int attempt = blk >= lists_from ? 0 : 1; attempt < 2 && !on_lists; ++attempt) {
       int rc = load_state(s, s->fwd_ckpt[(size_t)blk]);
       if (rc != PS_OK) return rc;
       k_tape_write<T><<<gp, STEP_THREADS, 0, st>>>(bufs<T>(s), tape_row<T>(tape, row_b, n, 0));
       if (attempt == 0) {
         rc = record_run<T, MULTI>(s, kb, tape, row_b, lists, build, on_lists);
       } else {
-        if (record && offs_own == nullptr && s->adj_bytes < base + offs_b) {
-          PS_CUDA(dev_alloc(s, &offs_own, offs_b));
+        if (blk >= lists_from) lists_from = blk + 1;
+        if (offs_own == nullptr && s->adj_bytes < base + offs_b) {
+          if (dev_alloc(s, &offs_own, offs_b) != cudaSuccess) {  // room for one of the two only
+            cudaGetLastError();
+            cudaFree(s->adj_arena);
+            s->adj_arena = nullptr;
+            s->adj_bytes = 0;
+            s->fwd_lists_from = n_blocks;
+            return backward_impl<T, MULTI>(s, dl_dstate, grads, dl_dstate0);
+          }
           offs = static_cast<uint32_t*>(offs_own);
         }
         rc = enqueue_steps_taped<T, MULTI>(s, kb, tape, row_b, offs, offs_stride);
-        if (record) s->record_skip = RECORD_SKIP;
-        record = record && s->run_arena != nullptr;
       }
       if (rc != PS_OK) return rc;
       PS_CUDA(cudaGetLastError());
@@ -1406,6 +1418,7 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
     }
     PS_CUDA(cudaGetLastError());
   }
+  if (!known) s->fwd_lists_from = lists_from;
   double* share_sums = red + align_up(sizeof(double) * n_sums, 256) / sizeof(double);
   for (int s0 = 0; s0 < s->n_scenes; s0 += 65535)
     k_adj_reduce<<<dim3((unsigned)shares, ADJ_NACC, (unsigned)std::min(65535, s->n_scenes - s0)), ADJ_REDUCE_THREADS, 0,
@@ -2150,8 +2163,9 @@ extern "C" int ps_forward_checkpointed(ps_sim* s, int64_t n_steps, int64_t every
   const int64_t n_blocks = (n_steps + every - 1) / every;
   const size_t ckpt_b = align_up(2 * state_bytes(s) + 4 * (size_t)s->n_total, 256);
   const size_t need = std::max<size_t>(ckpt_b * (size_t)(n_blocks + 1), 256);
+  s->fwd_steps = 0;  // (until the pass is complete)
+  s->fwd_lists_from = -1;
   if (s->fwd_bytes < need || s->fwd_bytes / 2 > need) {  // (a much shorter pass gives the rest back)
-    s->fwd_steps = 0;
     cudaFree(s->fwd_arena);
     s->fwd_arena = nullptr;
     s->fwd_bytes = 0;
