@@ -111,7 +111,9 @@ int32_t ps_bounds_checked(void);
 int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t precision, int32_t device, ps_sim** out);
 
 /* Upload host state, scenes concatenated in order (replaces the H2D copy
- * of ParticleModelCUDA.cpp:36-43).  Also sizes the grids on first call. */
+ * of ParticleModelCUDA.cpp:36-43).  Also sizes the grids on first call.  Radii
+ * must not be negative and masses must be positive in every call, and in later
+ * calls 2 r must not exceed the scene's cell edge (PS_ERR_INVALID). */
 int ps_set_state(ps_sim* sim, const double* aos, int64_t n_total);
 
 /* Download state in original particle order (ParticleModelCUDA::getParticles,

@@ -490,8 +490,10 @@ int check_device_error(ps_sim* s) {
 
 // ---- conversion kernels between the host AoS and the device SoA ------------
 // Upload check of a new state against the grid sized by the first upload:
-// each particle must fit a cell (2 r <= cell edge of its scene) and have a
-// positive mass; the lowest failing index is kept in *bad (NaN fails too).
+// each particle must fit a cell (2 r <= cell edge of its scene), its radius
+// must not be negative (a run uses the sign of a radius as a mark) and its
+// mass must be positive, as in the first one; the lowest failing index is kept
+// in *bad (NaN fails too).
 __global__ void k_upload_check(const double* __restrict__ aos, const uint32_t* __restrict__ pbase, int n_scenes,
                                const double* __restrict__ interval, uint32_t* bad, uint32_t n) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -505,7 +507,7 @@ __global__ void k_upload_check(const double* __restrict__ aos, const uint32_t* _
       hi = mid - 1;
   }
   const double r = aos[8 * (size_t)p + 6], m = aos[8 * (size_t)p + 7];
-  if (!(2.0 * r <= interval[lo]) || !(m > 0.0)) atomicMin(bad, p);
+  if (!(r >= 0.0) || !(2.0 * r <= interval[lo]) || !(m > 0.0)) atomicMin(bad, p);
 }
 
 template <class T>
@@ -1569,7 +1571,7 @@ extern "C" int ps_set_state(ps_sim* s, const double* aos, int64_t n_total) {
     PS_CUDA(cudaStreamSynchronize(s->stream));
     if (h_bad != 0xffffffffu)
       return fail(PS_ERR_INVALID,
-                  "ps_set_state: particle " + std::to_string(h_bad) + " does not fit the grid sized by the first upload");
+                  "ps_set_state: particle " + std::to_string(h_bad) + " does not fit the grid sized by the first upload, or has a negative radius or a non-positive mass");
   }
   if (s->precision == PS_FP32)
     k_upload<float><<<g, STEP_THREADS, 0, s->stream>>>(s->staging, static_cast<float4*>(s->P0),

@@ -69,3 +69,22 @@ def test_backward_passes_of_one_forward_pass_are_equal(need_gpu, speed, every, p
             out += [sim.backward(g) for _ in range(3)]
     for grads, g0 in out[1:]:
         assert np.array_equal(grads[0], out[0][0][0]) and np.array_equal(g0, out[0][1])
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_later_upload_with_a_negative_radius_is_refused(need_gpu, prec):
+    # as the first upload refuses it; a radius of zero stays accepted
+    sc = scenes.pile(300, seed=5, k_spring=1.0)
+    bad, zero = sc.state.copy(), sc.state.copy()
+    bad[7, 6] *= -1.0
+    zero[7, 6] = 0.0
+    with psb200.Simulation(sc, prec) as sim:
+        sim.set_state()
+        before = sim.get_state()
+        with pytest.raises(psb200.PSError, match="particle 7 .* negative radius"):
+            sim.set_state(bad)
+        assert np.array_equal(sim.get_state(), before)
+        sim.set_state(zero)
+        sim.step(30)
+        got = sim.get_state()
+    assert same(got, O.run(sc.copy(state=zero, interval=2.1 * sc.r_max()), 30, prec), prec)
