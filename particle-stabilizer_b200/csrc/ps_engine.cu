@@ -448,6 +448,12 @@ int regrid(ps_sim* s) {
 constexpr int ERR_BITS = 0, ERR_BAD = 8, ERR_RUN = 16, ERR_WORDS = 18;
 constexpr int ERR_TICKET = 24;  // blocks of k_stats that have finished (zero between launches)
 
+// Steps of a run that is to tell which path the scene calls for.  Six tell (a
+// sphere pushed out of a wall, two calm steps to the first lists, two on
+// them), and a grid step in the run takes 145 us where the step kernels take
+// 83 us (1M spheres, FP32).
+constexpr int64_t RUN_PROBE_STEPS = 6;
+
 // After a run that rebuilt so often, the next
 // RUN_BACKOFF_MIN steps (doubling up to RUN_BACKOFF_MAX while that repeats)
 // take the step kernels, which pipeline a rebuild better.
@@ -1088,7 +1094,7 @@ RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
   R.tape_build = nullptr;
   R.max_builds = 0;
   R.bar = R.bar_next = nullptr;  // (run_launch)
-  R.report = set ? R.ctl + RUN_REPORT : s->err + ERR_RUN;
+  R.report = s->err + ERR_RUN;
   return R;
 }
 
@@ -1132,13 +1138,23 @@ int run_launch(ps_sim* s, uint32_t steps, RunBufs<T> R, uint32_t run_id) {
 }
 
 template <class T>
-int run_dispatch(ps_sim* s, uint32_t steps, bool prepare, bool set = false) {
-  if (s->multi) {
-    if (s->has_mesh) return prepare ? run_prepare<T, true, true>(s) : run_launch<T, true, true, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
-    return prepare ? run_prepare<T, true, false>(s) : run_launch<T, true, false, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
-  }
-  if (s->has_mesh) return prepare ? run_prepare<T, false, true>(s) : run_launch<T, false, true, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
-  return prepare ? run_prepare<T, false, false>(s) : run_launch<T, false, false, false>(s, steps, run_bufs<T>(s, set), set ? 0u : ++s->run_id);
+int run_dispatch_prepare(ps_sim* s) {
+  if (s->multi) return s->has_mesh ? run_prepare<T, true, true>(s) : run_prepare<T, true, false>(s);
+  return s->has_mesh ? run_prepare<T, false, true>(s) : run_prepare<T, false, false>(s);
+}
+
+// A run shorter than a probe tells nothing: it always starts with a rebuild.
+template <class T>
+int run_dispatch(ps_sim* s, uint32_t steps, bool set = false) {
+  RunBufs<T> R = run_bufs<T>(s, set);
+  uint32_t id = 0;
+  if (!set && steps >= RUN_PROBE_STEPS)
+    id = ++s->run_id;
+  else
+    R.report = R.ctl + RUN_REPORT;
+  if (s->multi)
+    return s->has_mesh ? run_launch<T, true, true, false>(s, steps, R, id) : run_launch<T, true, false, false>(s, steps, R, id);
+  return s->has_mesh ? run_launch<T, false, true, false>(s, steps, R, id) : run_launch<T, false, false, false>(s, steps, R, id);
 }
 
 // ---- differentiation -----------------------------------------------------------
@@ -1664,7 +1680,7 @@ int step_graphs(ps_sim* s, int64_t n_steps) {
 }
 
 void run_alloc(ps_sim* s) {
-  const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, 0, true) : run_dispatch<double>(s, 0, true);
+  const int rc = s->precision == PS_FP32 ? run_dispatch_prepare<float>(s) : run_dispatch_prepare<double>(s);
   if (rc == PS_OK && s->run_arena == nullptr && s->run_bytes > 0) {
     size_t left = 0, total = 0;
     if (cudaMemGetInfo(&left, &total) != cudaSuccess || s->run_bytes > left / 4 ||
@@ -1697,25 +1713,23 @@ cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes) {
 // A simulation's first run is of RUN_PROBE_STEPS steps, whose report the
 // call waits for; after a backoff such a probe is followed by the step
 // kernels until a call that waits for the stream anyway has read its report.
-// What a report says only chooses the path; both give the same states.  Six
-// steps tell (a sphere pushed out of a wall, two calm steps to the first
-// lists, two on them), and a grid step in the run takes 145 us where the step
-// kernels take 83 us (1M spheres, FP32).
-constexpr int64_t RUN_PROBE_STEPS = 6;
-
+// What a report says only chooses the path; both give the same states.
+// A settled scene's steps are divided evenly among the launches they need, so
+// that none is so short that its first rebuild counts as often.
 int step_run(ps_sim* s, int64_t n_steps) {
   for (int64_t left = n_steps; left > 0;) {
     int64_t L;
     int rc;
     const bool waiting = !s->run_settled && s->run_seen != s->run_id;  // a probe is on its way
-    if (s->run_backoff > 0 || waiting) {
-      L = std::min(left, waiting ? RUN_BACKOFF_MIN : s->run_backoff);
+    if (s->run_backoff > 0 || waiting || (!s->run_settled && left < RUN_PROBE_STEPS)) {
+      L = std::min(left, s->run_backoff > 0 ? s->run_backoff : RUN_BACKOFF_MIN);
       s->run_backoff = std::max<int64_t>(0, s->run_backoff - L);
       rc = step_graphs(s, L);
       s->grid_valid = true;
     } else {
-      L = std::min(left, s->run_settled ? run_block(s) : RUN_PROBE_STEPS);
-      rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, false) : run_dispatch<double>(s, (uint32_t)L, false);
+      const int64_t launches = (left + run_block(s) - 1) / run_block(s);
+      L = s->run_settled ? (left + launches - 1) / launches : RUN_PROBE_STEPS;
+      rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L) : run_dispatch<double>(s, (uint32_t)L);
       s->grid_valid = false;  // the grid arrays are those of the last rebuild
       s->last_launches += 1;
       if (rc == PS_OK && !s->run_known && left > L) rc = check_device_error(s);
@@ -1738,7 +1752,7 @@ constexpr int64_t LIST_BACKOFF_WINDOW = 256, LIST_BACKOFF_RATE = 4, LIST_BACKOFF
 // Runs with the program's skin and capacity; returns when they are done.
 int step_lists(ps_sim* s, int64_t n_steps) {
   if (s->run_grid == 0) {
-    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, 0, true) : run_dispatch<double>(s, 0, true);
+    const int rc = s->precision == PS_FP32 ? run_dispatch_prepare<float>(s) : run_dispatch_prepare<double>(s);
     if (rc != PS_OK) return rc;
   }
   const size_t need = run_need(s, run_sms(s), (size_t)s->list_cap);
@@ -1754,8 +1768,8 @@ int step_lists(ps_sim* s, int64_t n_steps) {
   PS_CUDA(cudaMemsetAsync(ctl + RUN_FULL, 0, 2 * sizeof(uint32_t), s->stream));  // and RUN_BUILDS
   for (int64_t left = n_steps; left > 0;) {
     const int64_t L = std::min(left, run_block(s));
-    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, false, true)
-                                           : run_dispatch<double>(s, (uint32_t)L, false, true);
+    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, true)
+                                           : run_dispatch<double>(s, (uint32_t)L, true);
     if (rc != PS_OK) return rc;
     s->last_launches += 1;
     left -= L;

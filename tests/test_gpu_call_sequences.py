@@ -88,3 +88,17 @@ def test_later_upload_with_a_negative_radius_is_refused(need_gpu, prec):
         sim.step(30)
         got = sim.get_state()
     assert same(got, O.run(sc.copy(state=zero, interval=2.1 * sc.r_max()), 30, prec), prec)
+
+
+@pytest.mark.parametrize("steps", [513, 1025])
+def test_calls_a_little_longer_than_a_launch_stay_settled(need_gpu, steps):
+    # a calm scene: as many launches as the steps need, in every call
+    want = -(-steps // 512)
+    with psb200.Simulation(scenes.settle_pile(side=10), "f32") as sim:
+        sim.set_state()
+        sim.step(60)
+        sim.sync()
+        for _ in range(5):
+            sim.step(steps)
+            assert sim.launches() == want
+            sim.sync()
