@@ -130,7 +130,9 @@ int ps_get_state(ps_sim* sim, double* aos_out, int64_t n_total);
  * memory, and scenes that move too fast for lists to last run as CUDA graphs
  * of the step kernels, which rebuild the grid in every step.  All give the
  * same states bit for bit.  The first such call on a simulation's grid waits
- * for its first six steps, to see which of the two the scene calls for. */
+ * for its first six steps, to see which of the two the scene calls for, and
+ * every call waits for all launches of many steps but its last one, to see
+ * whether the scene still does. */
 int ps_step(ps_sim* sim, int64_t n_steps);
 
 /* Wait for the stream and check the device error word. */

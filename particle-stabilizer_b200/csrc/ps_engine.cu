@@ -183,7 +183,6 @@ struct ps_sim {
   uint32_t run_turn = 0, list_turn = 0;   // launches on the control words of run_arena and of list_arena
   uint32_t run_id = 0, run_seen = 0;      // runs launched, and the last one whose report was read (run_read)
   bool run_settled = false;               // what that report said
-  bool run_known = false;                 // a run was launched on this grid
   int64_t run_backoff = 0, run_backoff_len = 0;  // steps left to the step kernels after an unsettled run
 };
 
@@ -1710,9 +1709,11 @@ cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes) {
   return e;
 }
 
-// A simulation's first run is of RUN_PROBE_STEPS steps, whose report the
-// call waits for; after a backoff such a probe is followed by the step
-// kernels until a call that waits for the stream anyway has read its report.
+// A simulation's first run, and the first one after a backoff, is of
+// RUN_PROBE_STEPS steps.  A call that has steps left waits for each run's
+// report, so that a scene that turns fast or calm inside a long call changes
+// its path there.  The last run's report is read by a call that waits for the
+// stream anyway; until then an unsettled scene stays on the step kernels.
 // What a report says only chooses the path; both give the same states.
 // A settled scene's steps are divided evenly among the launches they need, so
 // that none is so short that its first rebuild counts as often.
@@ -1732,8 +1733,7 @@ int step_run(ps_sim* s, int64_t n_steps) {
       rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L) : run_dispatch<double>(s, (uint32_t)L);
       s->grid_valid = false;  // the grid arrays are those of the last rebuild
       s->last_launches += 1;
-      if (rc == PS_OK && !s->run_known && left > L) rc = check_device_error(s);
-      s->run_known = true;
+      if (rc == PS_OK && left > L) rc = check_device_error(s);
     }
     if (rc != PS_OK) return rc;
     left -= L;
@@ -1930,7 +1930,7 @@ int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   s->adj_bytes = 0;
   s->run_grid = 0;
   s->run_seen = s->run_id;
-  s->run_settled = s->run_known = false;
+  s->run_settled = false;
   s->fwd_steps = 0;
   s->l2_window_on = s->l2_window_tried = false;
   s->grid_sized = false;

@@ -102,3 +102,29 @@ def test_calls_a_little_longer_than_a_launch_stay_settled(need_gpu, steps):
             sim.step(steps)
             assert sim.launches() == want
             sim.sync()
+
+
+def turns_fast() -> scenes.Scene:
+    """A pile in free fall under a strong gravity, calm for 600 steps and too
+    fast for lists after them."""
+    sc = scenes.pile(1000, seed=26, k_spring=1.0)
+    st = sc.state.copy()
+    st[:, 3:6] *= 0.1
+    st[:, 2] += 2.0
+    return sc.copy(state=st, box_max=(*sc.box_max[:2], 3.0), gravity=(0.0, 0.0, -1e4))
+
+
+@pytest.mark.parametrize("make,steps,lo,hi", [(turns_fast, 1800, 1000, 7000), (lambda: calms_down(1.0), 5000, 1024, 7000)],
+                         ids=["turns fast", "calms down"])
+def test_a_long_call_changes_its_path_inside(need_gpu, make, steps, lo, hi):
+    # one call; the step kernels take four launches a step, runs next to none
+    out = []
+    for name in ("step", "profile_steps"):
+        with psb200.Simulation(make(), "f32") as sim:
+            sim.set_state()
+            getattr(sim, name)(steps)
+            launches = sim.launches()
+            out.append(sim.get_state())
+        if name == "step":
+            assert lo < launches < hi
+    assert np.array_equal(out[0], out[1])
