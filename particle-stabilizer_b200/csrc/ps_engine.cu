@@ -480,9 +480,8 @@ int check_device_error(ps_sim* s) {
     if (e & PS_DEVERR_BOUNDS) m += " index out of bounds (bounds-checked build; the access was skipped);";
     if (e & PS_DEVERR_LIST_BARRIER) {
       m += " grid barrier wait expired;";
-      // a run left in the middle: its counts and control words
-      cudaMemsetAsync(s->count, 0, sizeof(uint32_t) * (size_t)n_scan(s), s->stream);
-      cudaMemsetAsync(s->tile_sum, 0, sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), s->stream);
+      // the control words of a run left in the middle
+      if (s->list_arena != nullptr) cudaMemsetAsync(s->list_arena, 0, 256, s->stream);
       if (s->run_arena != nullptr) cudaMemsetAsync(s->run_arena, 0, 256, s->stream);
     }
     uint32_t zero = 0;
@@ -1462,6 +1461,18 @@ int backward_impl(ps_sim* s, const double* dl_dstate, ps_grad* grads, double* dl
 }  // namespace
 
 // ---- C ABI -------------------------------------------------------------------
+#ifdef PS_DEBUG_BOUNDS
+// Sets bits of the device error word, as a kernel of the simulation would: for
+// tests of what is queued behind one that failed.  Not in the product library.
+extern "C" int ps_debug_set_error(ps_sim* s, uint32_t bits) {
+  if (s == nullptr) return fail(PS_ERR_INVALID, "ps_debug_set_error: null simulation");
+  DeviceGuard guard(s->device);
+  PS_CUDA(cudaMemcpyAsync(s->err, &bits, sizeof(bits), cudaMemcpyHostToDevice, s->stream));
+  PS_CUDA(cudaStreamSynchronize(s->stream));
+  return PS_OK;
+}
+#endif
+
 extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t precision, int32_t device,
                          ps_sim** out) {
   if (out == nullptr || scenes == nullptr || n_scenes <= 0)
@@ -1779,12 +1790,7 @@ int step_lists(ps_sim* s, int64_t n_steps) {
   static_assert(RUN_BUILDS == RUN_FULL + 1, "read together");
   PS_CUDA(cudaMemcpyAsync(told, ctl + RUN_FULL, sizeof(told), cudaMemcpyDeviceToHost, s->stream));
   const int rc = check_device_error(s);  // waits for the stream
-  if (rc != PS_OK) {
-    cudaFree(s->list_arena);  // with what a run left in its control words
-    s->list_arena = nullptr;
-    s->list_bytes = 0;
-    return rc;
-  }
+  if (rc != PS_OK) return rc;
   s->list_fallbacks += told[0] != 0u;
   s->list_rebuilds += told[1];
   s->list_win_steps += n_steps;

@@ -80,6 +80,7 @@ enum : int {
   RUN_BUILDS = 9,   // builds after a run's first
   RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
   RUN_BAR_ODD = 12, // grid barrier of odd launches
+  RUN_LEFT = 14,    // CTAs that left because a barrier gave up
 };
 
 template <class T>
@@ -122,8 +123,11 @@ struct RunBufs {
 // however that ended: two words take turns, and a launch clears the other one.
 // Every wait is bounded: a CTA that gives up records PS_DEVERR_LIST_BARRIER
 // and leaves the kernel, and no later barrier can then complete.  The limit
-// is seconds, because one phase of a diverged scene (spheres crowded into one
-// cell) may take long.
+// is about a minute, because one phase of a diverged scene (spheres crowded
+// into one cell) may take long.  What was queued behind such a launch stays
+// inside its arrays: later runs see the bit and return at once, and the last
+// CTA to leave clears the counts that the step kernels start from (run_leave).
+// The host clears the bit and the control words with its report.
 constexpr uint32_t RUN_BARRIER_SPIN_LIMIT = 1u << 26;
 
 __device__ __forceinline__ bool run_barrier(uint32_t* word, uint32_t* err) {
@@ -151,6 +155,21 @@ __device__ __forceinline__ bool run_barrier(uint32_t* word, uint32_t* err) {
   }
   __syncthreads();
   return s_ok != 0;
+}
+
+template <class T>
+__device__ __noinline__ void run_leave(const StepBufs<T>& b, uint32_t* ctl) {
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ctl + RUN_LEFT, 1u) + 1u == gridDim.x;
+  }
+  __syncthreads();
+  if (!s_last) return;  // (a CTA that passed the last barrier has no counts to clear)
+  __threadfence();
+  for (uint32_t c = threadIdx.x; c < b.n_scan; c += STEP_THREADS) b.count[c] = 0u;
+  for (uint32_t t = threadIdx.x; t < b.n_tiles; t += STEP_THREADS) b.tile_sum[t] = 0u;
 }
 
 template <class T>
@@ -899,6 +918,8 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
           uint32_t move_blocks, uint32_t run_id) {
   uint32_t* maxd = R.ctl + RUN_MAXD;
   if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.bar_next) = 0ull;
+  // (set by an earlier launch: of this one, no CTA gives up before the others have read it)
+  if (*reinterpret_cast<volatile uint32_t*>(b.err) & PS_DEVERR_LIST_BARRIER) return;
   uint32_t streak = *reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_STREAK);
   run_begin<T, MULTI, MESH>(b, sp0, mv, R);
   int cur = 1;           // buffer with the state before the step's contacts
@@ -912,7 +933,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   if (!(before > 0.0f) || TAPE) before = INFINITY;
   RunOwn<T> own;
   for (uint32_t s = 0; s < steps; ++s) {
-    if (!run_barrier(R.bar, b.err)) return;
+    if (!run_barrier(R.bar, b.err)) return run_leave(b, R.ctl);
     const float m = sqrtf(__uint_as_float(*reinterpret_cast<volatile uint32_t*>(maxd + s % 3u)));
     if (blockIdx.x == 0 && threadIdx.x == 0) maxd[(s + 2u) % 3u] = 0u;
     streak = m <= RUN_CALM_MAX ? (streak < RUN_CALM_STEPS ? streak + 1u : streak) : 0u;
@@ -934,7 +955,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
       frac = fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest);
       frac = R.skin > 0.0f ? R.skin : (lists ? frac : 0.0f);
       if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, n_cells, scatter_blocks, move_blocks))
-        return;
+        return run_leave(b, R.ctl);
       cur = 1 - cur;
       D = 0.0f;
       fresh = true;
@@ -953,7 +974,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     cur = 1 - cur;
   }
   // the state is in buffer `cur`; at rest the positions are in P0 and the velocities in V1
-  if (!run_barrier(R.bar, b.err)) return;
+  if (!run_barrier(R.bar, b.err)) return run_leave(b, R.ctl);
   for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += gridDim.x * STEP_THREADS) {
     if (cur == 1)
       R.P[0][i] = R.P[1][i];

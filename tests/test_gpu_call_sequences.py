@@ -2,12 +2,17 @@
 earlier ones left on the device: grids resized between runs, and the like.
 States are compared bit for bit with the oracle or with the step kernels,
 which ps_profile_steps always takes."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import psb200
 from psb200 import scenes
 from oracle import ps_oracle as O
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +133,54 @@ def test_a_long_call_changes_its_path_inside(need_gpu, make, steps, lo, hi):
         if name == "step":
             assert lo < launches < hi
     assert np.array_equal(out[0], out[1])
+
+
+AFTER_A_BARRIER_GAVE_UP = r"""
+import sys
+import numpy as np
+import psb200
+from psb200 import scenes
+
+psb200.LIB_PATH = psb200.DEBUG_LIB_PATH
+BARRIER = 1 << 4  # PS_DEVERR_LIST_BARRIER, which such a kernel leaves in the error word
+sc = scenes.settle_pile(side=8)
+
+
+def run(skin, preset):
+    with psb200.Simulation(sc, "f32") as sim:
+        sim.set_state()
+        sim.set_neighbor_lists(skin, 48)
+        sim.step(60)
+        sim.sync()
+        before = sim.get_state()
+        if preset:
+            assert psb200.lib().ps_debug_set_error(sim.h, BARRIER) == 0
+            for call in (lambda: sim.step(64), sim.sync):  # (lists: the step itself waits)
+                try:
+                    call()
+                except psb200.PSError as e:
+                    assert "grid barrier wait expired" in str(e)
+                    break
+            else:
+                raise AssertionError("no error reported")
+            assert np.array_equal(sim.get_state(), before), "the run did not return at once"
+        sim.step(64)
+        sim.step(5)
+        return sim.get_state()
+
+
+for skin in (0.0, 0.1):
+    assert np.array_equal(run(skin, True), run(skin, False))
+print("DONE", flush=True)
+"""
+
+
+def test_runs_behind_one_whose_barrier_gave_up_return_at_once(need_gpu):
+    # the bit is set by the test, in the bounds-checked build; no kernel waits
+    assert os.path.exists(psb200.DEBUG_LIB_PATH)
+    env = dict(os.environ)
+    env["PYTHONPATH"] = os.pathsep.join([ROOT, os.path.join(ROOT, "particle-stabilizer_b200", "python"),
+                                         env.get("PYTHONPATH", "")])
+    r = subprocess.run([sys.executable, "-c", AFTER_A_BARRIER_GAVE_UP], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.rstrip().endswith("DONE"), r.stdout[-3000:] + r.stderr[-3000:]
