@@ -1755,55 +1755,69 @@ int step_run(ps_sim* s, int64_t n_steps) {
 // A rebuild costs a few list steps; when a window of at least
 // LIST_BACKOFF_WINDOW list steps rebuilt more often than once per
 // LIST_BACKOFF_RATE steps (a scene moving fast against its skin, or
-// diverging), the following steps run on the grid path, for a stretch that
-// doubles while this repeats.
+// diverging, or too many spheres with more neighbours than a list holds), the
+// following steps run on the grid path, for a stretch that doubles while this
+// repeats.
 constexpr int64_t LIST_BACKOFF_WINDOW = 256, LIST_BACKOFF_RATE = 4, LIST_BACKOFF_MIN = 1024,
                   LIST_BACKOFF_MAX = 65536;
 
-// Runs with the program's skin and capacity; returns when they are done.
+// A call's steps with the program's skin and capacity, or on the grid path
+// while the backoff lasts.  Each run is waited for, so that a long call
+// changes its path as soon as its runs call for it.
 int step_lists(ps_sim* s, int64_t n_steps) {
   if (s->run_grid == 0) {
     const int rc = s->precision == PS_FP32 ? run_dispatch_prepare<float>(s) : run_dispatch_prepare<double>(s);
     if (rc != PS_OK) return rc;
   }
-  const size_t need = run_need(s, run_sms(s), (size_t)s->list_cap);
-  if (s->list_arena == nullptr || s->list_bytes < need) {
-    cudaFree(s->list_arena);
-    s->list_arena = nullptr;
-    s->list_bytes = 0;
-    PS_CUDA(dev_alloc(s, &s->list_arena, need));
-    s->list_bytes = need;
-    PS_CUDA(cudaMemsetAsync(s->list_arena, 0, 256, s->stream));
-  }
-  uint32_t* ctl = static_cast<uint32_t*>(s->list_arena);
-  PS_CUDA(cudaMemsetAsync(ctl + RUN_FULL, 0, 2 * sizeof(uint32_t), s->stream));  // and RUN_BUILDS
+  bool full = false;  // a list was too short in this call
   for (int64_t left = n_steps; left > 0;) {
+    if (s->list_backoff > 0) {
+      const int64_t L = std::min(left, s->list_backoff);
+      const int rc = step_graphs(s, L);
+      if (rc != PS_OK) return rc;
+      s->grid_valid = true;
+      s->list_backoff -= L;
+      s->list_grid_steps += L;
+      left -= L;
+      continue;
+    }
+    const size_t need = run_need(s, run_sms(s), (size_t)s->list_cap);
+    if (s->list_arena == nullptr || s->list_bytes < need) {
+      cudaFree(s->list_arena);
+      s->list_arena = nullptr;
+      s->list_bytes = 0;
+      PS_CUDA(dev_alloc(s, &s->list_arena, need));
+      s->list_bytes = need;
+      PS_CUDA(cudaMemsetAsync(s->list_arena, 0, 256, s->stream));
+    }
+    uint32_t* ctl = static_cast<uint32_t*>(s->list_arena);
+    PS_CUDA(cudaMemsetAsync(ctl + RUN_FULL, 0, 2 * sizeof(uint32_t), s->stream));  // and RUN_BUILDS
     const int64_t L = std::min(left, run_block(s));
-    const int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, true)
-                                           : run_dispatch<double>(s, (uint32_t)L, true);
+    int rc = s->precision == PS_FP32 ? run_dispatch<float>(s, (uint32_t)L, true) : run_dispatch<double>(s, (uint32_t)L, true);
     if (rc != PS_OK) return rc;
     s->last_launches += 1;
+    s->grid_valid = false;  // the grid arrays are those of the last rebuild
     left -= L;
-  }
-  s->grid_valid = false;  // the grid arrays are those of the last rebuild
-  uint32_t told[2] = {};
-  static_assert(RUN_BUILDS == RUN_FULL + 1, "read together");
-  PS_CUDA(cudaMemcpyAsync(told, ctl + RUN_FULL, sizeof(told), cudaMemcpyDeviceToHost, s->stream));
-  const int rc = check_device_error(s);  // waits for the stream
-  if (rc != PS_OK) return rc;
-  s->list_fallbacks += told[0] != 0u;
-  s->list_rebuilds += told[1];
-  s->list_win_steps += n_steps;
-  s->list_win_rebuilds += told[1];
-  if (s->list_win_steps >= LIST_BACKOFF_WINDOW) {
-    if (s->list_win_rebuilds * LIST_BACKOFF_RATE > s->list_win_steps) {
-      s->list_backoff_len = std::min<int64_t>(std::max<int64_t>(2 * s->list_backoff_len, LIST_BACKOFF_MIN),
-                                              LIST_BACKOFF_MAX);
-      s->list_backoff = s->list_backoff_len;
-    } else {
-      s->list_backoff_len = 0;
+    uint32_t told[2] = {};
+    static_assert(RUN_BUILDS == RUN_FULL + 1, "read together");
+    PS_CUDA(cudaMemcpyAsync(told, ctl + RUN_FULL, sizeof(told), cudaMemcpyDeviceToHost, s->stream));
+    rc = check_device_error(s);  // waits for the stream
+    if (rc != PS_OK) return rc;
+    if (told[0] != 0u && !full) ++s->list_fallbacks;
+    full |= told[0] != 0u;
+    s->list_rebuilds += told[1];
+    s->list_win_steps += L;
+    s->list_win_rebuilds += told[1];
+    if (s->list_win_steps >= LIST_BACKOFF_WINDOW) {
+      if (s->list_win_rebuilds * LIST_BACKOFF_RATE > s->list_win_steps) {
+        s->list_backoff_len = std::min<int64_t>(std::max<int64_t>(2 * s->list_backoff_len, LIST_BACKOFF_MIN),
+                                                LIST_BACKOFF_MAX);
+        s->list_backoff = s->list_backoff_len;
+      } else {
+        s->list_backoff_len = 0;
+      }
+      s->list_win_steps = s->list_win_rebuilds = 0;
     }
-    s->list_win_steps = s->list_win_rebuilds = 0;
   }
   return PS_OK;
 }
@@ -1847,20 +1861,13 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
   DeviceGuard guard(s->device);
   const bool lists = s->list_skin > 0.0;
   int rc = PS_OK;
-  int64_t left = n_steps;
-  if (lists && s->list_backoff > 0) {
-    const int64_t g = std::min(left, s->list_backoff);
-    rc = step_graphs(s, g);
+  if (lists) {
+    rc = step_lists(s, n_steps);
+  } else if (n_steps >= RUN_MIN_STEPS && s->run_arena != nullptr && !s->run_off) {
+    rc = step_run(s, n_steps);
+  } else {
+    rc = step_graphs(s, n_steps);
     s->grid_valid = true;
-    s->list_backoff -= g;
-    s->list_grid_steps += g;
-    left -= g;
-  }
-  if (!lists && left >= RUN_MIN_STEPS && s->run_arena != nullptr && !s->run_off) {
-    rc = step_run(s, left);
-  } else if (rc == PS_OK && left > 0) {
-    rc = lists ? step_lists(s, left) : step_graphs(s, left);
-    if (!lists) s->grid_valid = true;
   }
   if (rc != PS_OK) return rc;
   s->stepped = true;

@@ -26,7 +26,8 @@
 //     the build can leave it; a bit of its count word says so, and the other
 //     spheres do not compute a cell at all.
 //   * A sphere with more than the list's capacity of neighbours walks the
-//     cells of the last build instead (run_slow).
+//     cells of the last build instead (run_slow); where such spheres are too
+//     many for that, the launch goes on without lists (RUN_CROWD).
 //   * In a triangle container a build also lists the triangles that a sphere
 //     may come to touch; one that moves a good part of the skin at once walks
 //     its bin.
@@ -81,6 +82,7 @@ enum : int {
   RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
   RUN_BAR_ODD = 12, // grid barrier of odd launches
   RUN_LEFT = 14,    // CTAs that left because a barrier gave up
+  RUN_CROWD = 16,   // what the spheres beyond their lists cost (64 bits), of the last build
 };
 
 template <class T>
@@ -292,6 +294,7 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
   const vec4_t<T> P = Ps[i];
   const T skin = frac * sp.interval;
   uint32_t k = 0, word = 0;
+  uint32_t cand = 0, trips = 0;  // candidates, and the trips of a warp that goes through them column by column
   if (isfinite(P.x) && isfinite(P.y) && isfinite(P.z)) {
     int32_t cx, cy, cz;
     cell_coords<T>(b.scell[i], sp, cx, cy, cz);
@@ -328,6 +331,8 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
           lo[q] = ok ? b.offset[col + (uint32_t)s.z0] : 0u;
           hi[q] = ok ? b.offset[col + (uint32_t)s.z1 + 1u] : 0u;
           if (!in_bounds(hi[q], (uint64_t)b.n + 1u, b.err)) hi[q] = lo[q] = 0u;
+          cand += hi[q] - lo[q];
+          trips += (hi[q] - lo[q] + 31u) / 32u;
         }
 #pragma unroll
         for (int q = 0; q < COLS; ++q)
@@ -358,6 +363,8 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
     }
   }
   if (k > R.cap) {
+    // passes of run_slow times their trips, per trip that 32 lanes' own walks take
+    atomicAdd(reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD), (1ull + k / 32u) * trips * 32u / max(cand, 1u));
     word |= RUN_OVERFLOW, k = 0;
     R.ctl[RUN_FULL] = 1u;
   }
@@ -371,8 +378,12 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
 // The lanes take the list's entries side by side (`mine`), each forms its
 // pair's key and force, and the forces are added in the order of the keys.
 // A list of more than an entry per lane, and the cells of the last build in
-// place of a list that overflowed, are gone through for the smallest key
-// above the last one in turn.
+// place of a list that overflowed, are gone through once for every 32 pairs in
+// contact: a pass keeps the 32 smallest keys above the last one, ordered by
+// lane.  (A pass for every pair, as this was at first, takes the cube of the
+// spheres that touch one another: 400 on top of one another among 4,000 took
+// 3.8 ms a step, now 47 us; twenty spheres ten times as large as the 83,474
+// others 1.89 ms, now 0.28 ms.)
 template <class T>
 __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_t mine, const uint32_t* list,
                                               const StepBufs<T>& b, const SceneParams<T>& sp, const vec4_t<T>* Ps,
@@ -427,13 +438,19 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_
   const T skin = frac * sp.interval;
   const Span<T> s = reach_span<T>(P, (fabs(P.w) + T(0.5) * sp.interval + T(2) * skin) * T(1.001), sp);
   for (uint64_t from = 0;;) {
-    uint64_t best = NONE;
-    T bf = T(0), bdx = T(0), bdy = T(0), bdz = T(0);
-    auto consider = [&](uint32_t j) {
-      const uint64_t key = key_of(j);
-      if (key >= from && key < best) {
-        best = key;
-        bf = f, bdx = dx, bdy = dy, bdz = dz;
+    uint64_t kept = NONE;  // ascending by lane
+    uint32_t kept_j = i;
+    auto offer = [&](uint64_t key, uint32_t j) {
+      const uint64_t most = __shfl_sync(0xffffffffu, kept, 31);
+      for (uint32_t who = __ballot_sync(0xffffffffu, key >= from && key < most); who != 0u; who &= who - 1u) {
+        const int l = __ffs(who) - 1;
+        const uint64_t k = __shfl_sync(0xffffffffu, key, l), below = __shfl_up_sync(0xffffffffu, kept, 1);
+        const uint32_t kj = __shfl_sync(0xffffffffu, j, l), below_j = __shfl_up_sync(0xffffffffu, kept_j, 1);
+        if (kept > k) {
+          const bool here = lane == 0u || below < k;
+          kept = here ? k : below;
+          kept_j = here ? kj : below_j;
+        }
       }
     };
     if (word & RUN_OVERFLOW) {
@@ -442,20 +459,22 @@ __device__ __forceinline__ vec4_t<T> run_slow(uint32_t i, uint32_t word, uint32_
           const uint32_t col = sp.cbase + ((uint32_t)bx * (uint32_t)sp.nb[1] + (uint32_t)by) * (uint32_t)sp.nb[2];
           const uint32_t j1 = b.offset[col + (uint32_t)s.z1 + 1u];
           if (!in_bounds(j1, (uint64_t)b.n + 1u, b.err)) continue;
-          for (uint32_t j = b.offset[col + (uint32_t)s.z0] + lane; j < j1; j += 32u) consider(j);
+          for (uint32_t j0 = b.offset[col + (uint32_t)s.z0]; j0 < j1; j0 += 32u) {
+            const uint32_t j = j0 + lane;
+            offer(j < j1 ? key_of(j) : NONE, j);
+          }
         }
     } else {
-      for (uint32_t k = lane; k < nl; k += 32u) {
-        const uint32_t j = list[(size_t)k * b.n + i] & ~RUN_FAR_CELL;
-        if (in_bounds(j, b.n, b.err)) consider(j);
+      for (uint32_t k0 = 0; k0 < nl; k0 += 32u) {
+        const uint32_t j = k0 + lane < nl ? list[(size_t)(k0 + lane) * b.n + i] & ~RUN_FAR_CELL : i;
+        offer(in_bounds(j, b.n, b.err) ? key_of(j) : NONE, j);
       }
     }
-    __syncwarp();
-    f = bf, dx = bdx, dy = bdy, dz = bdz;
-    const uint64_t next = smallest(best);
-    if (next == NONE) return V;
-    apply(__ffs(__ballot_sync(0xffffffffu, best == next)) - 1);
-    from = next + 1u;
+    if (kept != NONE) (void)key_of(kept_j);  // the force of the lane's pair
+    const int pairs = __popc(__ballot_sync(0xffffffffu, kept != NONE));
+    for (int l = 0; l < pairs; ++l) apply(l);
+    if (pairs < 32) return V;
+    from = __shfl_sync(0xffffffffu, kept, 31) + 1u;
   }
 }
 
@@ -493,11 +512,12 @@ __device__ __noinline__ void run_begin(const StepBufs<T>& b, const SceneParams<T
 }
 
 // Grid of the state in buffer `cur`, sorted into the other one, and with
-// frac > 0 its lists.  False: a barrier gave up.
+// frac > 0 its lists.  wait: RUN_CROWD is complete at the end.  False: a
+// barrier gave up.
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
                                          const RunBufs<T>& R, int cur, bool counted, float frac, uint32_t build,
-                                         int64_t n_cells, uint32_t scatter_blocks, uint32_t move_blocks) {
+                                         bool wait, int64_t n_cells, uint32_t scatter_blocks, uint32_t move_blocks) {
   const uint32_t stride = gridDim.x * STEP_THREADS;
   if (!counted) {
     vec4_t<T>* Ps = R.p(cur);
@@ -525,6 +545,8 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
       scan_tile_with_sums<true, STEP_SCAN_ITEMS_SMALL>(t, b.count, b.offset, n_cells, b.tile_sum);
   }
   if (!run_barrier(R.bar, b.err)) return false;
+  // (behind a barrier that every CTA came to after it read the word)
+  if (frac > 0.0f && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD) = 0ull;
   for (uint32_t blk = blockIdx.x; blk < scatter_blocks; blk += gridDim.x)
     scatter_block<true>(blk, b.cell, b.slot, b.orig, b.offset, b.tmp, b.count, b.n, b.tile_sum, b.n_tiles, b.err);
   if (!run_barrier(R.bar, b.err)) return false;
@@ -540,8 +562,25 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
     const T rmax = (T)__uint_as_float(R.ctl[RUN_RMAX]) * T(1.0001);
     for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += stride)
       run_build_one<T, MULTI, MESH, TAPE>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax, build);
+    if (wait && !run_barrier(R.bar, b.err)) return false;
   }
   return true;
+}
+
+// Whether too many spheres had more neighbours than a list holds at the
+// launch's last build with lists; the launch then goes on without.  A trip of
+// run_slow costs about four of the walk of a grid step: where the spheres
+// beyond their lists take more than that walk takes for all spheres, it is the
+// cheaper one.  (50,000-sphere pile, a capacity of 2: 49 us a step on lists,
+// 32 us without; 79,420 spheres, 3 % of them four times as large, a capacity
+// of 16: 36 us on lists, 151 us in the step kernels.)  A recorded run has to
+// keep all its lists.
+// Where lists begin, the build is waited for, because a step on them may take
+// very long; spheres that crowd together later do so step by step, and the
+// next build is soon enough.
+template <bool TAPE, class T>
+__device__ __forceinline__ bool run_crowded(const StepBufs<T>& b, const RunBufs<T>& R) {
+  return 4ull * *reinterpret_cast<volatile unsigned long long*>(R.ctl + RUN_CROWD) > (TAPE ? 0u : b.n);
 }
 
 // One step without lists on a grid built for it; the next step's cells are
@@ -925,6 +964,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   int cur = 1;           // buffer with the state before the step's contacts
   bool lists = false;    // the lists are those of a build that still covers the motion
   bool counted = true;   // the state's cells are counted already
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD) = 0ull;
   float D = 0.0f;        // motion since the last build, in cells
   float frac = 0.0f;     // skin of the last build, in cells
   uint32_t rebuilds = 0, build = 0;
@@ -945,7 +985,8 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
         build = rebuilds;
         streak = RUN_CALM_STEPS;
       }
-      lists = streak >= RUN_CALM_STEPS || R.skin > 0.0f;
+      const bool was = lists;
+      lists = !run_crowded<TAPE>(b, R) && (streak >= RUN_CALM_STEPS || R.skin > 0.0f);
       // (a single fast step, a sphere pushed out of a wall, is no measure)
       // (A recorded run depends on its starting state alone, for the backward
       // pass to give the same sums every time; its builds have to last for
@@ -953,9 +994,14 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
       const float last_for = TAPE ? fmaxf(RUN_STEPS_PER_BUILD, 0.7f * (float)steps) : RUN_STEPS_PER_BUILD;
       const float widest = TAPE && s == 0u ? RUN_SKIN_FIRST : RUN_SKIN_MAX;
       frac = fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest);
-      frac = R.skin > 0.0f ? R.skin : (lists ? frac : 0.0f);
-      if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, n_cells, scatter_blocks, move_blocks))
+      frac = !lists ? 0.0f : (R.skin > 0.0f ? R.skin : frac);
+      if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, lists && !was, n_cells, scatter_blocks,
+                                               move_blocks))
         return run_leave(b, R.ctl);
+      if (lists && !was && run_crowded<TAPE>(b, R)) {
+        if (TAPE) return;
+        lists = false;
+      }
       cur = 1 - cur;
       D = 0.0f;
       fresh = true;

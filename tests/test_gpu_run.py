@@ -173,3 +173,32 @@ def test_set_lists_of_any_capacity(need_gpu, cap):
         overflows = sim.list_stats()[1]
     assert same(got, want)
     assert (overflows > 0) == (cap < 200)  # all 200 small spheres are neighbours of the large one
+
+
+def heap(k: int, n: int = 8000) -> scenes.Scene:
+    """k spheres on top of one another, all in contact until their collisions
+    part them, among n slow ones."""
+    sc = scenes.pile(n, seed=81, k_spring=1e-4)
+    st = sc.state.copy()
+    st[:, 3:6] *= 0.02
+    st[:k, :3] = st[n // 2, :3] + np.random.default_rng(82).normal(0, 2e-4, size=(k, 3))
+    return sc.copy(state=st, dt=1e-6)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("k", [32, 33, 34, 64, 65, 66, 97, 400])
+def test_lists_shorter_than_the_spheres_in_contact(need_gpu, k, prec):
+    # contacts of a sphere beyond its list are taken 32 at a time; 400 such
+    # spheres are too many, and the run goes on without lists
+    sc = heap(k)
+    want = both([sc], prec, (40, 9))[1]  # of the step kernels
+    for skin in (0.0, 0.05):
+        with psb200.Simulation(sc, prec) as sim:
+            sim.set_state()
+            sim.set_neighbor_lists(skin, 16)
+            sim.step(40)
+            sim.step(9)
+            got = (sim.get_state(), *sim.buckets())
+            overflows = sim.list_stats()[1]
+        assert same(got, want)
+        assert skin == 0.0 or overflows > 0
