@@ -179,6 +179,8 @@ struct ps_sim {
   size_t run_bytes = 0;
   unsigned run_grid = 0;                  // CTAs: one wave, or fewer for a small scene
   bool run_own = false;                   // those CTAs have a thread for every sphere
+  unsigned record_grid = 0;               // the same of recorded runs, whose kernel is another (0: not asked yet)
+  bool record_own = false;
   bool run_off = false;                   // ps_autotune times the step kernels
   uint32_t run_turn = 0, list_turn = 0;   // launches on the control words of run_arena and of list_arena
   uint32_t run_id = 0, run_seen = 0;      // runs launched, and the last one whose report was read (run_read)
@@ -1059,15 +1061,15 @@ int run_sms(const ps_sim* s) {
   return sms;
 }
 
-// Spheres of one CTA of the run kernel.
-uint32_t run_share(const ps_sim* s) {
-  const int64_t stride = (int64_t)s->run_grid * STEP_THREADS;
+// Spheres of one CTA of a run of `grid` CTAs.
+uint32_t run_share(const ps_sim* s, unsigned grid) {
+  const int64_t stride = (int64_t)grid * STEP_THREADS;
   return (uint32_t)((s->n_total + stride - 1) / stride) * STEP_THREADS;
 }
 
 // set: with the skin and the capacity of ps_set_neighbor_lists
 template <class T>
-RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
+RunBufs<T> run_bufs(ps_sim* s, unsigned grid, bool set = false) {
   const size_t n = (size_t)s->n_total;
   RunBufs<T> R;
   R.P[0] = static_cast<vec4_t<T>*>(s->P0);
@@ -1084,8 +1086,8 @@ RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
   R.list = reinterpret_cast<uint32_t*>(p);
   p += align_up(4 * n * R.cap, 256);
   R.later = reinterpret_cast<uint32_t*>(p);
-  R.later_stride = run_share(s);
-  p += align_up(4 * (size_t)s->run_grid * R.later_stride, 256);
+  R.later_stride = run_share(s, grid);
+  p += align_up(4 * (size_t)grid * R.later_stride, 256);
   R.tris = s->has_mesh ? reinterpret_cast<uint32_t*>(p) : nullptr;
   R.tape = nullptr;
   R.tape_row_bytes = 0;
@@ -1096,17 +1098,18 @@ RunBufs<T> run_bufs(ps_sim* s, bool set = false) {
   return R;
 }
 
-template <class T, bool MULTI, bool MESH>
-int run_prepare(ps_sim* s) {
-  int per_sm = 0, sms = 0;
-  PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, true, false>, STEP_THREADS, 0));
-  s->run_own = (int64_t)blocks_for(s->n_total) <= (int64_t)per_sm * sms;
-  if (!s->run_own)
-    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, false, false>, STEP_THREADS, 0));
+// The grid of a kernel's cooperative launches, by that kernel's own residency.
+template <class T, bool MULTI, bool MESH, bool TAPE>
+int run_prepare(ps_sim* s, unsigned& grid, bool& own) {
+  int per_sm = 0;
+  const int sms = run_sms(s);
+  PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, true, TAPE>, STEP_THREADS, 0));
+  own = (int64_t)blocks_for(s->n_total) <= (int64_t)per_sm * sms;
+  if (!own)
+    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_run<T, MULTI, MESH, false, TAPE>, STEP_THREADS, 0));
   if (per_sm < 1 || sms < 1) return fail(PS_ERR_CUDA, "ps_step: the run kernel cannot be resident");
-  s->run_grid = std::min<unsigned>((unsigned)(per_sm * sms),
-                                   std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
+  grid = std::min<unsigned>((unsigned)(per_sm * sms),
+                            std::max<unsigned>(blocks_for(s->n_total), (unsigned)step_scan_tiles(n_scan(s))));
   return PS_OK;
 }
 
@@ -1117,7 +1120,7 @@ int run_launch(ps_sim* s, uint32_t steps, RunBufs<T> R, uint32_t run_id) {
   R.bar_next = R.ctl + (turn & 1u ? RUN_BAR : RUN_BAR_ODD);
   const StepBufs<T> b = bufs<T>(s);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(s->run_grid);
+  cfg.gridDim = dim3(TAPE ? s->record_grid : s->run_grid);
   cfg.blockDim = dim3(STEP_THREADS);
   cfg.stream = s->stream;
   cudaLaunchAttribute at[2];
@@ -1128,8 +1131,8 @@ int run_launch(ps_sim* s, uint32_t steps, RunBufs<T> R, uint32_t run_id) {
   at[1].val.accessPolicyWindow = cudaAccessPolicyWindow{};
   cfg.attrs = at;
   cfg.numAttrs = s->l2_window_on ? 2 : 1;
-  PS_CUDA(cudaLaunchKernelEx(&cfg, s->run_own ? k_run<T, MULTI, MESH, true, TAPE> : k_run<T, MULTI, MESH, false, TAPE>, b, params<T>(s)[0], (const MeshView*)s->d_mesh_view,
-                             R, steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
+  PS_CUDA(cudaLaunchKernelEx(&cfg, (TAPE ? s->record_own : s->run_own) ? k_run<T, MULTI, MESH, true, TAPE> : k_run<T, MULTI, MESH, false, TAPE>,
+                             b, params<T>(s)[0], (const MeshView*)s->d_mesh_view, R, steps, n_scan(s), (uint32_t)move_blocks(s->n_total, b.n_tiles),
                              (uint32_t)move_blocks(s->n_total, 0), run_id));
   ++turn;  // (a launch that failed has cleared nothing)
   return PS_OK;
@@ -1137,14 +1140,18 @@ int run_launch(ps_sim* s, uint32_t steps, RunBufs<T> R, uint32_t run_id) {
 
 template <class T>
 int run_dispatch_prepare(ps_sim* s) {
-  if (s->multi) return s->has_mesh ? run_prepare<T, true, true>(s) : run_prepare<T, true, false>(s);
-  return s->has_mesh ? run_prepare<T, false, true>(s) : run_prepare<T, false, false>(s);
+  s->record_grid = 0;
+  if (s->multi)
+    return s->has_mesh ? run_prepare<T, true, true, false>(s, s->run_grid, s->run_own)
+                       : run_prepare<T, true, false, false>(s, s->run_grid, s->run_own);
+  return s->has_mesh ? run_prepare<T, false, true, false>(s, s->run_grid, s->run_own)
+                     : run_prepare<T, false, false, false>(s, s->run_grid, s->run_own);
 }
 
 // A run shorter than a probe tells nothing: it always starts with a rebuild.
 template <class T>
 int run_dispatch(ps_sim* s, uint32_t steps, bool set = false) {
-  RunBufs<T> R = run_bufs<T>(s, set);
+  RunBufs<T> R = run_bufs<T>(s, s->run_grid, set);
   uint32_t id = 0;
   if (!set && steps >= RUN_PROBE_STEPS)
     id = ++s->run_id;
@@ -1260,7 +1267,11 @@ constexpr uint32_t TAPE_BUILDS = 3;
 template <class T, bool MULTI>
 int record_run(ps_sim* s, int64_t steps, char* tape, size_t row_bytes, char* lists, std::vector<uint32_t>& build, bool& ok) {
   const size_t n = (size_t)s->n_total;
-  RunBufs<T> R = run_bufs<T>(s);
+  if (s->record_grid == 0) {
+    const int rc = run_prepare<T, MULTI, false, true>(s, s->record_grid, s->record_own);
+    if (rc != PS_OK) return rc;
+  }
+  RunBufs<T> R = run_bufs<T>(s, s->record_grid);
   R.tape = tape;
   R.tape_row_bytes = row_bytes;
   R.max_builds = TAPE_BUILDS;
