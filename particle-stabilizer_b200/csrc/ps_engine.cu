@@ -558,6 +558,8 @@ __global__ void k_counts_from_offsets(const uint32_t* offset, uint32_t* counts, 
 }
 
 // ---- set-up ------------------------------------------------------------------
+cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes);
+
 template <class T>
 SceneParams<T> make_params(const ps_scene_desc& d, const GridHost& g, int64_t pbase, int64_t pcount) {
   SceneParams<T> sp{};
@@ -694,7 +696,7 @@ int upload_grids(ps_sim* s, std::vector<SceneParams<T>>& sps) {
   const size_t tiles_b = align_up(sizeof(uint32_t) * (size_t)step_scan_tiles(n_scan(s)), 256);
   const size_t bounds_b = align_up(sizeof(T) * bounds.size(), 256), scenes_b = sizeof(SceneParams<T>) * sps.size();
   s->cell_bytes = 2 * cells_b + tiles_b;
-  PS_CUDA(cudaMalloc(&s->cell_arena, s->cell_bytes + bounds_b + scenes_b));
+  PS_CUDA(dev_alloc(s, &s->cell_arena, s->cell_bytes + bounds_b + scenes_b));
   char* c = static_cast<char*>(s->cell_arena);
   s->count = reinterpret_cast<uint32_t*>(c);
   s->offset = reinterpret_cast<uint32_t*>(c + cells_b);
@@ -795,11 +797,11 @@ int upload_mesh(ps_sim* s) {
     }
   }
   const size_t bt = tri.size() * sizeof(T), ba = aabb.size() * sizeof(T);
-  PS_CUDA(cudaMalloc(&s->d_tri, std::max<size_t>(bt, 16)));
-  PS_CUDA(cudaMalloc(&s->d_aabb, std::max<size_t>(ba, 16)));
-  PS_CUDA(cudaMalloc(&s->d_bin_offset, bin_offset.size() * sizeof(uint32_t)));
-  PS_CUDA(cudaMalloc(&s->d_bin_tri, std::max<size_t>(bin_tri.size(), 1) * sizeof(uint32_t)));
-  PS_CUDA(cudaMalloc(&s->d_mesh_view, sizeof(MeshView)));
+  PS_CUDA(dev_alloc(s, &s->d_tri, std::max<size_t>(bt, 16)));
+  PS_CUDA(dev_alloc(s, &s->d_aabb, std::max<size_t>(ba, 16)));
+  PS_CUDA(dev_alloc(s, reinterpret_cast<void**>(&s->d_bin_offset), bin_offset.size() * sizeof(uint32_t)));
+  PS_CUDA(dev_alloc(s, reinterpret_cast<void**>(&s->d_bin_tri), std::max<size_t>(bin_tri.size(), 1) * sizeof(uint32_t)));
+  PS_CUDA(dev_alloc(s, reinterpret_cast<void**>(&s->d_mesh_view), sizeof(MeshView)));
   PS_CUDA(cudaMemcpy(s->d_tri, tri.data(), bt, cudaMemcpyHostToDevice));
   PS_CUDA(cudaMemcpy(s->d_aabb, aabb.data(), ba, cudaMemcpyHostToDevice));
   PS_CUDA(cudaMemcpy(s->d_bin_offset, bin_offset.data(), bin_offset.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -897,7 +899,6 @@ size_t run_need(const ps_sim* s, int sms, size_t cap) {
 }
 
 void run_alloc(ps_sim* s);
-cudaError_t dev_alloc(ps_sim* s, void** p, size_t bytes);
 
 // Size every scene's grid from its radii and allocate the per-cell arrays.
 int size_grids(ps_sim* s, const double* aos) {
@@ -1530,10 +1531,14 @@ extern "C" int ps_create(const ps_scene_desc* scenes, int32_t n_scenes, int32_t 
   int sms = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   s->run_bytes = s->n_total > 0 ? run_need(s, sms, RUN_LIST_CAP) : 0;
-  const size_t br = s->run_bytes <= RUN_WITH_PARTICLES ? align_up(s->run_bytes, 256) : 0;
-  if (e == cudaSuccess)
-    e = cudaMalloc(&s->part_arena,
-                   4 * b4 + 5 * bu + bs + 256 + bp + bi + bc + br + 2 * sizeof(StatsPartial) * kStatsBlocks + 256);
+  size_t br = s->run_bytes <= RUN_WITH_PARTICLES ? align_up(s->run_bytes, 256) : 0;
+  const size_t part_b = 4 * b4 + 5 * bu + bs + 256 + bp + bi + bc + 2 * sizeof(StatsPartial) * kStatsBlocks + 256;
+  if (e == cudaSuccess) e = cudaMalloc(&s->part_arena, part_b + br);
+  if (e == cudaErrorMemoryAllocation && br > 0) {  // no room for the lists
+    cudaGetLastError();
+    br = s->run_bytes = 0;
+    e = cudaMalloc(&s->part_arena, part_b);
+  }
   if (e != cudaSuccess) {
     delete s;
     return fail(e == cudaErrorMemoryAllocation ? PS_ERR_NOMEM : PS_ERR_CUDA, std::string("ps_create: ") + cudaGetErrorString(e));

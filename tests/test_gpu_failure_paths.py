@@ -4,6 +4,9 @@ really fails), more particles than the slot tags allow, a grid with more
 cells than 32-bit cell ids reach, and a device that does not exist.  After
 each, a normal simulation on the same device still equals the oracle."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -11,6 +14,7 @@ import pytest
 import psb200
 from psb200 import scenes
 from oracle import ps_oracle as O
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +75,43 @@ def test_device_that_does_not_exist(need_gpu):
     rc, msg = create_raw(100, 0, device=99)
     assert rc == PS_ERR_INVALID and "no CUDA device" in msg, (rc, msg)
     still_healthy()
+
+
+NEARLY_FULL = r"""
+import numpy as np
+import torch
+import psb200
+from psb200 import scenes
+
+sc = scenes.pile(480000, seed=8, k_spring=1.0).copy(interval=0.05)
+
+
+def run(sim):
+    sim.set_state()
+    sim.step(9)
+    return sim.get_state()
+
+
+with psb200.Simulation(sc, "f32") as sim:  # (loads the kernels)
+    want = run(sim)
+    sim.step(9)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+room = 96 << 20  # 71 MB of particle arrays fit, with 64 MB of lists they do not
+hog = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+with psb200.Simulation(sc, "f32") as sim:
+    got = run(sim)
+    assert sim.launches() > 9, "the lists found room"
+assert np.array_equal(got, want)
+print("DONE", flush=True)
+"""
+
+
+def test_simulation_whose_lists_do_not_fit(need_gpu):
+    # the particle arrays fit into what the device has left, their lists do
+    # not: the simulation is created all the same and steps without them
+    env = dict(os.environ)
+    env["PYTHONPATH"] = os.pathsep.join([ROOT, os.path.join(ROOT, "particle-stabilizer_b200", "python"),
+                                         env.get("PYTHONPATH", "")])
+    r = subprocess.run([sys.executable, "-c", NEARLY_FULL], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.rstrip().endswith("DONE"), r.stdout[-3000:] + r.stderr[-3000:]
