@@ -211,8 +211,11 @@ int ps_backward(ps_sim* sim, const double* dl_dstate, ps_grad* grads, double* dl
  * of that scene; f >= 1) and a graph block length L (steps per captured CUDA
  * graph), keeps the fastest pair, and restores the state.  ms_table (may be
  * NULL) receives n_factors x n_blocks milliseconds per step, factor-major.
- * The trials run the step kernels, to which graph blocks and contact kernels
- * belong; the chosen cell size holds for every path.
+ * These are times of the step kernels, to which graph blocks and contact
+ * kernels belong, or in neighbour-list mode of steps on lists.  Where a call
+ * of trial_steps steps takes a run instead (ps_step: 8 steps or more of a
+ * scene that is calm enough), such calls are timed as well, and f is the one
+ * on which they are fastest; L is then the fastest one on that f.
  * The cell size changes the grid and with it the summation order of the
  * contacts, so later trajectories are those of the chosen grid: deterministic,
  * and equal to the oracle's with that cell size, but not bit-equal to runs
@@ -254,8 +257,8 @@ int ps_tune_neighbor_lists(ps_sim* sim, int64_t trial_steps, const double* skins
 typedef struct ps_tune_result {
   double cell_factor;        /* chosen f                                          */
   int64_t graph_block;       /* chosen L                                          */
-  double ms_per_step;        /* trial time per step with the choice               */
-  double before_ms_per_step; /* trial time per step with the grid, L and contact  */
+  double ms_per_step;        /* smallest time in ms_table and contact_ms          */
+  double before_ms_per_step; /* the same kind of time with the grid, L and contact */
                              /* kernel in effect when ps_autotune was called      */
   int32_t contact_walk;      /* chosen contact kernel: PS_WALK_LANE/_WARP/_ADAPTIVE */
   int32_t contact_block;     /* and its threads per CTA                           */

@@ -1960,6 +1960,7 @@ int resize_grids(ps_sim* s, const std::vector<double>& host_state) {
   s->run_grid = 0;
   s->run_seen = s->run_id;
   s->run_settled = false;
+  s->run_backoff = s->run_backoff_len = 0;
   s->fwd_steps = 0;
   s->l2_window_on = s->l2_window_tried = false;
   s->grid_sized = false;
@@ -1982,7 +1983,7 @@ extern "C" int ps_autotune(ps_sim* s, int64_t trial_steps, const double* cell_fa
   for (int32_t l = 0; l < n_blocks; ++l)
     if (graph_blocks[l] < 1) return fail(PS_ERR_INVALID, "ps_autotune: graph blocks must be >= 1");
   DeviceGuard guard(s->device);
-  struct StepKernelsOnly {  // the trials time the step kernels
+  struct StepKernelsOnly {  // the trials time the step kernels, unless they say otherwise
     ps_sim* s;
     explicit StepKernelsOnly(ps_sim* sim) : s(sim) { s->run_off = true; }
     ~StepKernelsOnly() { s->run_off = false; }
@@ -2000,10 +2001,10 @@ extern "C" int ps_autotune(ps_sim* s, int64_t trial_steps, const double* cell_fa
   cudaEvent_t ea, eb;
   PS_CUDA(cudaEventCreate(&ea));
   PS_CUDA(cudaEventCreate(&eb));
-  // one trial: warm-up (captures the graphs), restore, timed steps, restore
-  auto trial = [&](double& ms_per_step) -> int {
+  // one trial: `warm` steps (captures the graphs), restore, timed steps, restore
+  auto trial = [&](double& ms_per_step, int64_t warm) -> int {
     int r = load_state(s, saved);
-    if (r == PS_OK) r = ps_step(s, std::min(trial_steps, s->graph_block));
+    if (r == PS_OK) r = ps_step(s, warm);
     if (r == PS_OK) r = load_state(s, saved);
     if (r != PS_OK) return r;
     cudaEventRecord(ea, s->stream);
@@ -2022,25 +2023,46 @@ extern "C" int ps_autotune(ps_sim* s, int64_t trial_steps, const double* cell_fa
     return resize_grids(s, host);
   };
   double before = 0.0;
-  rc = trial(before);
+  rc = trial(before, std::min(trial_steps, s->graph_block));
   double best = INFINITY, best_f = cell_factors[0];
   int64_t best_l = graph_blocks[0];
+  // the same of calls that take a run instead, while they do on every grid
+  double best_run = INFINITY, run_f = 0.0;
+  int64_t run_l = 0;
+  bool runs = s->list_skin <= 0.0 && trial_steps >= RUN_MIN_STEPS && s->run_arena != nullptr;
   for (int32_t f = 0; f < n_factors && rc == PS_OK; ++f) {
     rc = apply_factor(cell_factors[f]);
+    double run_ms = INFINITY, best_here = INFINITY;
+    if (rc == PS_OK && runs) {
+      s->run_off = false;
+      rc = trial(run_ms, trial_steps);
+      s->run_off = true;
+      runs = s->last_launches < trial_steps;
+      if (runs && run_ms < best_run) {
+        best_run = run_ms;
+        run_f = cell_factors[f];
+        run_l = graph_blocks[0];
+      }
+    }
     for (int32_t l = 0; l < n_blocks && rc == PS_OK; ++l) {
       for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
       s->graphs.clear();
       s->graph_block = graph_blocks[l];
       double ms = 0.0;
-      rc = trial(ms);
+      rc = trial(ms, std::min(trial_steps, s->graph_block));
       if (ms_table != nullptr) ms_table[(size_t)f * (size_t)n_blocks + (size_t)l] = ms;
       if (rc == PS_OK && ms < best) {
         best = ms;
         best_f = cell_factors[f];
         best_l = graph_blocks[l];
       }
+      if (rc == PS_OK && ms < best_here) {
+        best_here = ms;
+        if (run_f == cell_factors[f]) run_l = graph_blocks[l];
+      }
     }
   }
+  if (runs) best_f = run_f, best_l = run_l;
   if (rc == PS_OK) rc = apply_factor(best_f);
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
   s->graphs.clear();
@@ -2055,7 +2077,7 @@ extern "C" int ps_autotune(ps_sim* s, int64_t trial_steps, const double* cell_fa
     for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);
     s->graphs.clear();
     double ms = 0.0;
-    rc = trial(ms);
+    rc = trial(ms, std::min(trial_steps, s->graph_block));
     out->contact_ms[v] = ms;
     if (rc == PS_OK && ms < best_k) {
       best_k = ms;

@@ -184,3 +184,23 @@ def test_runs_behind_one_whose_barrier_gave_up_return_at_once(need_gpu):
     r = subprocess.run([sys.executable, "-c", AFTER_A_BARRIER_GAVE_UP], cwd=ROOT, env=env, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and r.stdout.rstrip().endswith("DONE"), r.stdout[-3000:] + r.stderr[-3000:]
+
+
+def test_tuned_cell_size_is_that_of_the_calls_path(need_gpu):
+    # a million spheres, calm enough for runs: the step kernels are fastest
+    # on the smallest cells, calls of many steps on the largest
+    sc, factors, n = scenes.c2_scene(k_spring=0.25), (1.0, 2.0), 100
+    ms = {}
+    for f in factors:
+        with psb200.Simulation(sc.copy(interval=2.0 * f * sc.r_max()), "f32") as sim:
+            sim.set_state()
+            sim.checkpoint_save(0)
+            sim.step(3)  # (the step kernels, which the tuner uses too)
+            sim.step(n)
+            for _ in range(3):
+                sim.checkpoint_load(0)
+                ms[f] = min(ms.get(f, np.inf), sim.time_steps(n))
+    with psb200.Simulation(sc, "f32") as sim:
+        sim.set_state()
+        chosen = sim.autotune(trial_steps=n, cell_factors=factors, graph_blocks=(100,))["cell_factor"]
+    assert ms[chosen] <= 1.15 * min(ms.values())
