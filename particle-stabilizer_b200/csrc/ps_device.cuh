@@ -81,23 +81,6 @@ __device__ __forceinline__ uint32_t ld_pl(const uint32_t* p) {
   else
     return *p;
 }
-template <class T, bool COH>
-__device__ __forceinline__ vec4_t<T> ld4c(const vec4_t<T>* p) {
-  if constexpr (!COH) {
-    return ld4<T>(p);
-  } else if constexpr (sizeof(T) == 4) {
-    return __ldcg(p);
-  } else {
-    const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-    const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-    vec4_t<T> v;
-    v.x = a.x;
-    v.y = a.y;
-    v.z = b.x;
-    v.w = b.y;
-    return v;
-  }
-}
 
 // Wait until the grid this kernel depends on has completed and its writes
 // are visible, when it was launched with programmatic stream serialization
@@ -128,7 +111,6 @@ struct SceneParams {
   uint32_t pbase; // first particle slot
   uint32_t pcount;
   // triangle container (mesh_tris == 0: box walls)
-  uint32_t mesh_tri_base;  // first triangle in the global soup
   uint32_t mesh_tris;
   uint32_t mesh_bin_base;  // first bin of this scene's triangle bins
   int32_t mesh_nb[3];      // triangle-bin grid

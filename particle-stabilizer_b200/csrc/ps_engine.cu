@@ -115,7 +115,7 @@ struct ps_sim {
   bool multi = false, has_mesh = false;
 
   // grids (sized on the first ps_set_state)
-  bool grid_sized = false, grid_valid = false, stepped = false;
+  bool grid_sized = false, grid_valid = false;
   std::vector<GridHost> grids;
   int64_t c_total = 0, bins_total = 0, tri_total = 0;
 
@@ -311,7 +311,6 @@ int64_t enqueue_steps(ps_sim* s, int64_t steps) {
   const StepBufs<T> b = bufs<T>(s);
   const SceneParams<T> sp0 = params<T>(s)[0];
   const unsigned gb = blocks_for(s->n_total);
-  const unsigned gp = blocks_for(s->n_total);
   const unsigned gs = (unsigned)step_scan_tiles(n_scan(s));
   cudaStream_t st = s->stream;
   int64_t launches = 0;
@@ -349,7 +348,6 @@ void enqueue_steps_recorded(ps_sim* s, int64_t steps, std::vector<LaunchRecord>&
   const StepBufs<T> b = bufs<T>(s);
   const SceneParams<T> sp0 = params<T>(s)[0];
   const unsigned gb = blocks_for(s->n_total);
-  const unsigned gp = blocks_for(s->n_total);
   const unsigned gs = (unsigned)step_scan_tiles(n_scan(s));
   cudaStream_t st = s->stream;
   size_t r = 0;
@@ -589,7 +587,6 @@ SceneParams<T> make_params(const ps_scene_desc& d, const GridHost& g, int64_t pb
   sp.cbase = (uint32_t)g.cbase;
   sp.pbase = (uint32_t)pbase;
   sp.pcount = (uint32_t)pcount;
-  sp.mesh_tri_base = (uint32_t)g.tri_base;
   sp.mesh_tris = (uint32_t)g.n_tri;
   sp.mesh_bin_base = (uint32_t)g.bin_base;
   sp.mesh_iv = (T)g.mesh_iv;
@@ -1885,9 +1882,7 @@ extern "C" int ps_step(ps_sim* s, int64_t n_steps) {
     rc = step_graphs(s, n_steps);
     s->grid_valid = true;
   }
-  if (rc != PS_OK) return rc;
-  s->stepped = true;
-  return PS_OK;
+  return rc;
 }
 
 extern "C" int ps_checkpoint_save(ps_sim* s, int32_t slot) {
