@@ -244,10 +244,14 @@ __device__ __forceinline__ void cell_ranges(const StepBufs<T>& b, const ScenePar
 
 // Cells [c0, c1] of one axis that can hold a point within `reach` of x.
 // The hash is monotonic in x, so the cells of x - reach and x + reach bound
-// them; the pad covers the rounding of x +- reach.
+// them; the pad covers the rounding of x +- reach, by eight units of the last
+// place (far from the origin a pad of FP32's size took FP64 scenes into cells
+// whose spheres are out of reach: 60,000 spheres 1e6 from it, 2.1 ms a step
+// instead of 0.13).
 template <class T>
 __device__ __forceinline__ void axis_span(T x, T reach, T lo, T iv, int32_t nb, int32_t& c0, int32_t& c1) {
-  const T pad = reach + (fabs(x) + fabs(lo)) * T(1.0 / 1048576.0);
+  constexpr T ULPS = sizeof(T) == 4 ? T(1.0 / 1048576.0) : T(1.0 / 562949953421312.0);  // 2^-20, 2^-49
+  const T pad = reach + (fabs(x) + fabs(lo)) * ULPS;
   c0 = axis_cell<T>(x - pad, lo, iv, nb);
   c1 = axis_cell<T>(x + pad, lo, iv, nb);
 }

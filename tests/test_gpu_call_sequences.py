@@ -204,3 +204,30 @@ def test_tuned_cell_size_is_that_of_the_calls_path(need_gpu):
         sim.set_state()
         chosen = sim.autotune(trial_steps=n, cell_factors=factors, graph_blocks=(100,))["cell_factor"]
     assert ms[chosen] <= 1.15 * min(ms.values())
+
+
+def moved_by(sc: scenes.Scene, d) -> scenes.Scene:
+    """The same scene elsewhere (a power of two keeps the digits that count)."""
+    d = np.asarray(d, dtype=np.float64)
+    st = sc.state.copy()
+    st[:, :3] += d
+    tri = None if sc.tri is None else (sc.tri.reshape(-1, 3, 3) + d).reshape(-1, 9)
+    return sc.copy(state=st, tri=tri, box_min=tuple(np.add(sc.box_min, d)), box_max=tuple(np.add(sc.box_max, d)))
+
+
+@pytest.mark.parametrize("make", [lambda: scenes.pile(60000, seed=91, k_spring=0.05)], ids=["box"])
+def test_scenes_far_from_the_origin(need_gpu, make):
+    # FP64: digits enough, and about as fast as at the origin
+    ms = []
+    for d in ((0.0, 0.0, 0.0), (2.0 ** 20, -(2.0 ** 20), 2.0 ** 20)):
+        sc = moved_by(make(), d)
+        out = []
+        for fn in ("step", "profile_steps"):
+            with psb200.Simulation(sc, "f64") as sim:
+                sim.set_state()
+                getattr(sim, fn)(60)
+                out.append(sim.get_state())
+                if fn == "step":
+                    ms.append(min(sim.time_steps(100) for _ in range(3)))
+        assert np.array_equal(out[0], out[1])
+    assert ms[1] < 2.0 * ms[0], ms
