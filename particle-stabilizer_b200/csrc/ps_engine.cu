@@ -760,7 +760,8 @@ int upload_mesh(ps_sim* s) {
       const T iv = (T)g.mesh_iv;
       double size = g.mesh_iv;  // of the coordinates, for the rounding of the device's own tests
       for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
-      const double reach = 1.001 * g.mesh_reach + 1e-6 * size;
+      const double ulp = (double)std::numeric_limits<T>::epsilon() * size;
+      const double reach = 1.001 * g.mesh_reach + 8.0 * ulp;
       for (int64_t t = 0; t < g.n_tri; ++t) {
         const int64_t gt = g.tri_base + t;
         int32_t b0[3], b1[3];
@@ -770,13 +771,13 @@ int upload_mesh(ps_sim* s) {
         }
         const double* n = nrm.data() + 3 * gt;
         const double* v0 = s->tris[sc].data() + 9 * t;
-        const double far = reach + (0.5 + 1e-3) * g.mesh_iv * (std::fabs(n[0]) + std::fabs(n[1]) + std::fabs(n[2])) + 1e-5 * size;
+        const double far = reach + (0.5 + 1e-3) * g.mesh_iv * (std::fabs(n[0]) + std::fabs(n[1]) + std::fabs(n[2])) + 80.0 * ulp;
         double off = 0.0;  // of its vertices from the plane (not a number for a triangle without a normal)
         for (int k = 3; k < 9; k += 3) {
           const double d = std::fabs(n[0] * (v0[k] - v0[0]) + n[1] * (v0[k + 1] - v0[1]) + n[2] * (v0[k + 2] - v0[2]));
           if (!(d <= off)) off = d;
         }
-        const bool flat = off <= 1e-6 * size;  // it is flat and its normal is good
+        const bool flat = off <= 8.0 * ulp;  // it is flat and its normal is good
         for (int32_t x = b0[0]; x <= b1[0]; ++x)
           for (int32_t y = b0[1]; y <= b1[1]; ++y)
             for (int32_t z = b0[2]; z <= b1[2]; ++z) {
@@ -953,8 +954,9 @@ int size_grids(ps_sim* s, const double* aos) {
       if (!(g.mesh_iv > 0.0)) g.mesh_iv = 1.0;
       double size = 0.0;
       for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
-      for (int a = 0; a < 3; ++a) {  // room for every centre that can touch the mesh
-        const double room = 1.01 * g.mesh_reach + 1e-5 * size;
+      const double ulp = (s->precision == PS_FP32 ? std::numeric_limits<float>::epsilon() : std::numeric_limits<double>::epsilon()) * size;
+      for (int a = 0; a < 3; ++a) {  // room for every centre that can touch the mesh, and for the rounding of its own tests
+        const double room = 1.01 * g.mesh_reach + 80.0 * ulp;
         g.mesh_lo[a] -= room;
         g.mesh_hi[a] += room;
         g.mesh_nb[a] = (int32_t)((g.mesh_hi[a] - g.mesh_lo[a]) / g.mesh_iv) + 1;

@@ -215,7 +215,8 @@ def moved_by(sc: scenes.Scene, d) -> scenes.Scene:
     return sc.copy(state=st, tri=tri, box_min=tuple(np.add(sc.box_min, d)), box_max=tuple(np.add(sc.box_max, d)))
 
 
-@pytest.mark.parametrize("make", [lambda: scenes.pile(60000, seed=91, k_spring=0.05)], ids=["box"])
+@pytest.mark.parametrize("make", [lambda: scenes.pile(60000, seed=91, k_spring=0.05),
+                                  lambda: scenes.funnel_wall_scene(20000, seed=92)], ids=["box", "mesh"])
 def test_scenes_far_from_the_origin(need_gpu, make):
     # FP64: digits enough, and about as fast as at the origin
     ms = []
