@@ -1659,21 +1659,24 @@ namespace {
 // to 13.9 ms with a graph, 10.4 to 10.9 ms without).  The second time, it is
 // captured, so that a program's warm-up still takes that: the same 100 steps
 // repeated take 0.4 to 0.8 % longer one by one (9.38 to 9.66 ms against 9.45
-// to 9.73 ms).  The odd lengths around a probe seldom come again.  The trials
-// of ps_autotune (run_off) warm up once and always use graphs.
+// to 9.73 ms).  The odd lengths of a call's steps before or after a probe
+// seldom come again: they are launched one by one in scenes of any size
+// (30,000 spheres too fast for lists, first calls of 100, 100 and 300 steps:
+// 17.8 ms with a graph for them, 16.0 ms without).  The trials of ps_autotune
+// (run_off) warm up once and always use graphs.
 constexpr int64_t EAGER_MIN_SPHERES = 1 << 18;
 
 // Run n_steps on the step kernels as CUDA graphs of up to graph_block steps,
-// asynchronously.
-int step_graphs(ps_sim* s, int64_t n_steps) {
+// asynchronously.  part: the call has other steps besides.
+int step_graphs(ps_sim* s, int64_t n_steps, bool part = false) {
   setup_l2_window(s);
   ensure_l2_limit(s);
   int64_t left = n_steps;
   while (left > 0) {
     const int64_t L = std::min(left, s->graph_block);
     auto it = s->graphs.find(L);
-    if (it == s->graphs.end() && L < s->graph_block && s->n_total >= EAGER_MIN_SPHERES &&
-        !s->run_off && s->eager_lengths.insert(L).second) {
+    if (it == s->graphs.end() && L < s->graph_block && !s->run_off &&
+        (part || (s->n_total >= EAGER_MIN_SPHERES && s->eager_lengths.insert(L).second))) {
       s->precision == PS_FP32 ? enqueue_steps_dispatch<float>(s, L) : enqueue_steps_dispatch<double>(s, L);
       PS_CUDA(cudaGetLastError());
       s->last_launches += 1 + 4 * L;
@@ -1751,7 +1754,7 @@ int step_run(ps_sim* s, int64_t n_steps) {
     if (s->run_backoff > 0 || waiting || (!s->run_settled && left < RUN_PROBE_STEPS)) {
       L = std::min(left, s->run_backoff > 0 ? s->run_backoff : RUN_BACKOFF_MIN);
       s->run_backoff = std::max<int64_t>(0, s->run_backoff - L);
-      rc = step_graphs(s, L);
+      rc = step_graphs(s, L, L < n_steps);
       s->grid_valid = true;
     } else {
       const int64_t launches = (left + run_block(s) - 1) / run_block(s);
@@ -1788,7 +1791,7 @@ int step_lists(ps_sim* s, int64_t n_steps) {
   for (int64_t left = n_steps; left > 0;) {
     if (s->list_backoff > 0) {
       const int64_t L = std::min(left, s->list_backoff);
-      const int rc = step_graphs(s, L);
+      const int rc = step_graphs(s, L, L < n_steps);
       if (rc != PS_OK) return rc;
       s->grid_valid = true;
       s->list_backoff -= L;
