@@ -82,7 +82,7 @@ enum : int {
   RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
   RUN_BAR_ODD = 12, // grid barrier of odd launches
   RUN_LEFT = 14,    // CTAs that left because a barrier gave up
-  RUN_CROWD = 16,   // what the spheres beyond their lists cost (64 bits), of the last build
+  RUN_CROWD = 16,   // (2 words) spheres beyond their lists at the last build: run_crowded's cost and candidates
 };
 
 template <class T>
@@ -287,18 +287,50 @@ __host__ __device__ constexpr int run_batch() {
   return sizeof(T) == 4 ? 4 : 2;
 }
 
+// What the CTA's spheres beyond their lists cost at a build (run_crowded).
+struct RunCrowd {
+  float sum;      // of run_slow's trips
+  uint32_t most;  // the most of one sphere (the bits of a float that is not negative order like it)
+  uint32_t cand;  // the most candidates of one
+};
+
+// Sphere i, beyond its list, into `c` (shared): passes of run_slow over the
+// columns of `s`, 32 candidates a trip, and the keys that a pass keeps.
+template <class T>
+__device__ __noinline__ void run_cost(uint32_t i, const StepBufs<T>& b, const SceneParams<T>& sp, const vec4_t<T>* Ps,
+                                      const Span<T>& s, RunCrowd& c) {
+  const vec4_t<T> P = Ps[i];
+  uint32_t touch = 0, trips = 0, cand = 0;
+  for (int32_t bx = s.x0; bx <= s.x1; ++bx)
+    for (int32_t by = s.y0; by <= s.y1; ++by) {
+      const uint32_t col = sp.cbase + ((uint32_t)bx * (uint32_t)sp.nb[1] + (uint32_t)by) * (uint32_t)sp.nb[2];
+      const uint32_t j0 = b.offset[col + (uint32_t)s.z0], j1 = b.offset[col + (uint32_t)s.z1 + 1u];
+      if (!in_bounds(j1, (uint64_t)b.n + 1u, b.err)) continue;
+      cand += j1 - j0;
+      trips += (j1 - j0 + 31u) / 32u;
+      for (uint32_t j = j0; j < j1; ++j) {
+        const vec4_t<T> Q = Ps[j];
+        const T dx = P.x - Q.x, dy = P.y - Q.y, dz = P.z - Q.z, r = P.w + Q.w;
+        touch += dx * dx + dy * dy + dz * dz < r * r ? 1u : 0u;
+      }
+    }
+  const float cost = (1.0f + (float)(touch / 32u)) * (float)(trips + min(touch, 96u)) + 30.0f;
+  atomicAdd(&c.sum, cost);
+  atomicMax(&c.most, __float_as_uint(cost));
+  atomicMax(&c.cand, cand);
+}
+
 // List and count word of slot i of the sorted state (positions P, sorted
 // cell ids scell); columns are visited in ascending cell id, so a list is in
 // ascending (cell, original index).
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, const SceneParams<T>& sp,
                                               const MeshView* mv, const RunBufs<T>& R, const vec4_t<T>* Ps, T frac,
-                                              T rmax, uint32_t build) {
+                                              T rmax, uint32_t build, RunCrowd& crowd) {
   uint32_t* const list = R.template lists<TAPE>(build, b.n);
   const vec4_t<T> P = Ps[i];
   const T skin = frac * sp.interval;
   uint32_t k = 0, word = 0;
-  uint32_t cand = 0, trips = 0;  // candidates, and the trips of a warp that goes through them column by column
   if (isfinite(P.x) && isfinite(P.y) && isfinite(P.z)) {
     int32_t cx, cy, cz;
     cell_coords<T>(b.scell[i], sp, cx, cy, cz);
@@ -335,8 +367,6 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
           lo[q] = ok ? b.offset[col + (uint32_t)s.z0] : 0u;
           hi[q] = ok ? b.offset[col + (uint32_t)s.z1 + 1u] : 0u;
           if (!in_bounds(hi[q], (uint64_t)b.n + 1u, b.err)) hi[q] = lo[q] = 0u;
-          cand += hi[q] - lo[q];
-          trips += (hi[q] - lo[q] + 31u) / 32u;
         }
 #pragma unroll
         for (int q = 0; q < COLS; ++q)
@@ -367,12 +397,35 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
     }
   }
   if (k > R.cap) {
-    // passes of run_slow times their trips, per trip that 32 lanes' own walks take
-    atomicAdd(reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD), (1ull + k / 32u) * trips * 32u / max(cand, 1u));
+    run_cost<T>(i, b, sp, Ps, reach_span<T>(P, (P.w + rmax * sp.interval + skin) * T(1.001), sp), crowd);
     word |= RUN_OVERFLOW, k = 0;
     R.ctl[RUN_FULL] = 1u;
   }
   R.template counts<TAPE>(build, b.n)[i] = (uint16_t)(word | k);
+}
+
+// Whether, at the launch's last build with lists, the spheres beyond their
+// lists would take longer than steps without lists; the launch then goes on
+// without.  A CTA takes its own such spheres, a warp each: 0.25 us a trip for
+// the one with the most to do, against the rebuild and 0.2 us for every
+// candidate of a thread's spheres.  Both are good to a factor of two (us a step
+// with lists / without, and which the rule takes, FP32: 100 spheres in a heap
+// among 8,000, 543 / 72, without; 400 among 200,000, 14,430 / 341, without;
+// 600,000-sphere pile, lists of 1, 247 / 109, without; of 3, 68 / 103, with;
+// 79,420 spheres, 3 % of them four times as large, lists of 16, 37 / 189, with;
+// 20 of 83,474 ten times as large, lists of 48, 321 / 5,210, with; 3,000 in one
+// cell, 440 / 587, without).
+// A recorded run has to keep all its lists.
+// Where lists begin, the build is waited for, because a step on them may take
+// very long; spheres that crowd together later do so step by step, and the
+// next build is soon enough.
+template <bool TAPE, class T>
+__device__ __forceinline__ bool run_crowded(const StepBufs<T>& b, const RunBufs<T>& R) {
+  const volatile uint32_t* c = R.ctl + RUN_CROWD;
+  const float cost = __uint_as_float(c[0]), cand = (float)c[1];
+  if (TAPE) return cost > 0.0f;
+  const float share = (float)((b.n + gridDim.x * STEP_THREADS - 1u) / (gridDim.x * STEP_THREADS));
+  return 0.25f * cost > 20.0f + (float)b.n / 12000.0f + 0.2f * cand * share;
 }
 
 // Contacts of slot i in the exact order whatever has moved: the overlapping
@@ -550,7 +603,7 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
   }
   if (!run_barrier(R.bar, b.err)) return false;
   // (behind a barrier that every CTA came to after it read the word)
-  if (frac > 0.0f && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD) = 0ull;
+  if (frac > 0.0f && blockIdx.x == 0 && threadIdx.x < 2u) R.ctl[RUN_CROWD + threadIdx.x] = 0u;
   for (uint32_t blk = blockIdx.x; blk < scatter_blocks; blk += gridDim.x)
     scatter_block<true>(blk, b.cell, b.slot, b.orig, b.offset, b.tmp, b.count, b.n, b.tile_sum, b.n_tiles, b.err);
   if (!run_barrier(R.bar, b.err)) return false;
@@ -564,27 +617,20 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
   if (frac > 0.0f) {
     const vec4_t<T>* Ps = R.p(1 - cur);
     const T rmax = (T)__uint_as_float(R.ctl[RUN_RMAX]) * T(1.0001);
+    __shared__ RunCrowd crowd;
+    if (threadIdx.x == 0) crowd = {0.0f, 0u, 0u};
+    __syncthreads();
     for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += stride)
-      run_build_one<T, MULTI, MESH, TAPE>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax, build);
+      run_build_one<T, MULTI, MESH, TAPE>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax, build, crowd);
+    __syncthreads();
+    if (threadIdx.x == 0 && crowd.cand != 0u) {  // (the CTA with the most to do decides)
+      const float most = fmaxf(crowd.sum / (float)(STEP_THREADS / 32), __uint_as_float(crowd.most));
+      atomicMax(R.ctl + RUN_CROWD, __float_as_uint(most));
+      atomicMax(R.ctl + RUN_CROWD + 1, crowd.cand);
+    }
     if (wait && !run_barrier(R.bar, b.err)) return false;
   }
   return true;
-}
-
-// Whether too many spheres had more neighbours than a list holds at the
-// launch's last build with lists; the launch then goes on without.  A trip of
-// run_slow costs about four of the walk of a grid step: where the spheres
-// beyond their lists take more than that walk takes for all spheres, it is the
-// cheaper one.  (50,000-sphere pile, a capacity of 2: 49 us a step on lists,
-// 32 us without; 79,420 spheres, 3 % of them four times as large, a capacity
-// of 16: 36 us on lists, 151 us in the step kernels.)  A recorded run has to
-// keep all its lists.
-// Where lists begin, the build is waited for, because a step on them may take
-// very long; spheres that crowd together later do so step by step, and the
-// next build is soon enough.
-template <bool TAPE, class T>
-__device__ __forceinline__ bool run_crowded(const StepBufs<T>& b, const RunBufs<T>& R) {
-  return 4ull * *reinterpret_cast<volatile unsigned long long*>(R.ctl + RUN_CROWD) > (TAPE ? 0u : b.n);
 }
 
 // One step without lists on a grid built for it; the next step's cells are
@@ -961,20 +1007,20 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
           uint32_t move_blocks, uint32_t run_id) {
   uint32_t* maxd = R.ctl + RUN_MAXD;
   if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.bar_next) = 0ull;
-  // (set by an earlier launch: of this one, no CTA gives up before the others have read it)
-  if (*reinterpret_cast<volatile uint32_t*>(b.err) & PS_DEVERR_LIST_BARRIER) return;
+  const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(b.err) & PS_DEVERR_LIST_BARRIER;
   uint32_t streak = *reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_STREAK);
+  // the last step's m, of an earlier run if need be
+  float before = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_BEFORE));
+  if (!(before > 0.0f) || TAPE) before = INFINITY;
+  if (failed) return;  // (an earlier launch: of this one, no CTA gives up before the others have read the word)
   run_begin<T, MULTI, MESH>(b, sp0, mv, R);
   int cur = 1;           // buffer with the state before the step's contacts
   bool lists = false;    // the lists are those of a build that still covers the motion
   bool counted = true;   // the state's cells are counted already
-  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(R.ctl + RUN_CROWD) = 0ull;
+  if (blockIdx.x == 0 && threadIdx.x < 2u) R.ctl[RUN_CROWD + threadIdx.x] = 0u;
   float D = 0.0f;        // motion since the last build, in cells
   float frac = 0.0f;     // skin of the last build, in cells
   uint32_t rebuilds = 0, build = 0;
-  // the last step's m, of an earlier run if need be
-  float before = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_BEFORE));
-  if (!(before > 0.0f) || TAPE) before = INFINITY;
   RunOwn<T> own;
   for (uint32_t s = 0; s < steps; ++s) {
     if (!run_barrier(R.bar, b.err)) return run_leave(b, R.ctl);
