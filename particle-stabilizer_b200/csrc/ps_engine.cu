@@ -2145,12 +2145,15 @@ extern "C" int ps_tune_neighbor_lists(ps_sim* s, int64_t trial_steps, const doub
   cudaEvent_t ea, eb;
   PS_CUDA(cudaEventCreate(&ea));
   PS_CUDA(cudaEventCreate(&eb));
-  // one trial: the same steps twice from the saved state, the second timed
-  // (the first captures the graphs)
+  // one trial: the same steps from the saved state until they take the path
+  // and the graphs that they keep, then timed (without lists the first call may
+  // begin with a probe and the second capture its graphs)
   auto trial = [&](double skin, double& ms_per_step) -> int {
     int r = ps_set_neighbor_lists(s, skin, max_neighbours);
-    if (r == PS_OK) r = load_state(s, saved);
-    if (r == PS_OK) r = ps_step(s, trial_steps);
+    for (int warm = skin > 0.0 ? 1 : 2; warm > 0 && r == PS_OK; --warm) {
+      r = load_state(s, saved);
+      if (r == PS_OK) r = ps_step(s, trial_steps);
+    }
     if (r == PS_OK) r = load_state(s, saved);
     if (r != PS_OK) return r;
     s->eager_lengths.clear();  // no large scene's capture inside the timed call (the warm-up's probe changed its length)
