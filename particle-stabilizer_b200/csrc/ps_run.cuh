@@ -82,7 +82,7 @@ enum : int {
   RUN_REPORT = 10,  // (2 words) the report of runs that choose no path: recorded ones, and those with a set skin
   RUN_BAR_ODD = 12, // grid barrier of odd launches
   RUN_LEFT = 14,    // CTAs that left because a barrier gave up
-  RUN_CROWD = 16,   // (2 words) spheres beyond their lists at the last build: run_crowded's cost and candidates
+  RUN_CROWD = 16,   // spheres beyond their lists at the last build: 0 none, 1 some, 2 too many of some CTA
 };
 
 template <class T>
@@ -287,7 +287,7 @@ __host__ __device__ constexpr int run_batch() {
   return sizeof(T) == 4 ? 4 : 2;
 }
 
-// What the CTA's spheres beyond their lists cost at a build (run_crowded).
+// What the CTA's spheres beyond their lists cost at a build (run_tell_crowd).
 struct RunCrowd {
   float sum;      // of run_slow's trips
   uint32_t most;  // the most of one sphere (the bits of a float that is not negative order like it)
@@ -404,28 +404,31 @@ __device__ __forceinline__ void run_build_one(uint32_t i, const StepBufs<T>& b, 
   R.template counts<TAPE>(build, b.n)[i] = (uint16_t)(word | k);
 }
 
-// Whether, at the launch's last build with lists, the spheres beyond their
-// lists would take longer than steps without lists; the launch then goes on
-// without.  A CTA takes its own such spheres, a warp each: 0.25 us a trip for
-// the one with the most to do, against the rebuild and 0.2 us for every
-// candidate of a thread's spheres.  Both are good to a factor of two (us a step
-// with lists / without, and which the rule takes, FP32: 100 spheres in a heap
-// among 8,000, 543 / 72, without; 400 among 200,000, 14,430 / 341, without;
-// 600,000-sphere pile, lists of 1, 247 / 109, without; of 3, 68 / 103, with;
-// 79,420 spheres, 3 % of them four times as large, lists of 16, 37 / 189, with;
-// 20 of 83,474 ten times as large, lists of 48, 321 / 5,210, with; 3,000 in one
-// cell, 440 / 587, without).
-// A recorded run has to keep all its lists.
-// Where lists begin, the build is waited for, because a step on them may take
-// very long; spheres that crowd together later do so step by step, and the
-// next build is soon enough.
+// A CTA's verdict on its spheres beyond their lists: too many when they would
+// take longer than steps without lists.  It takes them a warp each, 0.25 us a
+// trip for the warp with the most to do, against the rebuild and 0.2 us for
+// every candidate of a thread's spheres.  Both are good to a factor of two (us
+// a step with lists / without, and which the rule takes, FP32: 100 spheres in a
+// heap among 8,000, 543 / 72, without; 400 among 200,000, 14,430 / 341,
+// without; 600,000-sphere pile, lists of 1, 247 / 109, without; of 3, 68 / 103,
+// with; 79,420 spheres, 3 % of them four times as large, lists of 16, 37 / 189,
+// with; 20 of 83,474 ten times as large, lists of 48, 321 / 5,210, with; 3,000
+// in one cell, 440 / 587, without).
+__device__ __noinline__ void run_tell_crowd(const RunCrowd& c, uint32_t n, uint32_t* ctl) {
+  const float cost = fmaxf(c.sum / (float)(STEP_THREADS / 32), __uint_as_float(c.most));
+  const float share = (float)((n + gridDim.x * STEP_THREADS - 1u) / (gridDim.x * STEP_THREADS));
+  const bool many = 0.25f * cost > 20.0f + (float)n / 12000.0f + 0.2f * (float)c.cand * share;
+  atomicMax(ctl + RUN_CROWD, many ? 2u : 1u);
+}
+
+// Whether some CTA found too many; the launch then goes on without lists.  (A
+// recorded run has to keep all its lists.)  It is asked before a build, when
+// the word is complete.  The first step on lists does not depend on it
+// (run_fresh); a CTA that sees the verdict there reports an infinite motion,
+// so that the next step asks.
 template <bool TAPE, class T>
-__device__ __forceinline__ bool run_crowded(const StepBufs<T>& b, const RunBufs<T>& R) {
-  const volatile uint32_t* c = R.ctl + RUN_CROWD;
-  const float cost = __uint_as_float(c[0]), cand = (float)c[1];
-  if (TAPE) return cost > 0.0f;
-  const float share = (float)((b.n + gridDim.x * STEP_THREADS - 1u) / (gridDim.x * STEP_THREADS));
-  return 0.25f * cost > 20.0f + (float)b.n / 12000.0f + 0.2f * cand * share;
+__device__ __forceinline__ bool run_crowded(const RunBufs<T>& R) {
+  return *reinterpret_cast<volatile uint32_t*>(R.ctl + RUN_CROWD) >= (TAPE ? 1u : 2u);
 }
 
 // Contacts of slot i in the exact order whatever has moved: the overlapping
@@ -569,12 +572,11 @@ __device__ __noinline__ void run_begin(const StepBufs<T>& b, const SceneParams<T
 }
 
 // Grid of the state in buffer `cur`, sorted into the other one, and with
-// frac > 0 its lists.  wait: RUN_CROWD is complete at the end.  False: a
-// barrier gave up.
+// frac > 0 its lists.  False: a barrier gave up.
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
                                          const RunBufs<T>& R, int cur, bool counted, float frac, uint32_t build,
-                                         bool wait, int64_t n_cells, uint32_t scatter_blocks, uint32_t move_blocks) {
+                                         int64_t n_cells, uint32_t scatter_blocks, uint32_t move_blocks) {
   const uint32_t stride = gridDim.x * STEP_THREADS;
   if (!counted) {
     vec4_t<T>* Ps = R.p(cur);
@@ -603,7 +605,7 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
   }
   if (!run_barrier(R.bar, b.err)) return false;
   // (behind a barrier that every CTA came to after it read the word)
-  if (frac > 0.0f && blockIdx.x == 0 && threadIdx.x < 2u) R.ctl[RUN_CROWD + threadIdx.x] = 0u;
+  if (frac > 0.0f && blockIdx.x == 0 && threadIdx.x == 0) R.ctl[RUN_CROWD] = 0u;
   for (uint32_t blk = blockIdx.x; blk < scatter_blocks; blk += gridDim.x)
     scatter_block<true>(blk, b.cell, b.slot, b.orig, b.offset, b.tmp, b.count, b.n, b.tile_sum, b.n_tiles, b.err);
   if (!run_barrier(R.bar, b.err)) return false;
@@ -623,12 +625,7 @@ __device__ __noinline__ bool run_rebuild(const StepBufs<T>& b, const SceneParams
     for (uint32_t i = blockIdx.x * STEP_THREADS + threadIdx.x; i < b.n; i += stride)
       run_build_one<T, MULTI, MESH, TAPE>(i, b, scene_of<T, MULTI>(i, sp0, b), mv, R, Ps, (T)frac, rmax, build, crowd);
     __syncthreads();
-    if (threadIdx.x == 0 && crowd.cand != 0u) {  // (the CTA with the most to do decides)
-      const float most = fmaxf(crowd.sum / (float)(STEP_THREADS / 32), __uint_as_float(crowd.most));
-      atomicMax(R.ctl + RUN_CROWD, __float_as_uint(most));
-      atomicMax(R.ctl + RUN_CROWD + 1, crowd.cand);
-    }
-    if (wait && !run_barrier(R.bar, b.err)) return false;
+    if (threadIdx.x == 0 && crowd.cand != 0u) run_tell_crowd(crowd, b.n, R.ctl);
   }
   return true;
 }
@@ -787,19 +784,75 @@ __device__ __forceinline__ void run_mesh_half(vec4_t<T>& P, vec4_t<T>& V, uint32
   mesh_apply<T>(m, c, P, V);
 }
 
+// The spheres that need run_slow's order, in the step right after a build and
+// where they are many: the
+// grid is that of the present positions, so the 27-cell walk of a grid step
+// gives the order, a lane to each sphere, and the step takes no longer than
+// one of those however many contacts they have.
+constexpr uint32_t RUN_FRESH_MIN = STEP_THREADS / 32;  // more than a warp each
+template <class T, bool MULTI, bool MESH, bool TAPE>
+__device__ __noinline__ float run_fresh(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
+                                        const RunBufs<T>& R, const RunLate& l, int cur, uint32_t build, uint32_t s,
+                                        bool last) {
+  const vec4_t<T>* Ps = R.p(cur);
+  const vec4_t<T>* Vs = R.v(cur);
+  float m = 0.0f;
+  for (uint32_t k = threadIdx.x; k < l.n_slow; k += STEP_THREADS) {
+    const uint32_t i = run_put<T>(l, R, k, true);
+    const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
+    vec4_t<T> P = Ps[i];
+    const vec4_t<T> Vi = Vs[i];
+    vec4_t<T> V = Vi;
+    const bool live = isfinite(P.x) && isfinite(P.y) && isfinite(P.z);
+    int32_t cx, cy, cz;
+    cell_coords<T>(b.scell[i], sp, cx, cy, cz);
+    uint32_t lo[9], hi[9];
+    cell_ranges<T>(b, sp, live, cx, cy, cz, lo, hi);
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      for (uint32_t j = lo[q]; j < hi[q]; ++j) {
+        if (q == 4 && j == i) continue;
+        contact_one<T, true>(Vs, j, P, Vi, Ps[j], sp.k_spring, sp.e_sphere, V.x, V.y, V.z);
+      }
+    if (TAPE) run_record<T>(R, b, s, i, P, V, Vi);
+    if (!last) {
+      const vec4_t<T> old = P;
+      integrate<T>(P, V, sp);
+      if constexpr (MESH) {
+        if (sp.mesh_tris > 0)
+          mesh_contacts<T>(P, V, sp, *mv, b.err);
+        else
+          walls<T>(P, V, sp);
+      } else {
+        walls<T>(P, V, sp);
+      }
+      run_finish<T, false>(P, [&] { return b.scell[i]; }, R.template counts<TAPE>(build, b.n)[i], sp, old, m);
+    }
+    (cur ? R.P[0] : R.P[1])[i] = P;
+    (cur ? R.V[0] : R.V[1])[i] = V;
+  }
+  return m;
+}
+
 // The step of the spheres put aside: a warp to each that needs run_slow's
 // order, half a warp to each near a triangle.
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
                                        const RunBufs<T>& R, const RunLate& l, int cur, float frac, uint32_t build,
-                                       uint32_t s, bool last) {
+                                       uint32_t s, bool last, bool fresh) {
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
   vec4_t<T>* Vd = R.v(1 - cur);
   const unsigned lane = threadIdx.x & 31u;
-  const uint32_t n_slow = l.n_slow, n_near = MESH ? l.n_near : 0u;
+  const uint32_t n_near = MESH ? l.n_near : 0u;
+  uint32_t n_slow = l.n_slow;
   float m = 0.0f;
+  if (fresh && n_slow > RUN_FRESH_MIN) {
+    m = run_fresh<T, MULTI, MESH, TAPE>(b, sp0, mv, R, l, cur, build, s, last);
+    n_slow = 0u;
+  }
+  if (fresh && run_crowded<TAPE>(R)) m = INFINITY;
   for (uint32_t k = threadIdx.x >> 5; k < n_slow; k += STEP_THREADS / 32) {
     const uint32_t i = run_put<T>(l, R, k, true);
     const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
@@ -973,7 +1026,7 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
   }
   __syncthreads();
   if (late.n_slow + late.n_near > 0u) {
-    m = fmaxf(m, run_late<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, frac, build, s, last));
+    m = fmaxf(m, run_late<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, frac, build, s, last, fresh));
     if constexpr (OWN) {
       __syncthreads();
       if (odd || near) {
@@ -1017,7 +1070,7 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
   int cur = 1;           // buffer with the state before the step's contacts
   bool lists = false;    // the lists are those of a build that still covers the motion
   bool counted = true;   // the state's cells are counted already
-  if (blockIdx.x == 0 && threadIdx.x < 2u) R.ctl[RUN_CROWD + threadIdx.x] = 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) R.ctl[RUN_CROWD] = 0u;
   float D = 0.0f;        // motion since the last build, in cells
   float frac = 0.0f;     // skin of the last build, in cells
   uint32_t rebuilds = 0, build = 0;
@@ -1028,15 +1081,14 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
     if (blockIdx.x == 0 && threadIdx.x == 0) maxd[(s + 2u) % 3u] = 0u;
     streak = m <= RUN_CALM_MAX ? (streak < RUN_CALM_STEPS ? streak + 1u : streak) : 0u;
     D = D * 1.000001f + m;
-    bool fresh = false;
+    bool fresh = false;  // the state's grid was built before this step
     if (!lists || !(D <= 0.49f * frac)) {
       if (TAPE) {  // a recorded run has lists in every step, or gives up
         if (m > RUN_CALM_MAX || rebuilds == R.max_builds) return;
         build = rebuilds;
         streak = RUN_CALM_STEPS;
       }
-      const bool was = lists;
-      lists = !run_crowded<TAPE>(b, R) && (streak >= RUN_CALM_STEPS || R.skin > 0.0f);
+      lists = !run_crowded<TAPE>(R) && (streak >= RUN_CALM_STEPS || R.skin > 0.0f);
       // (a single fast step, a sphere pushed out of a wall, is no measure)
       // (A recorded run depends on its starting state alone, for the backward
       // pass to give the same sums every time; its builds have to last for
@@ -1045,13 +1097,8 @@ __global__ void __launch_bounds__(STEP_THREADS, run_ctas<T, OWN>())
       const float widest = TAPE && s == 0u ? RUN_SKIN_FIRST : RUN_SKIN_MAX;
       frac = fminf(fmaxf(fminf(m, before) * (last_for / 0.49f), RUN_SKIN_MIN), widest);
       frac = !lists ? 0.0f : (R.skin > 0.0f ? R.skin : frac);
-      if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, lists && !was, n_cells, scatter_blocks,
-                                               move_blocks))
+      if (!run_rebuild<T, MULTI, MESH, TAPE>(b, sp0, mv, R, cur, counted, frac, build, n_cells, scatter_blocks, move_blocks))
         return run_leave(b, R.ctl);
-      if (lists && !was && run_crowded<TAPE>(b, R)) {
-        if (TAPE) return;
-        lists = false;
-      }
       cur = 1 - cur;
       D = 0.0f;
       fresh = true;
