@@ -237,7 +237,8 @@ int ps_backward(ps_sim* sim, const double* dl_dstate, ps_grad* grads, double* dl
  * default).  Results are bit-identical to the grid path: the overlapping
  * pairs of each sphere are applied in the grid walk's order.  A sphere with
  * more than max_neighbours neighbours (capped at 255) walks the cells of the
- * last build instead of a list.  When the device rebuilds more often
+ * last build instead of a list; where that would take longer than a step
+ * without lists, steps run without them.  When the device rebuilds more often
  * than once per 4 steps over 256 or more steps, the next 1,024 steps run on
  * the grid path (doubling, up to 65,536, while that repeats); both paths
  * give the same states.  In this mode ps_step returns after the device has

@@ -7,23 +7,34 @@
 //   d = x_i - x_j, L = |d|, ov = r_i + r_j - L > 0,
 //   f = k ov / (L m_i) - B (u.d) / L^2,  B = 2 m_j e / (m_i + m_j),  u = v_i - v_j
 //
+// A block of steps is recomputed from its checkpoint and recorded, one row of
+// the tape per step: row t + 1 holds the state after step t as the step's
+// contacts left it (positions, velocities, original ids) and the velocities
+// before the contacts, in slot order; row t is the step's input.  There are
+// two forms:
+//   * on lists, by a recorded run (k_run with TAPE): slots keep the order of
+//     the run's last build, and the lists and counts of each build are kept;
+//   * on the grid, by the step kernels, where a block moves too fast for lists
+//     or would need more builds than are kept: slots are in the canonical sort
+//     of their step, and the row also has the sorted cell ids and a copy of
+//     the step's cell offsets.
+// Either way row t + 1 is exactly the state after the walls that step t's
+// contacts read, so the reverse sweep needs no rebuild.
+//
 // Reverse sweep of one step, given the adjoints (xbar, vbar) of its output:
-//   k_adj_contacts   (sorted order, gather): for each particle, the terms of
-//                    the pairs where it receives and the pairs where it is the
-//                    source (pairs are symmetric), so no atomics; partials of
-//                    dL/dk and dL/de_sphere accumulated per sorted slot (a
-//                    scene owns a fixed slot range, so per-scene sums are
-//                    unchanged and the order is fixed by the canonical sort).
-//   k_adj_walls_integrate (the tape row's sorted order): through the walls
-//                    (clamp events recomputed from the recorded step input)
-//                    and the integrate; partials of dL/de_wall by slot.
-// The block recompute records, per step, the at-rest state after it in
-// sorted order (positions, velocities, original ids) together with the
-// step's grid (pre-contact velocities, sorted cell ids, and a copy of the
-// cell offsets).  Row t + 1 plus offsets t are then exactly the sorted
-// post-wall state and grid that step t's contacts read, so the reverse sweep
-// runs the contact adjoint on them directly, without rebuilding the grid,
-// and row t is the step's input for the walls/integrate adjoint.
+//   k_adj_list       (slots of the build, gather over the slot's list) or
+//   k_adj_contacts   (sorted order, gather over the 27 cells): for each
+//                    particle, the terms of the pairs where it receives and
+//                    the pairs where it is the source (pairs are symmetric),
+//                    so no atomics; partials of dL/dk and dL/de_sphere
+//                    accumulated per slot (a scene owns a fixed slot range,
+//                    so per-scene sums are unchanged and the order is fixed
+//                    by that of the slots).
+//   walls and integrate: through the walls (clamp events recomputed from the
+//                    recorded step input) and the integrate, with the partials
+//                    of dL/de_wall.  In k_adj_list where the step before has
+//                    the same slots, by k_adj_walls_integrate (slots of row t,
+//                    found through `inv`) where it has not.
 // Wall clamps and contact activation are piecewise events taken from the
 // forward values; radii and masses are constants.
 #pragma once
@@ -48,8 +59,8 @@ struct AdjBufs {
   vec4_t<T>* ax2;         // output of k_adj_contacts, in the order of step t's grid
   vec4_t<T>* av2;
   uint32_t* inv;          // slot in step t's grid of each original id (written by k_adj_contacts)
-  double* acc;            // ADJ_NACC rows of n, accumulated over steps: rows k, e by sorted
-                          // slot, wall rows by original index
+  double* acc;            // ADJ_NACC rows of n, accumulated over steps: rows k, e by the slot of
+                          // step t's order, wall rows by that of its input
   uint32_t n;             // row length of acc
 };
 

@@ -785,10 +785,9 @@ __device__ __forceinline__ void run_mesh_half(vec4_t<T>& P, vec4_t<T>& V, uint32
 }
 
 // The spheres that need run_slow's order, in the step right after a build and
-// where they are many: the
-// grid is that of the present positions, so the 27-cell walk of a grid step
-// gives the order, a lane to each sphere, and the step takes no longer than
-// one of those however many contacts they have.
+// where they are many: the grid is that of the present positions, so the
+// 27-cell walk of a grid step gives the order, a lane to each sphere, and the
+// step takes no longer than one of those however many contacts they have.
 constexpr uint32_t RUN_FRESH_MIN = STEP_THREADS / 32;  // more than a warp each
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ float run_fresh(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,

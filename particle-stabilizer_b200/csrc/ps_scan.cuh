@@ -6,9 +6,9 @@
 // One launch, one read and one write per element.  Each CTA takes a tile of
 // SCAN_TILE elements in ticket order (an atomic counter, so every
 // predecessor tile is already running), publishes its aggregate, then its
-// first warp looks back over 32 predecessor status words at a time until one
-// holds an inclusive prefix.  A status word packs (value << 32 | flag)
-// so value and flag travel in one 64-bit store.  Every wait on a predecessor
+// first warp looks back over 32 * SCAN_WINDOWS predecessor status words at a
+// time until one holds an inclusive prefix.  A status word packs
+// (value << 32 | flag) so value and flag travel in one 64-bit store.  Every wait on a predecessor
 // is bounded: after SCAN_SPIN_LIMIT polls the thread records
 // PS_DEVERR_SCAN_TIMEOUT in the error word and takes the missing value as 0,
 // so the kernel always returns.
@@ -21,7 +21,7 @@
 namespace psb {
 
 constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 32;  // per thread: 128 contiguous bytes
+constexpr int SCAN_ITEMS = 32;  // per thread, as 8 uint4: one of each row of its warp
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr uint32_t SCAN_SPIN_LIMIT = 1u << 20;
 
