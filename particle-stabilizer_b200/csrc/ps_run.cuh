@@ -788,6 +788,9 @@ __device__ __forceinline__ void run_mesh_half(vec4_t<T>& P, vec4_t<T>& V, uint32
 // where they are many: the grid is that of the present positions, so the
 // 27-cell walk of a grid step gives the order, a lane to each sphere, and the
 // step takes no longer than one of those however many contacts they have.
+// run_list_step calls it: a call inside run_late, whose registers it takes,
+// cost every step (4,000-sphere funnel, steps 42 to 328, each against the
+// kernel without this function in turn: 2,447 -> 2,628 us; now 2,600 -> 2,495).
 constexpr uint32_t RUN_FRESH_MIN = STEP_THREADS / 32;  // more than a warp each
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ float run_fresh(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
@@ -833,25 +836,22 @@ __device__ __noinline__ float run_fresh(const StepBufs<T>& b, const SceneParams<
   return m;
 }
 
-// The step of the spheres put aside: a warp to each that needs run_slow's
-// order, half a warp to each near a triangle.
+// The step of the spheres put aside: a warp to each of the n_slow that need
+// run_slow's order (none where run_fresh has taken them), half a warp to each
+// near a triangle.  (A function for each of the two kinds: 30,011-sphere pile,
+// 328 steps, 2,750 -> 2,804 us.  The part of run_slow for more than 32 pairs as
+// a function of its own: 2,717 -> 2,778.)
 template <class T, bool MULTI, bool MESH, bool TAPE>
 __device__ __noinline__ float run_late(const StepBufs<T>& b, const SceneParams<T>& sp0, const MeshView* mv,
                                        const RunBufs<T>& R, const RunLate& l, int cur, float frac, uint32_t build,
-                                       uint32_t s, bool last, bool fresh) {
+                                       uint32_t s, bool last, uint32_t n_slow) {
   const vec4_t<T>* Ps = R.p(cur);
   const vec4_t<T>* Vs = R.v(cur);
   vec4_t<T>* Pd = R.p(1 - cur);
   vec4_t<T>* Vd = R.v(1 - cur);
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t n_near = MESH ? l.n_near : 0u;
-  uint32_t n_slow = l.n_slow;
   float m = 0.0f;
-  if (fresh && n_slow > RUN_FRESH_MIN) {
-    m = run_fresh<T, MULTI, MESH, TAPE>(b, sp0, mv, R, l, cur, build, s, last);
-    n_slow = 0u;
-  }
-  if (fresh && run_crowded<TAPE>(R)) m = INFINITY;
   for (uint32_t k = threadIdx.x >> 5; k < n_slow; k += STEP_THREADS / 32) {
     const uint32_t i = run_put<T>(l, R, k, true);
     const SceneParams<T>& sp = scene_of<T, MULTI>(i, sp0, b);
@@ -1025,7 +1025,10 @@ __device__ __forceinline__ float run_list_step(const StepBufs<T>& b, const Scene
   }
   __syncthreads();
   if (late.n_slow + late.n_near > 0u) {
-    m = fmaxf(m, run_late<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, frac, build, s, last, fresh));
+    const bool walk = fresh && late.n_slow > RUN_FRESH_MIN;
+    if (walk) m = fmaxf(m, run_fresh<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, build, s, last));
+    m = fmaxf(m, run_late<T, MULTI, MESH, TAPE>(b, sp0, mv, R, late, cur, frac, build, s, last, walk ? 0u : late.n_slow));
+    if (fresh && run_crowded<TAPE>(R)) m = INFINITY;
     if constexpr (OWN) {
       __syncthreads();
       if (odd || near) {
