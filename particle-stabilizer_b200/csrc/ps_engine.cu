@@ -720,14 +720,22 @@ int upload_grids(ps_sim* s, std::vector<SceneParams<T>>& sps) {
 template <class T>
 int upload_mesh(ps_sim* s) {
   std::vector<T> tri, aabb;
-  std::vector<double> nrm;
+  std::vector<double> nrm, off_plane;
   std::vector<uint32_t> bin_offset((size_t)s->bins_total + 1, 0), bin_tri;
+  // a unit of the last place of a scene's coordinates, for the rounding of the device's own tests
+  auto ulp_of = [](const GridHost& g) {
+    double size = g.mesh_iv;
+    for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
+    return (double)std::numeric_limits<T>::epsilon() * size;
+  };
   tri.reserve((size_t)s->tri_total * 12);
   aabb.reserve((size_t)s->tri_total * 8);
   nrm.reserve((size_t)s->tri_total * 3);
+  off_plane.reserve((size_t)s->tri_total);
   for (int sc = 0; sc < s->n_scenes; ++sc) {
     const GridHost& g = s->grids[sc];
     const std::vector<double>& soup = s->tris[sc];
+    const double ulp = ulp_of(g);
     for (int64_t t = 0; t < g.n_tri; ++t) {
       const double* v = soup.data() + 9 * t;
       for (int k = 0; k < 9; ++k) tri.push_back((T)v[k]);
@@ -743,7 +751,14 @@ int upload_mesh(ps_sim* s) {
       for (int a = 0; a < 3; ++a) aabb.push_back(std::min(std::min((T)v[a], (T)v[3 + a]), (T)v[6 + a]));
       aabb.push_back(T(0));
       for (int a = 0; a < 3; ++a) aabb.push_back(std::max(std::max((T)v[a], (T)v[3 + a]), (T)v[6 + a]));
-      aabb.push_back(T(0));
+      const double* n = nrm.data() + nrm.size() - 3;
+      double off = 0.0;  // of its vertices from the plane (infinite for a triangle without a normal)
+      for (int k = 3; k < 9; k += 3) {
+        const double d = std::fabs(n[0] * (v[k] - v[0]) + n[1] * (v[k + 1] - v[1]) + n[2] * (v[k + 2] - v[2]));
+        off = d == d ? std::max(off, d) : INFINITY;
+      }
+      off_plane.push_back(off);
+      aabb.push_back((T)(1.001 * off + 8.0 * ulp));
     }
   }
   // two passes: count, then fill (ascending triangle id inside each bin)
@@ -758,9 +773,7 @@ int upload_mesh(ps_sim* s) {
       const GridHost& g = s->grids[sc];
       const T lo[3] = {(T)g.mesh_lo[0], (T)g.mesh_lo[1], (T)g.mesh_lo[2]};
       const T iv = (T)g.mesh_iv;
-      double size = g.mesh_iv;  // of the coordinates, for the rounding of the device's own tests
-      for (int a = 0; a < 3; ++a) size = std::max({size, std::fabs(g.mesh_lo[a]), std::fabs(g.mesh_hi[a])});
-      const double ulp = (double)std::numeric_limits<T>::epsilon() * size;
+      const double ulp = ulp_of(g);
       const double reach = 1.001 * g.mesh_reach + 8.0 * ulp;
       for (int64_t t = 0; t < g.n_tri; ++t) {
         const int64_t gt = g.tri_base + t;
@@ -772,12 +785,7 @@ int upload_mesh(ps_sim* s) {
         const double* n = nrm.data() + 3 * gt;
         const double* v0 = s->tris[sc].data() + 9 * t;
         const double far = reach + (0.5 + 1e-3) * g.mesh_iv * (std::fabs(n[0]) + std::fabs(n[1]) + std::fabs(n[2])) + 80.0 * ulp;
-        double off = 0.0;  // of its vertices from the plane (not a number for a triangle without a normal)
-        for (int k = 3; k < 9; k += 3) {
-          const double d = std::fabs(n[0] * (v0[k] - v0[0]) + n[1] * (v0[k + 1] - v0[1]) + n[2] * (v0[k + 2] - v0[2]));
-          if (!(d <= off)) off = d;
-        }
-        const bool flat = off <= 8.0 * ulp;  // it is flat and its normal is good
+        const bool flat = off_plane[(size_t)gt] <= 8.0 * ulp;  // it is flat and its normal is good
         for (int32_t x = b0[0]; x <= b1[0]; ++x)
           for (int32_t y = b0[1]; y <= b1[1]; ++y)
             for (int32_t z = b0[2]; z <= b1[2]; ++z) {

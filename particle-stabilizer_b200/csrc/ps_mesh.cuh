@@ -27,7 +27,7 @@ namespace psb {
 // Every scene's binned triangles.
 struct MeshView {
   const void* tri;     // three vec4 per triangle: v0, v1, v2, unit normal
-  const void* aabb;    // two vec4 per triangle: min xyz, max xyz
+  const void* aabb;    // two vec4 per triangle: min xyz, max xyz and (w) how far its vertices may be off its plane
   const uint32_t* bin_offset;  // CSR offsets per bin (+1)
   const uint32_t* bin_tri;     // triangle ids (global)
   uint32_t n_tri;      // triangles over all scenes
@@ -123,9 +123,11 @@ __device__ __forceinline__ Triangle<T> triangle(const MeshView& mv, uint32_t t) 
 
 // Closed test of triangle t's AABB against [lo, hi] (isIntersectedKernel :191-197).
 template <class T>
-__device__ __forceinline__ bool in_box(const MeshView& mv, uint32_t t, const V3<T>& lo, const V3<T>& hi) {
+__device__ __forceinline__ bool in_box(const MeshView& mv, uint32_t t, const V3<T>& lo, const V3<T>& hi,
+                                       T* off_plane = nullptr) {
   const vec4_t<T>* q = static_cast<const vec4_t<T>*>(mv.aabb) + 2 * (size_t)t;
   const vec4_t<T> mn = ld4<T>(q), mx = ld4<T>(q + 1);
+  if (off_plane != nullptr) *off_plane = mx.w;
   return lo.x <= mx.x && hi.x >= mn.x && lo.y <= mx.y && hi.y >= mn.y && lo.z <= mx.z && hi.z >= mn.z;
 }
 
@@ -260,12 +262,10 @@ __device__ __forceinline__ uint32_t mesh_candidates(const vec4_t<T>& P, T skin, 
   uint32_t n = 0;
   mesh_bins<T>({P.x - skin, P.y - skin, P.z - skin}, {P.x + skin, P.y + skin, P.z + skin}, sp, mv, err,
                [&](uint32_t t) {
-                 if (n > CAP || !in_box<T>(mv, t, lo, hi)) return;
+                 T off;  // (with the box: from the vertices here, funnels took 0.4 % longer)
+                 if (n > CAP || !in_box<T>(mv, t, lo, hi, &off)) return;
                  const Triangle<T> g = triangle<T>(mv, t);
-                 const V3<T> ab = v3sub(g.b, g.a), ac = v3sub(g.c, g.a);
                  const T h = (P.x - g.a.x) * g.n.x + (P.y - g.a.y) * g.n.y + (P.z - g.a.z) * g.n.z;
-                 // vertices off the plane: the normal of a triangle without area is rounding
-                 const T off = fabs(v3dot(ab, g.n)) + fabs(v3dot(ac, g.n));
                  if (fabs(h) > along + off) return;  // (a triangle without a normal stays)
                  uint32_t k = n;  // several bins: not in order, and not once
                  while (k > 0u && ids[k - 1] > t) --k;
